@@ -101,3 +101,21 @@ def test_autotune_keeps_state_and_parity():
                 break
     finally:
         d.close()
+
+
+@pytest.mark.parametrize("shape", [(40, 61), (33, 30)])
+@pytest.mark.parametrize("value", [0.0, 1e-310, 1e-250, 1e95])
+def test_extreme_depths_bit_exact(value, shape):
+    """Depths outside the range of the flux tile's straight-line arithmetic
+    (2^-300 .. 2^300; 0 is inside) in some tiles of an ordinary wet case, on
+    tile edges too: those tiles take the guarded forms and must still equal
+    the oracle bit for bit."""
+    from triton_b200 import scenarios
+    rows, cols = shape
+    sc = scenarios.mixed(rows=rows, cols=cols, seed=31, friction=False, with_extbc=False, with_sources=False,
+                         with_runoff=False, duration=4.0)
+    for r, c in ((1, 1), (8, 30), (9, 31 if cols > 31 else 5), (rows, cols)):
+        sc.h[r, c] = value
+        sc.qx[r, c] = sc.qy[r, c] = 0.0
+    steps, _ = run_lockstep(sc, exact=True, max_events=1, chunk=6)
+    assert 0 < steps <= 6  # an observation event may come first

@@ -31,7 +31,8 @@ struct CellQ {
   double zb;
 };
 
-template <typename T>
+// LINE: the FP64 straight-line forms, for cells that regular_cell() accepts.
+template <typename T, bool LINE = false>
 __device__ __forceinline__ CellQ<T> make_cell(T h, T qx, T qy, T z, T hextra, double zb = 0.0) {
   CellQ<T> c;
   c.h = h;
@@ -39,6 +40,17 @@ __device__ __forceinline__ CellQ<T> make_cell(T h, T qx, T qy, T z, T hextra, do
   c.qy = qy;
   c.z = z;
   c.zb = zb;
+  if constexpr (LINE && sizeof(T) == 8) {
+    const double hs = h > 0.0 ? h : 1.0;
+    const double y = rsqrt_line(hs);
+    const double s = sqrt_line(hs, y);
+    const double rh = recip_line(hs, y * y);
+    const bool flows = h >= hextra;
+    c.sq = h > 0.0 ? s : 0.0;
+    c.u = flows ? div_line(qx, hs, rh) : 0.0;
+    c.v = flows ? div_line(qy, hs, rh) : 0.0;
+    return c;
+  }
   c.sq = dev_fmax(dev_sqrt(h), T(0));
   if (h >= hextra) {
     const T rh = recip(h);
@@ -102,8 +114,21 @@ __device__ __forceinline__ T n_cross(T a, T b) {  // b*nx - a*ny
   return XFACE ? b : -a;
 }
 
-template <typename T, bool XFACE>
+// A quotient by a shared divisor, its reciprocal given: straight-line or guarded.
+template <bool LINE>
+__device__ __forceinline__ double quot(double a, double b, double y) {
+  return LINE ? div_line(a, b, y) : div_shared(a, b, y);
+}
+template <bool LINE>
+__device__ __forceinline__ float quot(float a, float b, float y) {
+  return div_shared(a, b, y);
+}
+
+// LINE (FP64): both cells are regular (regular_cell), so square roots,
+// reciprocals and shared quotients take their straight-line forms.
+template <typename T, bool XFACE, bool LINE = false>
 __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<T>& c2, const StepK<T>& K) {
+  constexpr bool L64 = LINE && sizeof(T) == 8;
   const T dx = K.dx, dt = K.dt, hextra = K.hextra;
   const T G = T(kGravity), SG = T(kSqrtG), E12 = eps12<T>();
   FaceOut<T> out;
@@ -118,12 +143,21 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
   // Roe-averaged state and wave speeds
   const T h12 = T(0.5) * (h1 + h2);
   const T dh = h2 - h1;
-  const T c12 = dev_sqrt(G * h12);
-  const T rc12 = recip(c12);  // shared divisors: exact quotients via div_shared
   const T ssq = sqh1 + sqh2;
-  const T rssq = recip(ssq);
-  const T u12 = div_shared(u1 * sqh1 + u2 * sqh2, ssq, rssq);
-  const T v12 = div_shared(v1 * sqh1 + v2 * sqh2, ssq, rssq);
+  T c12, rc12, rssq;  // shared divisors: exact quotients via quot
+  if constexpr (L64) {
+    const T gh = G * h12;
+    const T y = rsqrt_line(gh);
+    c12 = sqrt_line(gh, y);
+    rc12 = recip_line(c12, y);
+    rssq = recip_line(ssq);
+  } else {
+    c12 = dev_sqrt(G * h12);
+    rc12 = recip(c12);
+    rssq = recip(ssq);
+  }
+  const T u12 = quot<L64>(u1 * sqh1 + u2 * sqh2, ssq, rssq);
+  const T v12 = quot<L64>(v1 * sqh1 + v2 * sqh2, ssq, rssq);
   const T un = n_dot<T, XFACE>(u12, v12);
   T lam0 = un - c12, lam1 = un, lam2 = un + c12;
   T lamE0 = T(0), lamE2 = T(0);  // lamE1 is always zero
@@ -155,9 +189,9 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
 
   // wave strengths
   const T dqx = c2.qx - c1.qx, dqy = c2.qy - c1.qy;
-  const T aq = div_shared(n_dot<T, XFACE>(dqx, dqy) - un * dh, c12, rc12);
+  const T aq = quot<L64>(n_dot<T, XFACE>(dqx, dqy) - un * dh, c12, rc12);
   const T al0 = T(0.5) * (dh - aq);
-  const T al1 = div_shared(n_cross<T, XFACE>(dqx - u12 * dh, dqy - v12 * dh), c12, rc12);
+  const T al1 = quot<L64>(n_cross<T, XFACE>(dqx - u12 * dh, dqy - v12 * dh), c12, rc12);
   const T al2 = T(0.5) * (dh + aq);
 
   // upwinded bed-step source, limited where the step is higher than the water
@@ -184,7 +218,7 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
     hp = h2;
     if (above2) dzp = -h2;
   }
-  T be0 = div_shared(T(0.5) * G * (hp - T(0.5) * dev_fabs(dzp)) * dzp, c12, rc12);
+  T be0 = quot<L64>(T(0.5) * G * (hp - T(0.5) * dev_fabs(dzp)) * dzp, c12, rc12);
 
   // positivity limiter on subcritical wet-wet faces
   hp = h1 + al0;
@@ -192,8 +226,15 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
     // lam/(lam + lamE) is exactly 1 without an entropy-fix part (lam != 0 here)
     const T f0 = lamE2 == T(0) ? T(1) : div_rare(lam0, lam0 + lamE2);
     const T f2 = lamE0 == T(0) ? T(1) : div_rare(lam2, lam2 + lamE0);
-    be0 = dev_fmax(be0, f0 * (al0 * lam0 - div_nz(h1 * dx * T(0.5), dt, K.rdt) + lamE2 * h2));
-    be0 = dev_fmin(be0, f2 * (-al2 * lam2 + div_nz(h2 * dx * T(0.5), dt, K.rdt) + lamE0 * h1));
+    const T lo = f0 * (al0 * lam0 - div_nz(h1 * dx * T(0.5), dt, K.rdt) + lamE2 * h2);
+    const T hi = f2 * (-al2 * lam2 + div_nz(h2 * dx * T(0.5), dt, K.rdt) + lamE0 * h1);
+    if constexpr (L64) {  // no NaN here: plain selections
+      be0 = lo > be0 ? lo : be0;
+      be0 = hi < be0 ? hi : be0;
+    } else {
+      be0 = dev_fmax(be0, lo);
+      be0 = dev_fmin(be0, hi);
+    }
   }
   const T be2 = -be0;
   const T be1 = T(0);

@@ -3,7 +3,10 @@
 // bit for bit: div_by_rcp over operands shaped like the step's (dt*d/dx,
 // h*dx/2/dt: magnitudes 1e-14 .. 1e7 over divisors 1e-3 .. 1e3) and
 // div_shared over every finite dividend magnitude (subnormals included,
-// zeros of both signs) and divisors of either sign from 1e-30 to 1e30.
+// zeros of both signs) and divisors of either sign from 1e-30 to 1e30.  Also
+// the straight-line forms of the FP64 flux tile (tri_common.cuh) over their
+// whole range, 2^-300 .. 2^300, a part of it at operands whose result lies
+// next to the midpoint of two doubles or whose mantissa is all ones.
 #include <cuda_runtime.h>
 
 #include "tri_common.cuh"
@@ -22,6 +25,49 @@ __device__ __forceinline__ unsigned long long mix(unsigned long long x) {
 }
 
 __device__ __forceinline__ double unit(unsigned long long r) { return (double)(r >> 11) * (1.0 / 9007199254740992.0); }
+
+__device__ __forceinline__ bool differ(double a, double b) {
+  return __double_as_longlong(a) != __double_as_longlong(b);
+}
+
+// Mismatches of the straight-line forms for one random x of 2^-300 .. 2^300.
+__device__ int line_check(unsigned long long r1, unsigned long long r2) {
+  const int e = (int)((r1 >> 52) % 600) - 300;
+  const double m = __longlong_as_double((long long)((r1 & 0x000FFFFFFFFFFFFFull) | 0x3FF0000000000000ull));  // 1 .. 2
+  double x = ldexp(m, e);
+  switch (r2 & 7) {
+    case 0: {  // sqrt(x) next to the midpoint above m
+      const double s = ldexp(m, e / 2), u = ldexp(0x1p-53, e / 2);
+      x = s * s + 2.0 * s * u;
+      break;
+    }
+    case 1: {  // 1/x next to the midpoint above m
+      const double y = 1.0 / m;
+      x = ldexp(fma(-y * y, 0x1p-53, y), e);
+      break;
+    }
+    case 2:  // mantissa of (nearly) all ones or (nearly) all zeros
+      x = ldexp((r2 & 8) ? 2.0 - (double)((r2 >> 4) & 3) * 0x1p-52 - 0x1p-52 : 1.0 + (double)((r2 >> 4) & 3) * 0x1p-52, e);
+      break;
+    case 3: {  // sqrt(x) of (nearly) all ones
+      const double t = ldexp(2.0 - (double)((r2 >> 4) & 1) * 0x1p-52 - 0x1p-52, e / 2);
+      x = t * t;
+      x = __longlong_as_double(__double_as_longlong(x) + (long long)((r2 >> 5) & 3) - 1);
+      break;
+    }
+    default: break;
+  }
+  int bad = 0;
+  const double y = rsqrt_line(x), s = sqrt_line(x, y), rx = 1.0 / x;
+  bad += differ(s, sqrt(x));
+  if (__double2loint(x) != -1) bad += differ(recip_line(x, y * y), rx);  // such depths are not regular
+  bad += differ(recip_line(s, y), 1.0 / s);
+  bad += differ(recip_line(x), rx);
+  const double a = ldexp(1.0 + (double)(r2 >> 12) * 0x1p-52, (int)(r2 % 601) - 300) * ((r2 & 16) ? -1.0 : 1.0);
+  bad += differ(div_line(a, x, rx), a / x);
+  bad += div_line(0.0, x, rx) != 0.0;
+  return bad;
+}
 
 __global__ void k_div_check(long long n, unsigned long long seed, unsigned long long* bad) {
   unsigned long long local = 0;
@@ -44,6 +90,7 @@ __global__ void k_div_check(long long n, unsigned long long seed, unsigned long 
     const double b2 = exp10(-30.0 + 60.0 * unit(r4)) * ((r4 & 0x80) ? -1.0 : 1.0);
     const double q2 = div_shared(a2, b2, 1.0 / b2);
     if (__double_as_longlong(q2) != __double_as_longlong(a2 / b2)) local++;
+    local += (unsigned)line_check(mix(r3 ^ 0x2545F4914F6CDD1Dull), r4);
   }
   if (local) atomicAdd(bad, local);
 }

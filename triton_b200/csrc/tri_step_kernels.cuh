@@ -281,6 +281,22 @@ __device__ __forceinline__ FluxCtx<T> flux_ctx(DevClock* clk, const StateBufs<T>
   return X;
 }
 
+// The same with the dry-tile flags: [2][tiles] zero flags by buffer, then
+// [tiles] pinned.
+template <typename T, bool kSkip>
+__device__ __forceinline__ FluxCtx<T> flux_ctx_skip(DevClock* clk, const StateBufs<T>& sb, const BedMap<T>& bed,
+                                                    const T* n2, const int32_t* zone, const T* rates, int rows,
+                                                    int cols, int rb, T dx, T rdx, T hextra, uint8_t* tzero) {
+  FluxCtx<T> X = flux_ctx<T>(clk, sb, bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra);
+  if (kSkip) {
+    const size_t ntiles = (size_t)X.nstrips * (size_t)((rows - 2 + rb - 1) / rb);
+    X.tz_src = tzero + (size_t)clk->src * ntiles;
+    X.tz_dst = tzero + (size_t)clk->dst * ntiles;
+    X.tpin = tzero + 2 * ntiles;
+  }
+  return X;
+}
+
 // Zero bits (+0): a tile is skipped only where every value it would write
 // is +0 already, so skipping is exact.
 __device__ __forceinline__ bool nonzero_bits(double v) { return __double_as_longlong(v) != 0; }
@@ -323,8 +339,15 @@ __device__ __forceinline__ const P* launder_ptr(const P* p) {
 // stores, 20 with the reads; 25.5 against 23.8 G cell-updates/s at the best
 // launch shape).  The single-domain kernel keeps kReload off: its context
 // comes from kernel parameters, which the compiler reads at each use.
-template <typename T, bool kTrack, bool kReload = false>
-__device__ __forceinline__ void flux_tile(const FluxCtx<T>& X0, unsigned tile, int lane) {
+//
+// kLine (FP64): the tile is computed with the straight-line forms, which hold
+// for regular cells; where a lane meets another kind of cell, the whole tile
+// returns false without having added to the accounts or its dry flag, and
+// the caller computes it again with the guarded forms (the tile only reads
+// the source buffer, so it can be repeated).
+template <typename T, bool kTrack, bool kReload, bool kLine>
+__device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, unsigned tile, int lane) {
+  bool odd = false;  // this lane met a cell that is not regular
   const FluxCtx<T>& X = kReload ? *launder_ptr(&X0) : X0;
   const int rows = X.rows, cols = X.cols, rb = X.rb;
   const T hextra = X.K.hextra;
@@ -379,7 +402,8 @@ __device__ __forceinline__ void flux_tile(const FluxCtx<T>& X0, unsigned tile, i
     }
   };
   fetch(X, r0 - 1);
-  CellQ<T> prev = make_cell<T>(lh, lqx, lqy, lz, hextra, lzb);
+  if (kLine) odd = !regular_cell(lh, lqx, lqy);
+  CellQ<T> prev = make_cell<T, kLine>(lh, lqx, lqy, lz, hextra, lzb);
   if (r0 - 1 == 0 && owner) copy_ghost(X, 0);
   fetch(X, r0);
   RowParts<T> pp;
@@ -390,7 +414,8 @@ __device__ __forceinline__ void flux_tile(const FluxCtx<T>& X0, unsigned tile, i
     // the context is read where it is used, so with kReload none of it is
     // held across the face computations
     const FluxCtx<T>& XL = kReload ? *launder_ptr(&X0) : X0;
-    const CellQ<T> cur = make_cell<T>(lh, lqx, lqy, lz, XL.K.hextra, lzb);
+    if (kLine) odd |= !regular_cell(lh, lqx, lqy);
+    const CellQ<T> cur = make_cell<T, kLine>(lh, lqx, lqy, lz, XL.K.hextra, lzb);
     T cn2 = T(0);
     if (r <= r1) {
       if (upd) cn2 = XL.n2[(size_t)r * XL.cols + c];
@@ -398,7 +423,7 @@ __device__ __forceinline__ void flux_tile(const FluxCtx<T>& X0, unsigned tile, i
     }
     FaceOut<T> Y;
     Y.a0 = Y.a1 = Y.a2 = Y.b0 = Y.b1 = Y.b2 = T(0);
-    if (upd) Y = face_flux<T, false>(cur, prev, XL.K);
+    if (upd) Y = face_flux<T, false, kLine>(cur, prev, XL.K);
     if (r - 1 >= r0 && upd) {
       const FluxCtx<T>& XU = kReload ? *launder_ptr(&X0) : X0;
       const int cols = XU.cols;
@@ -459,7 +484,7 @@ __device__ __forceinline__ void flux_tile(const FluxCtx<T>& X0, unsigned tile, i
     left.zb = sizeof(T) == 4 ? __shfl_up_sync(0xffffffffu, cur.zb, 1) : 0.0;
     FaceOut<T> Xf;
     Xf.a0 = Xf.a1 = Xf.a2 = Xf.b0 = Xf.b1 = Xf.b2 = T(0);
-    if (lane >= 1 && incol && c >= 1) Xf = face_flux<T, true>(left, cur, XL.K);
+    if (lane >= 1 && incol && c >= 1) Xf = face_flux<T, true, kLine>(left, cur, XL.K);
     const T e0 = shfl_down1(Xf.a0), e1 = shfl_down1(Xf.a1), e2 = shfl_down1(Xf.a2);
     if (kAcct && upd) {
       // Inflow through faces shared with ghost cells, in depth units.  The
@@ -481,6 +506,7 @@ __device__ __forceinline__ void flux_tile(const FluxCtx<T>& X0, unsigned tile, i
     if (gcol) copy_ghost(XL, r);
     prev = cur;
   }
+  if (kLine && __any_sync(0xffffffffu, odd)) return false;
   if (kAcct) {
     acc_b = warp_sum<T>(acc_b);
     acc_r = warp_sum<T>(acc_r);
@@ -495,6 +521,28 @@ __device__ __forceinline__ void flux_tile(const FluxCtx<T>& X0, unsigned tile, i
     const bool nz = __any_sync(0xffffffffu, wrote_nonzero);
     if (lane == 0) X.tz_dst[tile] = (!nz && !X.tpin[tile]) ? 1 : 0;
   }
+  return true;
+}
+
+// The guarded forms, out of line: a tile with extreme values is rare.  The
+// single-domain kernel's context is formed again from the kernel parameters
+// (a context that the call took by reference would live in local memory).
+template <typename T>
+__device__ __noinline__ void flux_tile_guarded_ctx(const FluxCtx<T>* X, unsigned tile, int lane) {
+  flux_tile_form<T, false, true, false>(*X, tile, lane);
+}
+template <typename T, bool kSkip>
+__device__ __noinline__ void flux_tile_guarded(DevClock* clk, const StateBufs<T> sb, const BedMap<T> bed, const T* n2,
+                                               const int32_t* zone, const T* rates, int rows, int cols, int rb, T dx,
+                                               T rdx, T hextra, uint8_t* tzero, unsigned tile, int lane) {
+  flux_tile_form<T, kSkip, false, false>(
+      flux_ctx_skip<T, kSkip>(clk, sb, bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra, tzero), tile, lane);
+}
+
+// One tile of a batch member, its context in shared memory.
+template <typename T>
+__device__ __forceinline__ void flux_tile_member(const FluxCtx<T>& X, unsigned tile, int lane) {
+  if (!flux_tile_form<T, false, true, sizeof(T) == 8>(X, tile, lane)) flux_tile_guarded_ctx<T>(&X, tile, lane);
 }
 
 // kSkip: the domain keeps dry-tile flags (tzero) and skips dry tiles.
@@ -506,14 +554,10 @@ __global__ void __launch_bounds__(128, MINB) k_flux_update(DevClock* __restrict_
                                                      uint8_t* __restrict__ tzero) {
   pdl_wait();
   if (!clk->active) return;
-  FluxCtx<T> X = flux_ctx<T>(clk, sb, bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra);
+  const FluxCtx<T> X =
+      flux_ctx_skip<T, kSkip>(clk, sb, bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra, tzero);
   const int lane = threadIdx.x & 31;
   const unsigned ntiles = (unsigned)X.nstrips * (unsigned)((rows - 2 + rb - 1) / rb);
-  if (kSkip) {  // [2][ntiles] zero flags by buffer, then [ntiles] pinned
-    X.tz_src = tzero + (size_t)clk->src * ntiles;
-    X.tz_dst = tzero + (size_t)clk->dst * ntiles;
-    X.tpin = tzero + 2 * (size_t)ntiles;
-  }
   unsigned skipped = 0;  // interior cells of the tiles this warp skipped (lane 0)
   while (true) {
     unsigned tile = 0;  // lane 0 takes the next tile; bit 31: skip it (tiles < 2^31)
@@ -528,7 +572,8 @@ __global__ void __launch_bounds__(128, MINB) k_flux_update(DevClock* __restrict_
     tile = __shfl_sync(0xffffffffu, tile, 0);
     if ((tile & 0x7FFFFFFFu) >= ntiles) break;
     if (kSkip && (tile >> 31)) continue;
-    flux_tile<T, kSkip>(X, tile, lane);
+    if (!flux_tile_form<T, kSkip, false, sizeof(T) == 8>(X, tile, lane))
+      flux_tile_guarded<T, kSkip>(clk, sb, bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra, tzero, tile, lane);
   }
   pdl_trigger();  // no tile left for this warp
   if (kSkip && lane == 0 && skipped)  // spread over the slots: one address would serialize the atomics
@@ -1240,7 +1285,7 @@ __global__ void __launch_bounds__(128, MINB) k_batch_flux(const MemberDev<T>* __
       s_ctx[threadIdx.x >> 5] = flux_ctx<T>(M.clk, M.sb, M.bed, M.n2, M.zone, M.rates, M.rows, M.cols, M.rb, M.dx,
                                             M.rdx, M.hextra);
     __syncwarp();
-    flux_tile<T, false, true>(s_ctx[threadIdx.x >> 5], tile - M.tile_begin, lane);
+    flux_tile_member<T>(s_ctx[threadIdx.x >> 5], tile - M.tile_begin, lane);
   }
 }
 
@@ -1417,7 +1462,7 @@ __device__ __forceinline__ void steps_flux_item(const MemberDev<T>* __restrict__
       s_ctx[warp] = flux_ctx<T>(M.clk, M.sb, M.bed, M.n2, M.zone, M.rates, M.rows, M.cols, M.rb, M.dx, M.rdx,
                                 M.hextra);
     __syncwarp();
-    flux_tile<T, false, true>(s_ctx[warp], tile - M.tile_begin, lane);
+    flux_tile_member<T>(s_ctx[warp], tile - M.tile_begin, lane);
   }
   __syncwarp();
   if (lane == 0) {
