@@ -169,20 +169,21 @@ __device__ __forceinline__ double recip_line(double b) {
   const double e = fma(-b, y0, 1.0);
   return recip_line(b, __fma_ru(y0, fma(e, e, e), y0));
 }
-// RN(a/b) from y = RN(1/b), up to the sign of a zero quotient.
+// RN(a/b) for b > 0 from y = RN(1/b).  The residual is taken negated, so that
+// an exact quotient adds a zero of the sign that keeps a zero's own sign.
 __device__ __forceinline__ double div_line(double a, double b, double y) {
   const double q0 = a * y;
-  return fma(fma(-q0, b, a), y, q0);
+  return fma(fma(q0, b, -a), -y, q0);
 }
 
 // True where the straight-line forms are exact on everything a face of this
-// cell computes: h is 0 or within 2^-300 .. 2^300 and the discharges are at
-// most 2^300 in magnitude.  A depth whose low word is all ones is left out
+// cell computes: h is 0 or within 2^-300 .. 2^100 and the discharges are at
+// most 2^100 in magnitude.  A depth whose low word is all ones is left out
 // (see recip_line; one depth in 2^32).  (Quotients of dividends below 2^-900 can then be
 // off by 2^-700 at most, far below the 1e-12 flush of the contributions they
 // enter.)  Tested on the high words: integer slots, which the FP64 tile has.
 __device__ __forceinline__ bool regular_cell(double h, double qx, double qy) {
-  constexpr uint32_t kLo = (1023u - 300u) << 20, kHi = (1023u + 300u) << 20;
+  constexpr uint32_t kLo = (1023u - 300u) << 20, kHi = (1023u + 100u) << 20;
   const uint32_t hh = (uint32_t)__double2hiint(h), hl = (uint32_t)__double2loint(h);
   const uint32_t ax = (uint32_t)__double2hiint(qx) & 0x7FFFFFFFu, ay = (uint32_t)__double2hiint(qy) & 0x7FFFFFFFu;
   const bool hok = (hh - kLo <= kHi - kLo && hl != 0xFFFFFFFFu) || (hh | hl) == 0u;
@@ -223,7 +224,9 @@ __device__ __forceinline__ float sr_add(float a, float b, uint32_t r, float* exa
   const float err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
   *exact_lo = err;
   if (err == 0.0f) return s;
-  const float t = nextafterf(s, err > 0.0f ? INFINITY : -INFINITY);
+  // the neighbour of s on the error's side, one step of its bits (s is not 0:
+  // a sum that rounds to 0 is exact)
+  const float t = __uint_as_float(__float_as_uint(s) + ((err > 0.0f) == (s > 0.0f) ? 1u : 0xFFFFFFFFu));
   const float u = (float)(r >> 8) * 0x1p-24f;
   return u * fabsf(t - s) < fabsf(err) ? t : s;
 }

@@ -140,9 +140,18 @@ struct RowParts {
   T an;          // FP32 form: |e0| + |n0|, for the noise test of the depth update
 };
 
-template <typename T>
+// A friction quotient's dividend that div_line takes: 0 (of either sign) or at
+// least 2^-900 (a transverse discharge can decay to any size).
+__device__ __forceinline__ bool line_dividend(double a) {
+  const uint32_t hi = (uint32_t)__double2hiint(a) & 0x7FFFFFFFu;
+  return hi >= (1023u - 900u) << 20 || (hi | (uint32_t)__double2loint(a)) == 0u;
+}
+
+// LINE (FP64): the straight-line forms; *odd is set where they do not hold.
+template <typename T, bool LINE>
 __device__ __forceinline__ void update_cell(const CellQ<T>& c, const RowParts<T>& p, T s0, T s1, T s2, T n2v, T dt,
-                                            T hextra, T& ho, T& qxo, T& qyo, double& clip, uint32_t rnd) {
+                                            T hextra, T& ho, T& qxo, T& qyo, double& clip, uint32_t rnd, bool& odd) {
+  constexpr bool L64 = LINE && sizeof(T) == 8;
   const T E12 = eps12<T>();
   const T G = T(kGravity);
   const T hn = c.h;
@@ -182,8 +191,30 @@ __device__ __forceinline__ void update_cell(const CellQ<T>& c, const RowParts<T>
     const T ry1 = p.w2 + s2;
     const T mx = c.qx - p.r1 - rx1;
     const T my = c.qy - p.r2 - ry1;
-    const T modM = dev_sqrt(mx * mx + my * my);
-    if (n2v > E12 && hn >= hextra && modM > E12) {
+    const T mm = mx * mx + my * my;
+    T modM;
+    if constexpr (L64) {  // a square below 1e-30 is no flow either way
+      odd |= ((uint32_t)__double2hiint(mm) & 0x7FFFFFFFu) > (1023u + 600u) << 20;
+      const double ms = mm > 1e-30 ? mm : 1e-30;
+      modM = sqrt_line(ms, rsqrt_line(ms));
+    } else {
+      modM = dev_sqrt(mm);
+    }
+    if (L64 && n2v > E12 && hn >= hextra && modM > E12) {
+      // dividend of the friction term: 2^-300 .. 2^200 keeps it, its
+      // reciprocal and its square root normal for every regular depth
+      const double num = dt * G * n2v * modM, den = hn * hn * dev_cbrt(hn);
+      odd |= (uint32_t)__double2hiint(num) - ((1023u - 300u) << 20) > (500u << 20);
+      const double tt = div_line(num, den, recip_line(den));
+      const double t4 = T(1) + T(4) * tt;
+      const double sq = sqrt_line(t4, rsqrt_line(t4));
+      const double rtt = recip_line(tt);
+      const double ax = T(-0.5) * (mx - mx * sq), ay = T(-0.5) * (my - my * sq);
+      qxij = div_line(ax, tt, rtt);
+      qyij = div_line(ay, tt, rtt);
+      if (!line_dividend(ax)) qxij = div_rare(ax, tt);
+      if (!line_dividend(ay)) qyij = div_rare(ay, tt);
+    } else if (!L64 && n2v > E12 && hn >= hextra && modM > E12) {
       const T tt = fdiv(dt * G * n2v * modM, hn * hn * dev_cbrt(hn));
       const T sq = dev_sqrt(T(1) + T(4) * tt);
       if (sizeof(T) == 8) {  // the reference's expression (kernels_state.h:86-96), bit for bit
@@ -390,7 +421,6 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, unsigned ti
 
   // raw values of the next row are loaded one iteration ahead
   T lh = T(0), lqx = T(0), lqy = T(0), lz = T(0);
-  double lzb = 0.0;
   auto fetch = [&](const FluxCtx<T>& Z, int r) {
     if (incol) {
       const size_t id = (size_t)r * Z.cols + c;
@@ -398,14 +428,20 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, unsigned ti
       lqx = Z.qxi[id];
       lqy = Z.qyi[id];
       lz = Z.bed.z[id];  // FP32 form: the offset from the base of the cell's tile
-      lzb = Z.bed.base_at(r, c);
     }
   };
   fetch(X, r0 - 1);
-  if (kLine) odd = !regular_cell(lh, lqx, lqy);
-  CellQ<T> prev = make_cell<T, kLine>(lh, lqx, lqy, lz, hextra, lzb);
+  if (kLine) odd = !regular_cell(lh, lqx, lqy) || !(hextra >= T(0x1p-100));  // bounds the velocities
+  CellQ<T> prev = make_cell<T, kLine>(lh, lqx, lqy, lz, hextra);
   if (r0 - 1 == 0 && owner) copy_ghost(X, 0);
   fetch(X, r0);
+  // FP32 form: base level of the bed tile of this lane's column minus that of
+  // the column to the west, for the tile row of row r (0 within a tile)
+  double dzx = 0.0;
+  auto base_step = [&](const FluxCtx<T>& Z, int r) {
+    if (sizeof(T) == 4 && incol && lane >= 1 && (c & 31) == 0) dzx = Z.bed.base_at(r, c) - Z.bed.base_at(r, c - 1);
+  };
+  base_step(X, r0);
   RowParts<T> pp;
   pp.r0 = pp.r1 = pp.r2 = pp.w0 = pp.w1 = pp.w2 = pp.an = T(0);
   T pn2 = T(0);  // Manning of the previous row's cell
@@ -415,7 +451,7 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, unsigned ti
     // held across the face computations
     const FluxCtx<T>& XL = kReload ? *launder_ptr(&X0) : X0;
     if (kLine) odd |= !regular_cell(lh, lqx, lqy);
-    const CellQ<T> cur = make_cell<T, kLine>(lh, lqx, lqy, lz, XL.K.hextra, lzb);
+    const CellQ<T> cur = make_cell<T, kLine>(lh, lqx, lqy, lz, XL.K.hextra);
     T cn2 = T(0);
     if (r <= r1) {
       if (upd) cn2 = XL.n2[(size_t)r * XL.cols + c];
@@ -423,7 +459,12 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, unsigned ti
     }
     FaceOut<T> Y;
     Y.a0 = Y.a1 = Y.a2 = Y.b0 = Y.b1 = Y.b2 = T(0);
-    if (upd) Y = face_flux<T, false, kLine>(cur, prev, XL.K);
+    double dzy = 0.0;  // the same across the north face, where a tile row begins
+    if (sizeof(T) == 4 && (r & 31) == 0) {
+      if (incol) dzy = XL.bed.base_at(r - 1, c) - XL.bed.base_at(r, c);
+      base_step(XL, r);
+    }
+    if (upd) Y = face_flux<T, false, kLine>(cur, prev, XL.K, dzy);
     if (r - 1 >= r0 && upd) {
       const FluxCtx<T>& XU = kReload ? *launder_ptr(&X0) : X0;
       const int cols = XU.cols;
@@ -431,8 +472,8 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, unsigned ti
       const size_t id = (size_t)(r - 1) * cols + c;
       T hn, qn, vn;
       double clip;
-      update_cell<T>(prev, pp, Y.b0, Y.b1, Y.b2, pn2, dt, hextra, hn, qn, vn, clip,
-                     cell_hash((uint32_t)id, 2u * XU.step));
+      update_cell<T, kLine>(prev, pp, Y.b0, Y.b1, Y.b2, pn2, dt, hextra, hn, qn, vn, clip,
+                            cell_hash((uint32_t)id, 2u * XU.step), odd);
       if (kAcct) {
         // Inflow through the south face of a cell of the last interior row
         // (the other boundary faces are counted where their parts are
@@ -442,7 +483,8 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, unsigned ti
       }
       if (XU.nroff > 0) {  // update_runoff (kernels.h:128-149)
         const T h0 = hn;
-        const T net = XU.rates[(size_t)XU.zone[id] * XU.roff_rows + XU.roff_row];
+        // with one zone its rate, without the zone map
+        const T net = XU.rates[(size_t)(XU.nroff > 1 ? XU.zone[id] : 0) * XU.roff_rows + XU.roff_row];
         if (sizeof(T) == 8) {
           hn += net * dt;
         } else if (net != T(0)) {
@@ -481,10 +523,9 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, unsigned ti
     left.sq = shfl_up1(cur.sq);
     left.u = shfl_up1(cur.u);
     left.v = shfl_up1(cur.v);
-    left.zb = sizeof(T) == 4 ? __shfl_up_sync(0xffffffffu, cur.zb, 1) : 0.0;
     FaceOut<T> Xf;
     Xf.a0 = Xf.a1 = Xf.a2 = Xf.b0 = Xf.b1 = Xf.b2 = T(0);
-    if (lane >= 1 && incol && c >= 1) Xf = face_flux<T, true, kLine>(left, cur, XL.K);
+    if (lane >= 1 && incol && c >= 1) Xf = face_flux<T, true, kLine>(left, cur, XL.K, dzx);
     const T e0 = shfl_down1(Xf.a0), e1 = shfl_down1(Xf.a1), e2 = shfl_down1(Xf.a2);
     if (kAcct && upd) {
       // Inflow through faces shared with ghost cells, in depth units.  The
