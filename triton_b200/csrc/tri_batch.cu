@@ -39,6 +39,7 @@ struct tri_batch {
   int32_t* h_seen = nullptr;  // pinned, one per chunk slot
   uint32_t ntiles = 0, nwet = 0;
   int rb = 8, variant = 1, flux_blocks = 1;
+  bool shape_set = false;  // tuned or set by the caller: the default no longer applies
   int2* d_src_items = nullptr;
   std::vector<int32_t> src_waves;
   int2* d_bc_items = nullptr;
@@ -178,6 +179,19 @@ int build_table(tri_batch* b) {
 }
 
 int rebuild(tri_batch* b) { return b->prec == TRI_FP64 ? build_table<double>(b) : build_table<float>(b); }
+
+// The default shape for the present members (batched steps compute every tile).
+void choose_shape(tri_batch* b) {
+  if (b->shape_set || b->members.empty()) return;
+  const FluxShape s = flux_shape(b->prec == TRI_FP64, 1.0, [&](int rb) {
+    int64_t n = 0;
+    for (const tri_domain* d : b->members)
+      n += (int64_t)((d->desc.cols - 2 + kStripCols - 1) / kStripCols) * ((d->desc.rows - 2 + rb - 1) / rb);
+    return n;
+  });
+  b->variant = s.variant;
+  b->rb = s.rb;
+}
 
 // (member, item) pairs of every member's conflict-free waves, wave by wave.
 int build_items(tri_batch* b) {
@@ -429,6 +443,7 @@ int tri_batch_create(int32_t nmembers, tri_domain* const* members, void* stream,
   cudaEventCreateWithFlags(&b->ev[1], cudaEventDisableTiming);
   // the members' own streams must be idle before the batch uses their memory
   for (tri_domain* d : b->members) cudaStreamSynchronize(d->stream);
+  choose_shape(b);
   if ((rc = rebuild(b)) != TRI_OK) return fail(rc);
   if ((rc = build_items(b)) != TRI_OK) return fail(rc);
   *out = b;
@@ -466,6 +481,7 @@ int tri_batch_set_members(tri_batch* b, int32_t nmembers, tri_domain* const* mem
   TRI_CUDA_TRY(cudaStreamSynchronize(b->stream));
   for (tri_domain* d : next) TRI_CUDA_TRY(cudaStreamSynchronize(d->stream));
   b->members = std::move(next);
+  choose_shape(b);
   if ((rc = rebuild(b)) != TRI_OK) return rc;
   return build_items(b);
 }
@@ -546,6 +562,7 @@ int tri_batch_set_tuning(tri_batch* b, int32_t variant, int32_t rows_per_tile) {
   TRI_CUDA_TRY(cudaStreamSynchronize(b->stream));
   b->variant = variant;
   b->rb = rows_per_tile;
+  b->shape_set = true;
   return rebuild(b);
 }
 
@@ -591,14 +608,14 @@ int tri_batch_autotune(tri_batch* b, int32_t trial_steps, tri_tuning* out) {
     }
     return TRI_OK;
   };
-  const int heights[3] = {4, 8, 16};
+  const int heights[] = {1, 2, 4, 8, 16, 32};
   double best = 1e300;
   int best_v = b->variant, best_rb = b->rb, ncand = 0;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   for (int v = 0; v < kFluxVariants && rc == TRI_OK; v++) {
-    for (int hi = 0; hi < 3 && rc == TRI_OK; hi++) {
+    for (size_t hi = 0; hi < sizeof(heights) / sizeof(heights[0]) && rc == TRI_OK; hi++) {
       b->variant = v;
       b->rb = heights[hi];
       rc = rebuild(b);
@@ -631,6 +648,7 @@ int tri_batch_autotune(tri_batch* b, int32_t trial_steps, tri_tuning* out) {
   cudaEventDestroy(e1);
   b->variant = best_v;
   b->rb = best_rb;
+  b->shape_set = true;
   int rc2 = rebuild(b);
   if (rc2 == TRI_OK && snaps.size() && snaps.back().buf) rc2 = restore();
   for (Snap& s : snaps)

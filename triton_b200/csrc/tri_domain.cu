@@ -307,21 +307,21 @@ void size_flux_grid(tri_domain* d) {
   d->flux_blocks = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)sms * per_sm, (tiles + 3) / 4));
 }
 
-// Default shape before any tuning: the register budget of 5 blocks per SM
-// in FP64 and 8 in FP32 (the fastest on watersheds of 1024^2 to 8192^2) and
-// the largest tile height, 32 down to 8, that still gives every warp of a
-// full wave about eight tiles.
+// Default shape before any tuning (flux_shape); a domain with runoff computes
+// every tile, one without about half of them.
 void choose_shape(tri_domain* d) {
-  const int rows = d->desc.rows - 2, cols = d->desc.cols - 2;
-  int sms = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t strips = (cols + kStripCols - 1) / kStripCols;
-  const int64_t warps = (int64_t)sms * 12;
-  int rb = 32;
-  while (rb > 8 && strips * ((rows + rb - 1) / rb) < 8 * warps) rb /= 2;
-  d->flux_variant = d->prec == TRI_FP64 ? 1 : 2;
-  d->rb = rb;
+  const int64_t rows = d->desc.rows - 2, strips = (d->desc.cols - 2 + kStripCols - 1) / kStripCols;
+  const FluxShape s = flux_shape(d->prec == TRI_FP64, d->nroff > 0 ? 1.0 : 0.5,
+                                 [&](int rb) { return strips * ((rows + rb - 1) / rb); });
+  d->flux_variant = s.variant;
+  d->rb = s.rb;
   size_flux_grid(d);
+}
+
+// The default shape again after the runoff came or went, unless the shape was
+// tuned or set; the tile flags and graphs are dropped by the caller.
+void rechoose_shape(tri_domain* d) {
+  if (!d->shape_set) choose_shape(d);
 }
 
 int launch_one_step(tri_domain* d) {
@@ -652,6 +652,7 @@ int tri_domain_set_runoff(tri_domain* d, int32_t nzones, int32_t nrows, const do
   if (nzones <= 0) {
     d->nroff = 0;
     d->mirror->nroff = 0;
+    rechoose_shape(d);
     return TRI_OK;
   }
   TRI_CHECK_ARG(times && rates && zone_of_cell, "null runoff table");
@@ -675,6 +676,7 @@ int tri_domain_set_runoff(tri_domain* d, int32_t nzones, int32_t nrows, const do
   d->mirror->nroff = nzones;
   d->mirror->roff_rows = nrows;
   d->mirror->roff_t = d->roff_t;
+  rechoose_shape(d);
   return TRI_OK;
 }
 
@@ -962,7 +964,7 @@ int tri_domain_autotune(tri_domain* d, int32_t trial_steps, tri_tuning* out) {
     return TRI_OK;
   };
   int rc = save_restore(true);
-  const int heights[3] = {8, 16, 32};
+  const int heights[] = {1, 2, 4, 8, 16, 32};
   double best = 1e300;
   int best_v = d->flux_variant, best_rb = d->rb, ncand = 0;
   cudaEvent_t e0, e1;
@@ -971,7 +973,7 @@ int tri_domain_autotune(tri_domain* d, int32_t trial_steps, tri_tuning* out) {
   const bool timing = d->timing;
   d->timing = false;
   for (int v = 0; v < kFluxVariants && rc == TRI_OK; v++) {
-    for (int hi = 0; hi < 3 && rc == TRI_OK; hi++) {
+    for (size_t hi = 0; hi < sizeof(heights) / sizeof(heights[0]) && rc == TRI_OK; hi++) {
       if (heights[hi] > std::max(8, d->desc.rows - 2)) continue;
       d->flux_variant = v;
       d->rb = heights[hi];
@@ -1008,6 +1010,7 @@ int tri_domain_autotune(tri_domain* d, int32_t trial_steps, tri_tuning* out) {
   d->timing = timing;
   d->flux_variant = best_v;
   d->rb = best_rb;
+  d->shape_set = true;
   size_flux_grid(d);
   drop_graph(d);
   int rc2 = save_restore(false);
@@ -1027,7 +1030,7 @@ int tri_domain_get_tuning(tri_domain* d, tri_tuning* out) {
   TRI_CHECK_ARG(d && out, "null argument");
   out->variant = d->flux_variant;
   out->rows_per_tile = d->rb;
-  out->candidates = kFluxVariants * 3;
+  out->candidates = kFluxVariants * 6;
   out->flux_blocks = d->flux_blocks;
   out->ms_per_step = d->tuned_ms;
   return TRI_OK;
@@ -1040,6 +1043,7 @@ int tri_domain_set_tuning(tri_domain* d, int32_t variant, int32_t rows_per_tile)
   TRI_CUDA_TRY(cudaStreamSynchronize(d->stream));
   d->flux_variant = variant;
   d->rb = rows_per_tile;
+  d->shape_set = true;
   size_flux_grid(d);
   drop_graph(d);
   d->tz_dirty = true;

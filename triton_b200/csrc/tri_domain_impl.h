@@ -64,6 +64,7 @@ struct tri_domain {
   int vol_blocks = 0;
   // launch shape of the flux kernel (tile height, register variant, grid)
   int rb = 16, flux_blocks = 1, flux_variant = 1;
+  bool shape_set = false;  // tuned or set by the caller: the defaults no longer apply
   // dry-tile flags of the flux kernel for the current tile shape: [2][tiles]
   // (tile holds only +0 in buffer 0 / 1) then [tiles] pinned.  Any change of
   // state, forcing or shape outside the step kernels marks them dirty; they

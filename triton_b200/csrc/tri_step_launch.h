@@ -31,8 +31,37 @@ template <>
 struct FluxBudget<float> {
   static constexpr int v0 = 5, v1 = 6, v2 = 8, v3 = 10, v4 = 12;
 };
-// the variant untuned domains and batches start from
-constexpr int kFluxDefaultVariant = 1;
+
+// Default launch shape of the flux kernel: register budget and tile height.
+// tiles(rb): warp tiles of height rb in all; share: the part of them that is
+// computed in a step (the others are dry and skipped).  What decides is how
+// many tiles there are for `slots` = 16 resident warps per SM:
+//  - few (a small grid): a launch lasts as long as one tile, whose rows are a
+//    serial chain (about 2.5 us each), so the lowest height whose tiles are
+//    resident at once (rain on 256^2, FP64: 16 us with 1 row, 27 with 8; 512^2:
+//    26 with 4, 33 with 8);
+//  - many: the tallest that leaves a warp about four tiles, since a tile
+//    repeats one row of faces above it (rain on 2048^2, FP64: 199 us with 12
+//    rows, 214 with 4; FP32 4096^2: 442 with 32, 468 with 6) and the last
+//    round of tiles idles half the warps.
+// FP64 takes the largest register budget (no spills; more warps are not
+// faster: bowl 2048^2 97.4 us at 4 blocks per SM, 100.0 at 5, 112 at 6).  FP32
+// is bound by issue and takes 8 blocks per SM (rain 2048^2 129 us, 137 at 5),
+// but where one round holds all tiles the largest budget (bowl 256^2 12.6 us,
+// 14.0).
+struct FluxShape {
+  int variant, rb;
+};
+template <typename F>
+FluxShape flux_shape(bool fp64, double share, F tiles) {
+  constexpr double slots = 148 * 16;
+  for (int rb = 1; rb <= 4; rb++)
+    if (share * (double)tiles(rb) <= slots) return {0, rb};
+  int best = 4;
+  for (int rb : {6, 8, 12, 16, 24, 32})
+    if (share * (double)tiles(rb) >= 4 * slots) best = rb;
+  return {fp64 ? 0 : 2, best};
+}
 // rows per block of the staged wet-dry/dt kernel (its shared-memory tile),
 // and output rows per group of its copies (each group on its own mbarrier)
 template <typename T>

@@ -31,9 +31,6 @@ import numpy as np
 from .batch import Batch
 from .domain import Domain
 
-# Default launch shapes of the batched flux kernel (variant, rows per tile).
-SHAPES = {"fp64": (1, 16), "fp32": (1, 16)}
-
 
 @dataclass
 class Request:
@@ -71,7 +68,7 @@ class Server:
         self.budget = float(hbm_budget)
         self.chunk = int(chunk_steps)
         self.max_members = int(max_members)
-        self.shapes = dict(SHAPES, **(shapes or {}))
+        self.shapes = dict(shapes or {})  # launch shapes (variant, rows per tile); else the batch's own rule
         self.used = 0
         self.peak_used = 0
         self.batches: dict[str, Batch] = {}
@@ -137,7 +134,8 @@ class Server:
             if not doms:
                 return
             b = self.batches[prec] = Batch(doms)
-            b.set_shape(*self.shapes[prec])
+            if prec in self.shapes:
+                b.set_shape(*self.shapes[prec])
         else:
             b.set_members(doms)
 
