@@ -119,3 +119,54 @@ def test_extreme_depths_bit_exact(value, shape):
         sc.qx[r, c] = sc.qy[r, c] = 0.0
     steps, _ = run_lockstep(sc, exact=True, max_events=1, chunk=6)
     assert 0 < steps <= 6  # an observation event may come first
+
+
+@pytest.mark.parametrize("rows,cols,open_b", [(5, 31, 0), (33, 61, 1), (64, 30, 1), (40, 92, 0)])
+def test_tile_heights_match_oracle(rows, cols, open_b):
+    """Every tile height gives the oracle's bits: tiles of one row, heights that
+    leave a remainder, one tile over the whole height; strips of 30 columns with
+    1, 30 and 32 columns left; sources (two in one cell), runoff, zero-gradient
+    edges."""
+    from tests._harness import compare_fields, domain_bookkeeping, oracle_bookkeeping, oracle_from_scenario
+    from triton_b200 import scenarios
+    for variant, rb in ((0, 1), (1, 3), (2, 7), (0, 32), (0, 100)):
+        sc = scenarios.mixed(rows=rows, cols=cols, seed=41, open_boundaries=open_b, friction=False, with_extbc=False,
+                             duration=2.0)
+        o, d = oracle_from_scenario(sc), sc.to_domain()
+        try:
+            d.set_shape(variant, rb)
+            for _ in range(4):
+                n1, e1 = o.advance(10 ** 6)
+                n2, e2 = d.advance(10 ** 6)
+                assert (n1, e1) == (n2, e2)
+                assert d.get_clock().simtime == o.s.simtime
+                compare_fields(o, d, True, sc.hextra, where=f"height {rb}: ")
+                oracle_bookkeeping(o, e1)
+                domain_bookkeeping(d, e2)
+        finally:
+            d.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_tile_heights_agree_with_boundary_cells(precision):
+    """External boundary cells of every type, friction, arrival tracking: the
+    default height, tiles of one row and tall tiles give the same bits (a
+    corner's ghosts belong to its tile at any height)."""
+    from triton_b200 import scenarios
+    got = []
+    for rb in (0, 1, 4, 40):
+        sc = scenarios.mixed(rows=37, cols=65, seed=43, friction=True, duration=5.0)
+        sc.z[1:-1, 1:-1] += 700.0  # FP32: bed levels far from their bases' zero
+        d = sc.to_domain(precision)
+        try:
+            if rb:
+                d.set_shape(0, rb)
+            d.track_arrival(0.3)
+            d.set_clock(sim_duration=1e300, print_interval=1e300, time_series=0, it_print=0)
+            assert d.advance(61)[0] == 61
+            got.append([d.download(f) for f in ("h", "qx", "qy", "maxh")] + [d.arrival(), np.array(d.get_clock().simtime)])
+        finally:
+            d.close()
+    for other in got[1:]:
+        for a, b in zip(got[0], other):
+            assert np.array_equal(a, b)

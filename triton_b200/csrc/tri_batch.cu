@@ -40,12 +40,12 @@ struct tri_batch {
   uint32_t ntiles = 0, nwet = 0;
   int rb = 8, variant = 1, flux_blocks = 1;
   bool shape_set = false;  // tuned or set by the caller: the default no longer applies
-  int2* d_src_items = nullptr;
-  std::vector<int32_t> src_waves;
-  int2* d_bc_items = nullptr;
-  std::vector<int32_t> bc_waves;
-  int32_t* d_open = nullptr;  // members with open edges
-  int n_open = 0, open_dim = 0;
+  // graph mode: member of every post kernel block, tile flags ([tiles], then
+  // [tiles] pinned), the tiles' wave speeds, their forcing
+  int32_t* d_post_mem = nullptr;
+  uint32_t npost = 0;
+  int32_t* d_tlists = nullptr;
+  TileForcing tf{};
   // single-launch mode (TRI_BATCH_SINGLE_LAUNCH): progress counters per
   // member, the members' forcing wave offsets, resident grid
   int mode = TRI_BATCH_GRAPHS;
@@ -97,16 +97,16 @@ MemberDev<T> member_dev(tri_domain* d, int rb, uint32_t& tiles, uint32_t& wet) {
   m.wet_nbx = (uint32_t)((a.cols + kWetCols - 1) / kWetCols);
   m.wet_begin = wet;
   wet += m.wet_nbx * (uint32_t)((a.rows + kStageBand<T> - 1) / kStageBand<T>);
-  m.nsrc = a.nsrc;
-  m.src_cells = a.src_cells;
-  m.hyg_t = a.hyg_t;
-  m.hyg_v = (const T*)a.hyg_v;
-  m.bc_cells = a.bc_cells;
-  m.bc_types = a.bc_types;
-  m.bc_start = a.bc_start;
-  m.bc_nrows = a.bc_nrows;
-  m.bc_v1 = (const T*)a.bc_v1;
-  m.bc_v2 = (const T*)a.bc_v2;
+  m.f.nsrc = a.nsrc;
+  m.f.src_cells = a.src_cells;
+  m.f.hyg_t = a.hyg_t;
+  m.f.hyg_v = (const T*)a.hyg_v;
+  m.f.bc_cells = a.bc_cells;
+  m.f.bc_types = a.bc_types;
+  m.f.bc_start = a.bc_start;
+  m.f.bc_nrows = a.bc_nrows;
+  m.f.bc_v1 = (const T*)a.bc_v1;
+  m.f.bc_v2 = (const T*)a.bc_v2;
   m.wet_count = wet - m.wet_begin;
   m.src_order = d->nsrc > 0 ? d->src_order : nullptr;
   m.src_nw = d->nsrc > 0 ? (int)d->src_waves.size() - 1 : 0;
@@ -123,7 +123,23 @@ void drop_graph(tri_batch* b) {
   b->graph_steps = 0;
 }
 
-// Member table, tile and block counts, grid of the flux kernel.
+void free_tables(tri_batch* b) {
+  for (void** p : {&b->d_mem, (void**)&b->d_tile_mem, (void**)&b->d_wet_mem, (void**)&b->d_prog, (void**)&b->d_woff,
+                   (void**)&b->d_post_mem, (void**)&b->d_tlists}) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
+}
+
+// A new device array holding v (at least one element).
+template <typename V>
+int upload(const std::vector<V>& v, V** out) {
+  TRI_CUDA_TRY(cudaMalloc((void**)out, std::max<size_t>(v.size(), 1) * sizeof(V)));
+  if (!v.empty()) TRI_CUDA_TRY(cudaMemcpy(*out, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice));
+  return TRI_OK;
+}
+
+// Member table, tile and block counts, tile lists, grid of the flux kernel.
 template <typename T>
 int build_table(tri_batch* b) {
   std::vector<MemberDev<T>> tab;
@@ -131,11 +147,7 @@ int build_table(tri_batch* b) {
   for (tri_domain* d : b->members) tab.push_back(member_dev<T>(d, b->rb, tiles, wet));
   b->ntiles = tiles;
   b->nwet = wet;
-  for (void** p : {&b->d_mem, (void**)&b->d_tile_mem, (void**)&b->d_wet_mem, (void**)&b->d_prog,
-                   (void**)&b->d_woff}) {
-    if (*p) cudaFree(*p);
-    *p = nullptr;
-  }
+  free_tables(b);
   drop_graph(b);
   if (tab.empty()) return TRI_OK;
   // single-launch mode: every member's wave offsets in one buffer, progress counters
@@ -157,6 +169,20 @@ int build_table(tri_batch* b) {
   }
   TRI_CUDA_TRY(cudaMalloc((void**)&b->d_prog, tab.size() * sizeof(MemberProgress)));
   b->steps_grid = batch_steps_grid<T>(b->variant);
+  // post kernel blocks and forcing of all members' tiles
+  std::vector<int32_t> pm;
+  TileLists lists;
+  for (size_t m = 0; m < tab.size(); m++) {
+    tab[m].post_begin = (uint32_t)pm.size();
+    tab[m].post_count = post_blocks(tab[m].tile_end - tab[m].tile_begin, tiles, PostBlocks<T>::batch);
+    pm.insert(pm.end(), tab[m].post_count, (int32_t)m);
+    append_tile_lists(b->members[m], b->rb, (int32_t)tab[m].tile_begin, lists);
+  }
+  b->npost = (uint32_t)pm.size();
+  int rc = upload(pm, &b->d_post_mem);
+  if (rc == TRI_OK) rc = upload(lists.flat(), &b->d_tlists);
+  if (rc != TRI_OK) return rc;
+  b->tf = lists.at(b->d_tlists);
   std::vector<int32_t> tm(tiles), wm(wet);
   for (size_t m = 0; m < tab.size(); m++) {
     std::fill(tm.begin() + tab[m].tile_begin, tm.begin() + tab[m].tile_end, (int32_t)m);
@@ -193,58 +219,6 @@ void choose_shape(tri_batch* b) {
   b->rb = s.rb;
 }
 
-// (member, item) pairs of every member's conflict-free waves, wave by wave.
-int build_items(tri_batch* b) {
-  auto gather = [&](bool src, int2** dptr, std::vector<int32_t>& waves) -> int {
-    std::vector<std::vector<int2>> per;
-    for (size_t m = 0; m < b->members.size(); m++) {
-      tri_domain* d = b->members[m];
-      const std::vector<int32_t>& w = src ? d->src_waves : d->bc_waves;
-      const std::vector<int32_t>& o = src ? d->src_order_host : d->bc_order_host;
-      const int n = src ? d->nsrc : d->nbc;
-      if (n <= 0 || w.size() < 2) continue;
-      for (size_t k = 0; k + 1 < w.size(); k++) {
-        if (per.size() <= k) per.resize(k + 1);
-        for (int j = w[k]; j < w[k + 1]; j++) per[k].push_back(make_int2((int)m, o[j]));
-      }
-    }
-    std::vector<int2> flat;
-    waves.assign(1, 0);
-    for (auto& v : per) {
-      flat.insert(flat.end(), v.begin(), v.end());
-      waves.push_back((int32_t)flat.size());
-    }
-    if (*dptr) cudaFree(*dptr);
-    *dptr = nullptr;
-    if (!flat.empty()) {
-      TRI_CUDA_TRY(cudaMalloc((void**)dptr, flat.size() * sizeof(int2)));
-      TRI_CUDA_TRY(cudaMemcpy(*dptr, flat.data(), flat.size() * sizeof(int2), cudaMemcpyHostToDevice));
-    }
-    return TRI_OK;
-  };
-  int rc = gather(true, &b->d_src_items, b->src_waves);
-  if (rc == TRI_OK) rc = gather(false, &b->d_bc_items, b->bc_waves);
-  if (rc != TRI_OK) return rc;
-  // open-boundary members: ghost copies after the sources, before the
-  // external-boundary cells, as in the single-domain step
-  std::vector<int32_t> open;
-  b->open_dim = 0;
-  for (size_t m = 0; m < b->members.size(); m++) {
-    const tri_grid_desc& g = b->members[m]->desc;
-    if (!g.open_boundaries) continue;
-    open.push_back((int32_t)m);
-    b->open_dim = std::max(b->open_dim, std::max(g.rows, g.cols));
-  }
-  if (b->d_open) cudaFree(b->d_open);
-  b->d_open = nullptr;
-  b->n_open = (int)open.size();
-  if (!open.empty()) {
-    TRI_CUDA_TRY(cudaMalloc((void**)&b->d_open, open.size() * sizeof(int32_t)));
-    TRI_CUDA_TRY(cudaMemcpy(b->d_open, open.data(), open.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-  }
-  return TRI_OK;
-}
-
 BatchArgs batch_args(tri_batch* b) {
   BatchArgs a{};
   a.mem = b->d_mem;
@@ -256,15 +230,9 @@ BatchArgs batch_args(tri_batch* b) {
   a.nwet_blocks = b->nwet;
   a.flux_blocks = b->flux_blocks;
   a.flux_variant = b->variant;
-  a.src_items = b->d_src_items;
-  a.src_waves = b->src_waves.data();
-  a.n_src_waves = (int)b->src_waves.size() - 1;
-  a.bc_items = b->d_bc_items;
-  a.bc_waves = b->bc_waves.data();
-  a.n_bc_waves = (int)b->bc_waves.size() - 1;
-  a.open_members = b->d_open;
-  a.n_open = b->n_open;
-  a.open_dim = b->open_dim;
+  a.post_member = b->d_post_mem;
+  a.npost_blocks = b->npost;
+  a.tf = b->tf;
   return a;
 }
 
@@ -287,6 +255,14 @@ int launch_batch_single(tri_batch* b, int n) {
     n -= k;
   }
   return TRI_OK;
+}
+
+// Starts the members' first step of an advance (the single-launch kernel does
+// it itself).
+int launch_clocks(tri_batch* b) {
+  if (b->mode == TRI_BATCH_SINGLE_LAUNCH) return TRI_OK;
+  const BatchArgs a = batch_args(b);
+  return b->prec == TRI_FP64 ? launch_batch_clock<double>(a, b->stream) : launch_batch_clock<float>(a, b->stream);
 }
 
 int launch_batch(tri_batch* b, int n) {
@@ -323,12 +299,13 @@ int launch_batch(tri_batch* b, int n) {
   return TRI_OK;
 }
 
-// Prepares every member's clock for a batched advance (members at or past
+// Prepares every member's clock for a batched advance of at most 'limit'
+// steps (members at or past
 // their end stay halted for the whole call); counts the members that step.
 // Clocks go to the device on the batch stream, ahead of the batched launches;
 // a member without a valid CFL dt (new, or state uploaded) gets it first on
 // its own stream.
-int prepare_members(tri_batch* b, int* runnable) {
+int prepare_members(tri_batch* b, int limit, int* runnable) {
   *runnable = 0;
   for (tri_domain* d : b->members) {
     DevClock* m = d->mirror;
@@ -338,6 +315,8 @@ int prepare_members(tri_batch* b, int* runnable) {
     m->events = 0;
     m->steps = 0;
     m->status = 0;
+    m->limit = limit;
+    m->post_done = 0;
     const bool need_dt = live && !d->dt_valid && !m->time_increment_fixed;
     if (need_dt) {
       m->dt_key[m->rd] = kDtKeyInf;
@@ -445,7 +424,6 @@ int tri_batch_create(int32_t nmembers, tri_domain* const* members, void* stream,
   for (tri_domain* d : b->members) cudaStreamSynchronize(d->stream);
   choose_shape(b);
   if ((rc = rebuild(b)) != TRI_OK) return fail(rc);
-  if ((rc = build_items(b)) != TRI_OK) return fail(rc);
   *out = b;
   return TRI_OK;
 }
@@ -454,17 +432,10 @@ int tri_batch_destroy(tri_batch* b) {
   if (!b) return TRI_OK;
   if (b->stream) cudaStreamSynchronize(b->stream);
   drop_graph(b);
-  if (b->d_mem) cudaFree(b->d_mem);
-  if (b->d_tile_mem) cudaFree(b->d_tile_mem);
-  if (b->d_wet_mem) cudaFree(b->d_wet_mem);
+  free_tables(b);
   if (b->d_ctl) cudaFree(b->d_ctl);
   if (b->h_ctl) cudaFreeHost(b->h_ctl);
   if (b->h_seen) cudaFreeHost(b->h_seen);
-  if (b->d_src_items) cudaFree(b->d_src_items);
-  if (b->d_bc_items) cudaFree(b->d_bc_items);
-  if (b->d_open) cudaFree(b->d_open);
-  if (b->d_prog) cudaFree(b->d_prog);
-  if (b->d_woff) cudaFree(b->d_woff);
   for (int i = 0; i < 2; i++)
     if (b->ev[i]) cudaEventDestroy(b->ev[i]);
   if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
@@ -482,8 +453,7 @@ int tri_batch_set_members(tri_batch* b, int32_t nmembers, tri_domain* const* mem
   for (tri_domain* d : next) TRI_CUDA_TRY(cudaStreamSynchronize(d->stream));
   b->members = std::move(next);
   choose_shape(b);
-  if ((rc = rebuild(b)) != TRI_OK) return rc;
-  return build_items(b);
+  return rebuild(b);
 }
 
 int tri_batch_advance(tri_batch* b, int32_t max_steps, tri_batch_progress* p) {
@@ -491,10 +461,11 @@ int tri_batch_advance(tri_batch* b, int32_t max_steps, tri_batch_progress* p) {
   if (b->launched) return set_error(TRI_E_STATE, "batch has launched steps; call tri_batch_wait first");
   TRI_CHECK_ARG(max_steps >= 0, "max_steps must be >= 0");
   int runnable = 0;
-  int rc = prepare_members(b, &runnable);
+  int rc = prepare_members(b, max_steps, &runnable);
   if (rc != TRI_OK) return rc;
   if (runnable > 0 && max_steps > 0) {
     if ((rc = reset_ctl(b)) != TRI_OK) return rc;
+    if ((rc = launch_clocks(b)) != TRI_OK) return rc;
     // chunks of 8 batched steps (32 in single-launch mode), two in flight;
     // stop once every runnable member has raised an event
     const int chunk = b->mode == TRI_BATCH_SINGLE_LAUNCH ? 32 : 8;
@@ -523,10 +494,11 @@ int tri_batch_launch(tri_batch* b, int32_t steps) {
   TRI_CHECK_ARG(steps >= 0, "steps must be >= 0");
   if (b->launched) return set_error(TRI_E_STATE, "batch has launched steps; call tri_batch_wait first");
   int runnable = 0;
-  int rc = prepare_members(b, &runnable);
+  int rc = prepare_members(b, steps, &runnable);
   if (rc != TRI_OK) return rc;
   if (runnable > 0 && steps > 0) {
     if ((rc = reset_ctl(b)) != TRI_OK) return rc;
+    if ((rc = launch_clocks(b)) != TRI_OK) return rc;
     if ((rc = launch_batch(b, steps)) != TRI_OK) return rc;
   }
   b->launched = true;
@@ -626,8 +598,9 @@ int tri_batch_autotune(tri_batch* b, int32_t trial_steps, tri_tuning* out) {
         d->mirror->time_series = 0;
       }
       int runnable = 0;
-      if (rc == TRI_OK) rc = prepare_members(b, &runnable);
+      if (rc == TRI_OK) rc = prepare_members(b, INT32_MAX, &runnable);
       if (rc == TRI_OK) rc = reset_ctl(b);
+      if (rc == TRI_OK) rc = launch_clocks(b);
       if (rc == TRI_OK) rc = launch_batch(b, 2);  // warm-up, also builds the graph
       cudaEventRecord(e0, b->stream);
       if (rc == TRI_OK) rc = launch_batch(b, trial_steps);

@@ -217,76 +217,70 @@ StepArgs step_args(tri_domain* d) {
   a.dx = d->desc.cell_size;
   a.courant = d->desc.courant;
   a.hextra = d->desc.hextra;
-  a.open_boundaries = d->desc.open_boundaries;
   a.nsrc = d->nsrc;
   a.src_cells = d->src_cells;
-  a.src_order = d->src_order;
   a.hyg_t = d->hyg_t;
   a.hyg_v = d->hyg_v;
-  a.src_waves = d->src_waves.data();
-  a.n_src_waves = d->src_waves.empty() ? 0 : (int)d->src_waves.size() - 1;
-  a.nbc = d->nbc;
   a.bc_cells = d->bc_cells;
   a.bc_types = d->bc_types;
   a.bc_start = d->bc_start;
   a.bc_nrows = d->bc_nrows;
-  a.bc_order = d->bc_order;
   a.bc_v1 = d->bc_v1;
   a.bc_v2 = d->bc_v2;
-  a.bc_waves = d->bc_waves.data();
-  a.n_bc_waves = d->bc_waves.empty() ? 0 : (int)d->bc_waves.size() - 1;
   a.arrival = d->arrival;
   a.arrival_depth = d->arrival_depth;
-  a.tzero = d->tz_on ? d->tzero : nullptr;
-  a.tzero_wet = (d->arrival == nullptr || d->arrival_depth >= 0.0f) ? a.tzero : nullptr;
-  a.maxh_neg = d->maxh_neg;
+  a.tflag = d->tflag;
+  a.ntiles = (uint32_t)d->tz_tiles;
+  a.tf = d->tf;
+  a.open_boundaries = d->desc.open_boundaries;
+  a.skip_dry = d->nroff == 0;  // runoff reaches every cell
   return a;
 }
 
-// Resets the dry-tile flags of the flux kernel for the current tile shape
-// (nothing is known to be zero, so the next two steps compute every tile)
-// and marks the tiles that must never be skipped: those holding a source or
-// an external boundary cell, and the edge tiles when the open boundaries
-// rewrite the ghost ring.  Runoff reaches every cell, so a domain with runoff
-// computes every tile.  Called outside graph capture, before steps.
-int reset_tiles(tri_domain* d) {
-  const int rows = d->desc.rows, cols = d->desc.cols;
-  const int64_t ns = (cols - 2 + kStripCols - 1) / kStripCols, nty = (rows - 2 + d->rb - 1) / d->rb;
-  const int64_t nt = ns * nty;
-  d->tz_dirty = false;
-  d->tz_on = d->nroff == 0;
-  if (!d->tz_on) return TRI_OK;
-  if (nt > d->tz_cap) {
-    drop_graph(d);  // the graphs hold the old flag pointer
-    free_devp(d->tzero);
-    d->tz_cap = 0;
-    if (cudaMalloc((void**)&d->tzero, 3 * (size_t)nt) != cudaSuccess) {
-      d->tz_on = false;
-      return set_error(TRI_E_NOMEM, "cudaMalloc of %lld tile flags failed", (long long)(3 * nt));
-    }
-    d->tz_cap = nt;
+int64_t flux_tiles(const tri_domain* d, int rb) {
+  return (int64_t)((d->desc.cols - 2 + kStripCols - 1) / kStripCols) * ((d->desc.rows - 2 + rb - 1) / rb);
+}
+
+// Pins and forcing lists of the flux tiles for the current shape and forcing.
+// Pinned tiles are those that are written into after their flux update: they
+// hold a source or an external boundary cell, or lie on an open edge.  They
+// are never skipped nor flagged.  Called outside graph capture, before steps.
+int build_tile_lists(tri_domain* d) {
+  const int64_t nt = flux_tiles(d, d->rb);
+  TileLists lists;
+  append_tile_lists(d, d->rb, 0, lists);
+  std::vector<uint8_t> pin((size_t)nt, 0);
+  for (int32_t t : lists.tiles) pin[(size_t)t] = 1;
+  drop_graph(d);  // the graphs hold the old pointers and lists
+  TRI_CUDA_TRY(cudaStreamSynchronize(d->stream));
+  if (nt != d->tz_tiles) {
+    free_devp(d->tflag);
+      d->tz_tiles = 0;
+    if (cudaMalloc((void**)&d->tflag, 3 * (size_t)nt) != cudaSuccess)
+      return set_error(TRI_E_NOMEM, "cudaMalloc of %lld tile flags failed", (long long)nt);
+    d->tz_tiles = nt;
   }
-  if (nt != d->tz_tiles) drop_graph(d);  // the pinned table moved
-  d->tz_tiles = nt;
-  std::vector<uint8_t>& pin = d->tz_pin_host;
-  pin.assign((size_t)nt, 0);
-  auto pin_cell = [&](int64_t id) {
-    const int r = (int)(id / cols), c = (int)(id % cols);
-    const int64_t ry = std::min<int64_t>(std::max(r - 1, 0) / d->rb, nty - 1);
-    const int64_t sx = std::min<int64_t>(std::max(c - 1, 0) / kStripCols, ns - 1);
-    pin[(size_t)(ry * ns + sx)] = 1;
-  };
-  if (d->nsrc > 0)
-    for (int32_t id : d->src_cells_host) pin_cell(id);
-  if (d->nbc > 0)
-    for (int32_t id : d->bc_cells_host) pin_cell(id);
-  if (d->desc.open_boundaries)
-    for (int64_t ry = 0; ry < nty; ry++)
-      for (int64_t sx = 0; sx < ns; sx++)
-        if (ry == 0 || ry == nty - 1 || sx == 0 || sx == ns - 1) pin[(size_t)(ry * ns + sx)] = 1;
-  TRI_CUDA_TRY(cudaMemsetAsync(d->tzero, 0, 2 * (size_t)nt, d->stream));
-  TRI_CUDA_TRY(cudaMemcpyAsync(d->tzero + 2 * nt, pin.data(), (size_t)nt, cudaMemcpyHostToDevice, d->stream));
-  TRI_CUDA_TRY(cudaStreamSynchronize(d->stream));  // 'pin' may be reassigned before the copy ran
+  free_devp(d->tlists);
+  const std::vector<int32_t> flat = lists.flat();
+  TRI_CUDA_TRY(cudaMalloc((void**)&d->tlists, flat.size() * sizeof(int32_t)));
+  TRI_CUDA_TRY(cudaMemcpyAsync(d->tlists, flat.data(), flat.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
+                               d->stream));
+  d->tf = lists.at(d->tlists);
+  TRI_CUDA_TRY(cudaMemcpyAsync(d->tflag + 2 * nt, pin.data(), (size_t)nt, cudaMemcpyHostToDevice, d->stream));
+  TRI_CUDA_TRY(cudaStreamSynchronize(d->stream));
+  d->tile_lists_dirty = false;
+  return TRI_OK;
+}
+
+// Resets the tile flags: nothing is known to be zero or wet, so the next two
+// steps compute every tile.
+int reset_tiles(tri_domain* d) {
+  if (d->tile_lists_dirty) {
+    const int rc = build_tile_lists(d);
+    if (rc != TRI_OK) return rc;
+  }
+  d->tz_dirty = false;
+  TRI_CUDA_TRY(cudaMemsetAsync(d->tflag, 0, 2 * (size_t)d->tz_tiles, d->stream));
   return TRI_OK;
 }
 
@@ -315,6 +309,7 @@ void choose_shape(tri_domain* d) {
                                  [&](int rb) { return strips * ((rows + rb - 1) / rb); });
   d->flux_variant = s.variant;
   d->rb = s.rb;
+  d->tile_lists_dirty = true;
   size_flux_grid(d);
 }
 
@@ -428,6 +423,44 @@ int domain_push_clock(tri_domain* d) { return push_clock(d); }
 int domain_pull_clock(tri_domain* d) { return pull_clock(d); }
 int domain_launch_dt(tri_domain* d) { return launch_dt(d); }
 StepArgs domain_step_args(tri_domain* d) { return step_args(d); }
+
+void append_tile_lists(const tri_domain* d, int rb, int32_t first, TileLists& out) {
+  const int cols = d->desc.cols;
+  const int64_t ns = (cols - 2 + kStripCols - 1) / kStripCols, nt = flux_tiles(d, rb), nty = nt / ns;
+  struct Item {
+    int64_t tile;
+    int group;  // sources before boundary cells, each in its waves
+    int32_t item;
+  };
+  std::vector<Item> all;
+  auto add = [&](const std::vector<int32_t>& waves, const std::vector<int32_t>& order,
+                 const std::vector<int32_t>& cells, bool src) {
+    for (size_t w = 0; w + 1 < waves.size(); w++)
+      for (int32_t j = waves[w]; j < waves[w + 1]; j++) {
+        const int32_t k = order[j], id = cells[k];
+        const int64_t ry = (id / cols - 1) / rb, sx = (id % cols - 1) / kStripCols;  // interior cells
+        all.push_back({ry * ns + sx, (int)(2 * w) + (src ? 0 : 1), src ? k : -1 - k});
+      }
+  };
+  if (d->nsrc > 0) add(d->src_waves, d->src_order_host, d->src_cells_host, true);
+  if (d->nbc > 0) add(d->bc_waves, d->bc_order_host, d->bc_cells_host, false);
+  std::stable_sort(all.begin(), all.end(), [](const Item& a, const Item& b) {
+    if (a.tile != b.tile) return a.tile < b.tile;
+    return (a.item < 0) != (b.item < 0) ? b.item < 0 : a.group < b.group;
+  });
+  size_t i = 0;
+  for (int64_t t = 0; t < nt; t++) {
+    const int64_t ry = t / ns, sx = t % ns;
+    const bool edge = d->desc.open_boundaries && (ry == 0 || ry == nty - 1 || sx == 0 || sx == ns - 1);
+    if (!edge && (i == all.size() || all[i].tile != t)) continue;
+    out.tiles.push_back(first + (int32_t)t);
+    out.group_of.push_back((int32_t)out.item_of.size());
+    for (size_t j = i; i < all.size() && all[i].tile == t; i++) {
+      if (i == j || all[i - 1].group != all[i].group) out.item_of.push_back((int32_t)out.items.size());
+      out.items.push_back(all[i].item);
+    }
+  }
+}
 }  // namespace tri
 
 extern "C" {
@@ -498,6 +531,7 @@ int tri_domain_create(const tri_grid_desc* desc, void* stream, tri_domain** out)
   if (cudaMalloc((void**)&d->maxh_neg, sizeof(int32_t)) != cudaSuccess)
     return fail(set_error(TRI_E_CUDA, "flag allocation failed"));
   cudaMemsetAsync(d->maxh_neg, 0, sizeof(int32_t), d->stream);
+  d->mirror->maxh_neg = d->maxh_neg;
   d->vol_blocks = 296;
   if (cudaMalloc((void**)&d->vol_part, d->vol_blocks * sizeof(double)) != cudaSuccess ||
       cudaMalloc((void**)&d->vol_out, sizeof(double)) != cudaSuccess)
@@ -518,7 +552,8 @@ int tri_domain_destroy(tri_domain* d) {
   if (!d) return TRI_OK;
   if (d->stream) cudaStreamSynchronize(d->stream);
   drop_graph(d);
-  free_devp(d->tzero);
+  free_devp(d->tflag);
+  free_devp(d->tlists);
   free_devp(d->maxh_neg);
   for (int i = 0; i < 2; i++) {
     free_dev(d->h[i]);
@@ -648,7 +683,7 @@ int tri_domain_set_runoff(tri_domain* d, int32_t nzones, int32_t nrows, const do
                           const int32_t* zone_of_cell, int64_t ncells) {
   TRI_CHECK_ARG(d, "null domain");
   drop_graph(d);
-  d->tz_dirty = true;
+  d->tz_dirty = d->tile_lists_dirty = true;
   if (nzones <= 0) {
     d->nroff = 0;
     d->mirror->nroff = 0;
@@ -684,7 +719,7 @@ int tri_domain_set_sources(tri_domain* d, int32_t nsrc, const int32_t* cells, in
                            const double* flows) {
   TRI_CHECK_ARG(d, "null domain");
   drop_graph(d);
-  d->tz_dirty = true;
+  d->tz_dirty = d->tile_lists_dirty = true;
   if (nsrc <= 0) {
     d->nsrc = 0;
     d->mirror->nsrc = 0;
@@ -725,7 +760,7 @@ int tri_domain_set_extbc(tri_domain* d, int32_t ncells, const int32_t* cells, co
                          const double* var2) {
   TRI_CHECK_ARG(d, "null domain");
   drop_graph(d);
-  d->tz_dirty = true;
+  d->tz_dirty = d->tile_lists_dirty = true;
   if (ncells <= 0) {
     d->nbc = 0;
     return TRI_OK;
@@ -848,6 +883,7 @@ int tri_domain_advance(tri_domain* d, int32_t max_steps, tri_progress* p) {
   m->events = 0;
   m->steps = 0;
   m->status = 0;
+  m->limit = max_steps;
   const bool need_dt = !d->dt_valid && !m->time_increment_fixed;
   if (need_dt) m->dt_key[m->rd] = kDtKeyInf;
   int rc = push_clock(d);
@@ -977,6 +1013,7 @@ int tri_domain_autotune(tri_domain* d, int32_t trial_steps, tri_tuning* out) {
       if (heights[hi] > std::max(8, d->desc.rows - 2)) continue;
       d->flux_variant = v;
       d->rb = heights[hi];
+      d->tile_lists_dirty = true;
       size_flux_grid(d);
       drop_graph(d);
       rc = save_restore(false);
@@ -987,7 +1024,9 @@ int tri_domain_autotune(tri_domain* d, int32_t trial_steps, tri_tuning* out) {
       m->it_print = 0;
       m->time_series = 0;
       m->halt = 0;
-      m->dt_key[m->rd] = kDtKeyInf;
+      m->steps = 0;
+      m->limit = INT32_MAX;
+          m->dt_key[m->rd] = kDtKeyInf;
       rc = push_clock(d);
       if (rc == TRI_OK) rc = launch_dt(d);
       if (rc == TRI_OK) rc = launch_steps(d, 2);  // warm-up (also builds the graph)
@@ -1016,7 +1055,7 @@ int tri_domain_autotune(tri_domain* d, int32_t trial_steps, tri_tuning* out) {
   int rc2 = save_restore(false);
   *m = saved;
   d->dt_valid = saved_valid;
-  d->tz_dirty = true;
+  d->tz_dirty = d->tile_lists_dirty = true;
   if (rc2 == TRI_OK) rc2 = push_clock(d);
   cudaStreamSynchronize(d->stream);
   cudaFree(bak);
@@ -1046,7 +1085,7 @@ int tri_domain_set_tuning(tri_domain* d, int32_t variant, int32_t rows_per_tile)
   d->shape_set = true;
   size_flux_grid(d);
   drop_graph(d);
-  d->tz_dirty = true;
+  d->tz_dirty = d->tile_lists_dirty = true;
   return TRI_OK;
 }
 

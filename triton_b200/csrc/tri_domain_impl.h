@@ -65,18 +65,20 @@ struct tri_domain {
   // launch shape of the flux kernel (tile height, register variant, grid)
   int rb = 16, flux_blocks = 1, flux_variant = 1;
   bool shape_set = false;  // tuned or set by the caller: the defaults no longer apply
-  // dry-tile flags of the flux kernel for the current tile shape: [2][tiles]
-  // (tile holds only +0 in buffer 0 / 1) then [tiles] pinned.  Any change of
-  // state, forcing or shape outside the step kernels marks them dirty; they
-  // are reset (nothing known zero) before the next steps.
-  uint8_t* tzero = nullptr;
-  int64_t tz_cap = 0, tz_tiles = 0;
-  bool tz_on = false, tz_dirty = true;
+  // tile flags of the flux kernel for the current tile shape: [2][tiles] (by
+  // state buffer) then [tiles] pinned, and the lists of the tiles' forcing.  Any change of state, forcing or shape outside the
+  // step kernels marks the flags dirty; they are reset (nothing known) before
+  // the next steps.  A change of forcing or shape (tile_lists_dirty) also
+  // rebuilds the pins and lists.
+  uint8_t* tflag = nullptr;
+  int32_t* tlists = nullptr;
+  tri::TileForcing tf{};
+  int64_t tz_tiles = 0;
+  bool tz_dirty = true, tile_lists_dirty = true;
   int32_t* maxh_neg = nullptr;  // device flag: an uploaded max depth is negative (or NaN)
   int64_t work_steps = 0;       // steps advance() ran since tri_domain_set_timing
-  std::vector<uint8_t> tz_pin_host;
   double tuned_ms = 0;
-  // graphs of 'graph_steps' steps
+  // graph of 'graph_steps' steps
   cudaGraphExec_t graph = nullptr;
   int graph_steps = 0;
   bool use_graphs = true;
@@ -95,4 +97,30 @@ int domain_push_clock(tri_domain* d);
 int domain_pull_clock(tri_domain* d);
 int domain_launch_dt(tri_domain* d);
 StepArgs domain_step_args(tri_domain* d);
+// Host side of TileForcing.
+struct TileLists {
+  std::vector<int32_t> tiles, group_of, item_of, items;
+  // one array: tiles, group_of and item_of with their closing offsets, items
+  std::vector<int32_t> flat() const {
+    std::vector<int32_t> v(tiles);
+    v.insert(v.end(), group_of.begin(), group_of.end());
+    v.push_back((int32_t)item_of.size());
+    v.insert(v.end(), item_of.begin(), item_of.end());
+    v.push_back((int32_t)items.size());
+    v.insert(v.end(), items.begin(), items.end());
+    return v;
+  }
+  TileForcing at(const int32_t* dev) const {
+    TileForcing f;
+    f.tiles = dev;
+    f.group_of = f.tiles + tiles.size();
+    f.item_of = f.group_of + group_of.size() + 1;
+    f.items = f.item_of + item_of.size() + 1;
+    f.count = (int)tiles.size();
+    return f;
+  }
+};
+// Appends the forcing of d's flux tiles at height rb, its tiles counted from
+// 'first' on.
+void append_tile_lists(const tri_domain* d, int rb, int32_t first, TileLists& out);
 }  // namespace tri

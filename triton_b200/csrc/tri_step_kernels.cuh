@@ -2,16 +2,17 @@
 //
 // One time step of the reference (triton_simulate.h:191-346) becomes, on the
 // domain's stream:
-//   k_clock         1 thread: dt policy (compute_global_dt :202-226), runoff
-//                   row and hydrograph bracket (:246-285), step events
 //   k_flux_update   fluxes + conserved update + Manning friction + runoff
 //                   (kernels_flux.h, kernels_state.h, kernels.h:103-152)
-//   k_sources       point inflows (kernels.h:51-84), only with sources
-//   k_open_bc       open-boundary ghosts (kernels.h:437-512), only if open
-//   k_extbc         external boundary cells (kernels.h:237-424), only with extbc
-//   k_wetdry_dt     wet/dry masks + max depth (kernels_wetdry.h:25-93) fused
+//   k_forcing       point inflows (kernels.h:51-84), open-boundary ghosts
+//                   (kernels.h:437-512) and external boundary cells
+//                   (kernels.h:237-424), only where there are any
+//   k_post          wet/dry masks + max depth (kernels_wetdry.h:25-93) fused
 //                   with the NEXT step's CFL dt and its min reduction
-//                   (kernels.h:167-212)
+//                   (kernels.h:167-212); moves the clock on
+// The flux kernel's blocks begin with the step's clock work: dt policy
+// (compute_global_dt :202-226), runoff row and hydrograph bracket (:246-285),
+// step events.
 // Every kernel reads the step's parameters from the device clock, so a
 // sequence of steps needs no host round trip and can be captured in a graph.
 #pragma once
@@ -32,14 +33,14 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // ---------------------------------------------------------------------------
-// k_clock: the per-step scalar work of the reference host loop.
+// The per-step scalar work of the reference host loop.  begin_step only reads
+// the clock: in the single-domain step one thread of every flux block runs it
+// (about a microsecond before the block's first tile, against 3.3 us for a
+// launch of its own), block 0 leaves the outcome in c->now for the post kernel.
 // ---------------------------------------------------------------------------
-// Returns true when this step raised an event (the domain halts after it).
-__device__ __forceinline__ bool clock_step(DevClock* __restrict__ c) {
-  if (c->halt) {
-    c->active = 0;
-    return false;
-  }
+__device__ __forceinline__ StepNow begin_step(const DevClock* __restrict__ c) {
+  StepNow n;
+  n.active = !(c->halt || c->steps >= c->limit);
   const double t0 = c->simtime;
   double dt;
   if (!c->time_increment_fixed) {
@@ -51,19 +52,21 @@ __device__ __forceinline__ bool clock_step(DevClock* __restrict__ c) {
   } else {
     dt = c->time_step;
   }
-  c->global_dt = dt;
-  c->rdt = 1.0 / dt;
-  c->t_step = t0;
-  c->it_count++;
-  if (c->nroff > 0) {
+  n.dt = dt;
+  n.rdt = 1.0 / dt;
+  n.t_step = t0;
+  n.step = c->it_count + 1;
+  n.runoff_row = c->runoff_row;
+  if (n.active && c->nroff > 0) {
     const int last = c->roff_rows - 1;
     if (t0 > c->roff_t[last]) {
-      c->runoff_row = last;
-    } else if (c->runoff_row + 1 <= last && t0 > c->roff_t[c->runoff_row + 1]) {
-      c->runoff_row++;
+      n.runoff_row = last;
+    } else if (n.runoff_row + 1 <= last && t0 > c->roff_t[n.runoff_row + 1]) {
+      n.runoff_row++;
     }
   }
-  if (c->nsrc > 0) {
+  n.src_idx_low = n.src_idx_high = c->src_idx_low;
+  if (n.active && c->nsrc > 0) {
     int lo = c->src_idx_low, hi = c->hyg_rows - 1;
     bool found = false;
     for (int i = lo; i < hi; i++) {
@@ -75,38 +78,318 @@ __device__ __forceinline__ bool clock_step(DevClock* __restrict__ c) {
       }
     }
     if (!found) lo = hi;
-    c->src_idx_low = lo;
-    c->src_idx_high = hi;
+    n.src_idx_low = lo;
+    n.src_idx_high = hi;
   }
-  c->tile_next = 0;
-  c->src = c->cur;
-  c->dst = c->cur ^ 1;
-  c->cur = c->dst;
-  c->wr = c->rd ^ 1;
-  c->dt_key[c->wr] = kDtKeyInf;
-  c->rd = c->wr;
+  n.src = c->cur;
+  n.dst = c->cur ^ 1;
+  n.wr = c->rd ^ 1;
   const double t1 = t0 + dt;
-  c->simtime = t1;
-  c->average_dt += dt;
-  c->steps++;
+  n.t_end = t1;
   int ev = 0;
-  if (c->it_print > 0 && c->it_count % c->it_print == 0) ev |= TRI_EV_LOG;
+  if (c->it_print > 0 && n.step % c->it_print == 0) ev |= TRI_EV_LOG;
   if (c->time_series && t1 - c->last_obs_time >= c->print_observation) ev |= TRI_EV_OBS;
   if (t1 >= c->print_interval * (c->print_id + 1)) ev |= TRI_EV_PRINT;
   if (!(t1 < c->sim_duration)) ev |= TRI_EV_END;
-  c->active = 1;
-  if (ev) {
+  n.events = ev;
+  return n;
+}
+
+// The clock moves on by the step c->now (one thread).  Returns true when the
+// step raised an event (the domain halts after it).
+__device__ __forceinline__ bool end_step(DevClock* __restrict__ c) {
+  const StepNow& n = c->now;
+  c->global_dt = n.dt;
+  c->it_count = n.step;
+  c->runoff_row = n.runoff_row;
+  c->src_idx_low = n.src_idx_low;
+  c->tile_next = 0;
+  c->cur = n.dst;
+  c->rd = n.wr;
+  c->dt_key[n.wr ^ 1] = kDtKeyInf;  // the next step's slot
+  c->simtime = n.t_end;
+  c->average_dt += n.dt;
+  c->steps++;
+  if (n.events) {
     c->halt = 1;
-    c->events = ev;
+    c->events = n.events;
     return true;
   }
   return false;
 }
 
-static __global__ void k_clock(DevClock* __restrict__ c) {
+// ---------------------------------------------------------------------------
+// Forcing that writes into single cells of the destination buffer after their
+// flux update: point sources, open-boundary ghosts, external boundary cells,
+// in the reference's order.  One launch for all of it: a warp applies the items
+// of one flux tile (TileForcing; no item touches another tile's cells), where
+// a launch per kind and conflict-free wave took 4 to 8 us each, several a step.
+// (Applied by the flux kernel's own warps, at the end of each tile, it cost
+// every tile registers: bowl 2048^2 FP64 99.7 -> 102.6 us, a 24-member FP32
+// ensemble step 259 -> 270 us.)
+// ---------------------------------------------------------------------------
+// Point source `id` (compute_flow, kernels.h:51-84).
+template <typename T>
+__device__ __forceinline__ void source_apply(DevClock* __restrict__ clk, const StepNow& now, const StateBufs<T>& sb,
+                                             const ForcingDev<T>& f, T dx, int id) {
+  const int lo = now.src_idx_low, hi = now.src_idx_high;
+  const T dt = T(now.dt), simtime = T(now.t_step);
+  T* h = sb.H(now.dst);
+  const T flo = f.hyg_v[(size_t)lo * f.nsrc + id], fhi = f.hyg_v[(size_t)hi * f.nsrc + id];
+  const T tlo = T(f.hyg_t[lo]), thi = T(f.hyg_t[hi]);
+  T flow;
+  if (lo == hi) {
+    flow = flo;
+  } else {
+    const T td = simtime - tlo, td2 = thi - tlo;
+    flow = flo + (((fhi - flo) * td) / td2);
+  }
+  const int sid = f.src_cells[id];
+  T hij = h[sid];
+  const T hs = (flow * dt) / (dx * dx);
+  hij += hs;
+  h[sid] = hij;
+  atomicAdd(&clk->acc_step[kAccSources], (double)hs);
+}
+
+// Final values of copy_info_to_exterior_boundaries_west_east followed by
+// _north_south (kernels.h:437-512) in state buffer d, item k of max(rows, cols): ghost columns
+// take the adjacent interior column (rows 1..rows-2), ghost rows take the
+// adjacent interior row, corners the diagonal interior cell.
+template <typename T>
+__device__ __forceinline__ void open_bc_item(int d, const StateBufs<T>& sb, int rows, int cols, int k) {
+  T* h = sb.H(d);
+  T* qx = sb.QX(d);
+  T* qy = sb.QY(d);
+  auto cp = [&](size_t g, size_t i) {
+    h[g] = h[i];
+    qx[g] = qx[i];
+    qy[g] = qy[i];
+  };
+  if (k < rows) {
+    const int r = k;
+    if (r >= 1 && r <= rows - 2) {
+      cp((size_t)r * cols, (size_t)r * cols + 1);
+      cp((size_t)r * cols + cols - 1, (size_t)r * cols + cols - 2);
+    }
+  }
+  if (k < cols) {
+    const int cc = k;
+    const int ci = cc == 0 ? 1 : (cc == cols - 1 ? cols - 2 : cc);
+    cp((size_t)cc, (size_t)cols + ci);
+    cp((size_t)(rows - 1) * cols + cc, (size_t)(rows - 2) * cols + ci);
+  }
+}
+
+// The same for the ghosts next to one flux tile (rows r0..r1, columns from c0
+// on), by the warp that owns it.
+template <typename T>
+__device__ __forceinline__ void open_bc_tile(int d, const StateBufs<T>& sb, int rows, int cols, int r0, int r1,
+                                             int c0, int lane) {
+  T* h = sb.H(d);
+  T* qx = sb.QX(d);
+  T* qy = sb.QY(d);
+  auto cp = [&](size_t g, size_t i) {
+    h[g] = h[i];
+    qx[g] = qx[i];
+    qy[g] = qy[i];
+  };
+  const int c1 = min(c0 + kStripCols - 1, cols - 2);
+  for (int r = r0 + lane; r <= r1; r += 32) {
+    if (c0 == 1) cp((size_t)r * cols, (size_t)r * cols + 1);
+    if (c1 == cols - 2) cp((size_t)r * cols + cols - 1, (size_t)r * cols + cols - 2);
+  }
+  // ghost rows; a corner takes the diagonal interior cell
+  const int ca = c0 == 1 ? 0 : c0, cz = c1 == cols - 2 ? cols - 1 : c1;
+  for (int c = ca + lane; c <= cz; c += 32) {
+    const int ci = min(max(c, 1), cols - 2);
+    if (r0 == 1) cp((size_t)c, (size_t)cols + ci);
+    if (r1 == rows - 2) cp((size_t)(rows - 1) * cols + c, (size_t)(rows - 2) * cols + ci);
+  }
+}
+
+// compute_extbc_values for one boundary cell (kernels.h:254-420), single rank.
+template <typename T>
+__device__ __forceinline__ void extbc_apply(DevClock* __restrict__ clk, const StepNow& now, const StateBufs<T>& sb,
+                                            const BedMap<T>& bed, const T* __restrict__ n2, int id,
+                                            const ForcingDev<T>& f, int rows, int cols) {
+  const T* __restrict__ var1 = f.bc_v1;
+  const T* __restrict__ var2 = f.bc_v2;
+  const int d = now.dst;
+  T* h = sb.H(d);
+  T* qx = sb.QX(d);
+  T* qy = sb.QY(d);
+  const T dt = T(now.dt);
+  const T simtime = T(now.t_step);
+  const int ii = f.bc_cells[id];
+  const int bt = f.bc_types[id];
+  const int s0 = f.bc_start[id];
+  const int ix = ii / cols, iy = ii % cols;
+  const bool top = (ix == 1), btm = (ix == rows - 2), lt = (iy == 1), rt = (iy == cols - 2);
+  if (!(top || lt || rt || btm)) return;
+  bool corner = false;
+  int ib = ii, ibc = ii;
+  T f0 = T(1), f1 = T(0), f2 = T(0);
+  if (lt) {
+    ib = ii - 1;
+    f1 = T(-1);
+    f2 = T(0);
+  }
+  if (rt) {
+    ib = ii + 1;
+    f1 = T(1);
+    f2 = T(0);
+  }
+  if (top) {
+    ib = ii - cols;
+    f1 = T(0);
+    f2 = T(1);
+    if (lt) {
+      corner = true;
+      ibc = ii - 1;
+      f2 = T(0);
+    }
+    if (rt) {
+      corner = true;
+      ibc = ii + 1;
+      f2 = T(0);
+    }
+  }
+  if (btm) {
+    ib = ii + cols;
+    f1 = T(0);
+    f2 = T(-1);
+    if (lt) {
+      corner = true;
+      ibc = ii - 1;
+      f2 = T(0);
+    }
+    if (rt) {
+      corner = true;
+      ibc = ii + 1;
+      f2 = T(0);
+    }
+  }
+  T hij = h[ii], qxij = qx[ii], qyij = qy[ii];
+  if (bt == 0) {
+    h[ib] = hij;
+    qx[ib] = qxij;
+    qy[ib] = qyij;
+    if (corner) {
+      h[ibc] = hij;
+      qx[ibc] = qxij;
+      qy[ibc] = qyij;
+    }
+    return;
+  }
+  if (bt == 1) {
+    const T lvar = T(0.5) * (simtime + simtime + dt);
+    int lo = 0, hi = f.bc_nrows[id] - 1;
+    if (lvar < var1[s0]) {
+      lo = 0;
+      hi = 0;
+    } else if (lvar > var1[hi + s0]) {
+      lo = hi;
+    } else {
+      lo = 0;  // a non-monotone table leaves the reference's index unset; clamp to row 0
+      for (int i = 0; i < hi; i++) {
+        if (var1[i + s0] <= lvar && var1[i + 1 + s0] > lvar) {
+          lo = i;
+          hi = i + 1;
+          break;
+        }
+      }
+    }
+    T aux;
+    if (lo == hi) {
+      aux = var2[lo + s0];
+    } else {
+      const T td = lvar - var1[lo + s0];
+      const T td2 = var1[hi + s0] - var1[lo + s0];
+      aux = var2[lo + s0] + (((var2[hi + s0] - var2[lo + s0]) * td) / td2);
+    }
+    if (sizeof(T) == 8) {
+      hij = dev_fmax(aux - (T)bed.absolute(ii, ix, iy), T(0));
+    } else {  // FP32 form: level minus bed in FP64, then rounded
+      hij = (T)fmax((double)aux - bed.absolute(ii, ix, iy), 0.0);
+    }
+    atomicAdd(&clk->acc_step[kAccExtbc], (double)hij - (double)h[ii]);
+  } else {
+    const T aux = var1[s0];
+    T vel = T(0);
+    if (bt == 2) vel = dev_sqrt(aux * hij * dev_cbrt(hij) / dev_fmax(n2[ii], T(1e-6)));
+    if (bt == 3) vel = aux * dev_sqrt(T(kGravity) * hij);
+    qxij = hij * vel;
+    qyij = hij * vel;
+  }
+  h[ib] = hij * f0;
+  qx[ib] = qxij * f1;
+  qy[ib] = qyij * f2;
+  h[ii] = hij * f0;
+  qx[ii] = qxij * f1;
+  qy[ii] = qyij * f2;
+  if (corner) {
+    h[ibc] = hij * f0;
+    qx[ibc] = qxij * f1;
+    qy[ibc] = qyij * f2;
+  }
+}
+
+// Applies the forcing of list entry k's tile (whole warp).
+template <typename T>
+__device__ __forceinline__ void tile_forcing(DevClock* clk, const StepNow& now, const StateBufs<T>& sb,
+                                             const BedMap<T>& bed, const T* __restrict__ n2, const ForcingDev<T>& f,
+                                             const TileForcing& tf, bool open, T dx, int rows, int cols, int rb,
+                                             int tile, int k, int lane) {
+  int g = tf.group_of[k];
+  const int gz = tf.group_of[k + 1];
+  for (bool edges = open; g < gz || edges; g++) {
+    const int a = g < gz ? tf.item_of[g] : 0, z = g < gz ? tf.item_of[g + 1] : 0;
+    if (edges && (g >= gz || tf.items[a] < 0)) {  // after the sources, before the boundary cells
+      const int ns = (cols - 2 + kStripCols - 1) / kStripCols;
+      const int c0 = 1 + (tile % ns) * kStripCols, r0 = 1 + (tile / ns) * rb, r1 = min(r0 + rb - 1, rows - 2);
+      open_bc_tile<T>(now.dst, sb, rows, cols, r0, r1, c0, lane);
+      edges = false;
+      __syncwarp();
+    }
+    for (int i = a + lane; i < z; i += 32) {
+      const int id = tf.items[i];
+      if (id >= 0)
+        source_apply<T>(clk, now, sb, f, dx, id);
+      else
+        extbc_apply<T>(clk, now, sb, bed, n2, -1 - id, f, rows, cols);
+    }
+    __syncwarp();
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(128) k_forcing(DevClock* __restrict__ clk, const __grid_constant__ StateBufs<T> sb,
+                                                 const __grid_constant__ BedMap<T> bed, const T* __restrict__ n2,
+                                                 const __grid_constant__ ForcingDev<T> f,
+                                                 const __grid_constant__ TileForcing tf, bool open, T dx, int rows,
+                                                 int cols, int rb) {
   pdl_wait();
   pdl_trigger();
-  if (threadIdx.x == 0) clock_step(c);
+  const int k = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (k >= tf.count || !clk->now.active) return;
+  tile_forcing<T>(clk, clk->now, sb, bed, n2, f, tf, open, dx, rows, cols, rb, tf.tiles[k], k, threadIdx.x & 31);
+}
+
+// The same for the tiles of all members of a batch (tiles over all members).
+template <typename T>
+__global__ void __launch_bounds__(128) k_batch_forcing(const MemberDev<T>* __restrict__ mem,
+                                                       const int32_t* __restrict__ tile_member,
+                                                       const __grid_constant__ TileForcing tf) {
+  pdl_wait();
+  pdl_trigger();
+  const int k = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (k >= tf.count) return;
+  const int tile = tf.tiles[k];
+  const MemberDev<T>& M = mem[tile_member[tile]];
+  if (!M.clk->now.active) return;
+  tile_forcing<T>(M.clk, M.clk->now, M.sb, M.bed, M.n2, M.f, tf, M.open != 0, M.dx, M.rows, M.cols, M.rb,
+                  tile - (int)M.tile_begin, k, threadIdx.x & 31);
 }
 
 // ---------------------------------------------------------------------------
@@ -281,18 +564,17 @@ struct FluxCtx {
 };
 
 template <typename T>
-__device__ __forceinline__ FluxCtx<T> flux_ctx(DevClock* clk, const StateBufs<T>& sb, const BedMap<T>& bed,
-                                               const T* n2, const int32_t* zone, const T* rates, int rows, int cols,
-                                               int rb, T dx, T rdx, T hextra) {
+__device__ __forceinline__ FluxCtx<T> flux_ctx(DevClock* clk, const StepNow& now, const StateBufs<T>& sb,
+                                               const BedMap<T>& bed, const T* n2, const int32_t* zone, const T* rates,
+                                               int rows, int cols, int rb, T dx, T rdx, T hextra) {
   FluxCtx<T> X;
   X.clk = clk;
-  const int src = clk->src, dst = clk->dst;
-  X.hi = sb.H(src);
-  X.qxi = sb.QX(src);
-  X.qyi = sb.QY(src);
-  X.ho = sb.H(dst);
-  X.qxo = sb.QX(dst);
-  X.qyo = sb.QY(dst);
+  X.hi = sb.H(now.src);
+  X.qxi = sb.QX(now.src);
+  X.qyi = sb.QY(now.src);
+  X.ho = sb.H(now.dst);
+  X.qxo = sb.QX(now.dst);
+  X.qyo = sb.QY(now.dst);
   X.bed = bed;
   X.n2 = n2;
   X.zone = zone;
@@ -303,28 +585,26 @@ __device__ __forceinline__ FluxCtx<T> flux_ctx(DevClock* clk, const StateBufs<T>
   X.nstrips = (cols - 2 + kStripCols - 1) / kStripCols;
   X.nroff = clk->nroff;
   X.roff_rows = clk->roff_rows;
-  X.roff_row = clk->runoff_row;
-  X.step = (uint32_t)clk->it_count;
-  X.K = step_k<T>(dx, T(clk->global_dt), rdx, T(clk->rdt), hextra);
+  X.roff_row = now.runoff_row;
+  X.step = (uint32_t)now.step;
+  X.K = step_k<T>(dx, T(now.dt), rdx, T(now.rdt), hextra);
   X.tz_src = nullptr;
   X.tz_dst = nullptr;
   X.tpin = nullptr;
   return X;
 }
 
-// The same with the dry-tile flags: [2][tiles] zero flags by buffer, then
-// [tiles] pinned.
+// The same with the tile flags: [2][tiles] by buffer, then [tiles] pinned.
 template <typename T, bool kSkip>
-__device__ __forceinline__ FluxCtx<T> flux_ctx_skip(DevClock* clk, const StateBufs<T>& sb, const BedMap<T>& bed,
-                                                    const T* n2, const int32_t* zone, const T* rates, int rows,
-                                                    int cols, int rb, T dx, T rdx, T hextra, uint8_t* tzero) {
-  FluxCtx<T> X = flux_ctx<T>(clk, sb, bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra);
-  if (kSkip) {
-    const size_t ntiles = (size_t)X.nstrips * (size_t)((rows - 2 + rb - 1) / rb);
-    X.tz_src = tzero + (size_t)clk->src * ntiles;
-    X.tz_dst = tzero + (size_t)clk->dst * ntiles;
-    X.tpin = tzero + 2 * ntiles;
-  }
+__device__ __forceinline__ FluxCtx<T> flux_ctx_tiles(DevClock* clk, const StepNow& now, const StateBufs<T>& sb,
+                                                     const BedMap<T>& bed, const T* n2, const int32_t* zone,
+                                                     const T* rates, int rows, int cols, int rb, T dx, T rdx,
+                                                     T hextra, uint8_t* tflag) {
+  FluxCtx<T> X = flux_ctx<T>(clk, now, sb, bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra);
+  const size_t ntiles = (size_t)X.nstrips * (size_t)((rows - 2 + rb - 1) / rb);
+  if (kSkip) X.tz_src = tflag + (size_t)now.src * ntiles;
+  X.tz_dst = tflag + (size_t)now.dst * ntiles;
+  X.tpin = tflag + 2 * ntiles;
   return X;
 }
 
@@ -344,10 +624,10 @@ __device__ __forceinline__ bool tile_skippable(const FluxCtx<T>& X, unsigned til
   const int ns = X.nstrips, nty = (X.rows - 2 + X.rb - 1) / X.rb;
   const int sx = (int)(tile % ns), ry = (int)(tile / ns);
   if (!(X.tz_src[tile] & X.tz_dst[tile]) || X.tpin[tile]) return false;
-  if (sx > 0 && !X.tz_src[tile - 1]) return false;
-  if (sx < ns - 1 && !X.tz_src[tile + 1]) return false;
-  if (ry > 0 && !X.tz_src[tile - ns]) return false;
-  if (ry < nty - 1 && !X.tz_src[tile + ns]) return false;
+  if (sx > 0 && !(X.tz_src[tile - 1])) return false;
+  if (sx < ns - 1 && !(X.tz_src[tile + 1])) return false;
+  if (ry > 0 && !(X.tz_src[tile - ns])) return false;
+  if (ry < nty - 1 && !(X.tz_src[tile + ns])) return false;
   return true;
 }
 
@@ -573,11 +853,13 @@ __device__ __noinline__ void flux_tile_guarded_ctx(const FluxCtx<T>* X, unsigned
   flux_tile_form<T, false, true, false>(*X, tile, lane);
 }
 template <typename T, bool kSkip>
-__device__ __noinline__ void flux_tile_guarded(DevClock* clk, const StateBufs<T> sb, const BedMap<T> bed, const T* n2,
-                                               const int32_t* zone, const T* rates, int rows, int cols, int rb, T dx,
-                                               T rdx, T hextra, uint8_t* tzero, unsigned tile, int lane) {
+__device__ __noinline__ void flux_tile_guarded(DevClock* clk, const StepNow* now, const StateBufs<T>* sb,
+                                               const BedMap<T>* bed, const T* n2, const int32_t* zone, const T* rates,
+                                               int rows, int cols, int rb, T dx, T rdx, T hextra, uint8_t* tflag,
+                                               unsigned tile, int lane) {
   flux_tile_form<T, kSkip, false, false>(
-      flux_ctx_skip<T, kSkip>(clk, sb, bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra, tzero), tile, lane);
+      flux_ctx_tiles<T, kSkip>(clk, *now, *sb, *bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra, tflag), tile,
+      lane);
 }
 
 // One tile of a batch member, its context in shared memory.
@@ -586,17 +868,23 @@ __device__ __forceinline__ void flux_tile_member(const FluxCtx<T>& X, unsigned t
   if (!flux_tile_form<T, false, true, sizeof(T) == 8>(X, tile, lane)) flux_tile_guarded_ctx<T>(&X, tile, lane);
 }
 
-// kSkip: the domain keeps dry-tile flags (tzero) and skips dry tiles.
+// kSkip: the domain can have dry tiles (no runoff) and skips them.
 template <typename T, int MINB, bool kSkip>
-__global__ void __launch_bounds__(128, MINB) k_flux_update(DevClock* __restrict__ clk, StateBufs<T> sb,
-                                                     const BedMap<T> bed, const T* __restrict__ n2,
-                                                     const int32_t* __restrict__ zone, const T* __restrict__ rates,
-                                                     int rows, int cols, int rb, T dx, T rdx, T hextra,
-                                                     uint8_t* __restrict__ tzero) {
+__global__ void __launch_bounds__(128, MINB)
+    k_flux_update(DevClock* __restrict__ clk, const __grid_constant__ StateBufs<T> sb,
+                  const __grid_constant__ BedMap<T> bed, const T* __restrict__ n2, const int32_t* __restrict__ zone,
+                  const T* __restrict__ rates, int rows, int cols, int rb, T dx, T rdx, T hextra,
+                  uint8_t* __restrict__ tflag) {
+  __shared__ StepNow s_now;
   pdl_wait();
-  if (!clk->active) return;
-  const FluxCtx<T> X =
-      flux_ctx_skip<T, kSkip>(clk, sb, bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra, tzero);
+  if (threadIdx.x == 0) {
+    s_now = begin_step(clk);
+    if (blockIdx.x == 0) clk->now = s_now;
+  }
+  __syncthreads();
+  if (!s_now.active) return;
+  const FluxCtx<T> X = flux_ctx_tiles<T, kSkip>(clk, s_now, sb, bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra,
+                                                tflag);
   const int lane = threadIdx.x & 31;
   const unsigned ntiles = (unsigned)X.nstrips * (unsigned)((rows - 2 + rb - 1) / rb);
   unsigned skipped = 0;  // interior cells of the tiles this warp skipped (lane 0)
@@ -614,239 +902,14 @@ __global__ void __launch_bounds__(128, MINB) k_flux_update(DevClock* __restrict_
     if ((tile & 0x7FFFFFFFu) >= ntiles) break;
     if (kSkip && (tile >> 31)) continue;
     if (!flux_tile_form<T, kSkip, false, sizeof(T) == 8>(X, tile, lane))
-      flux_tile_guarded<T, kSkip>(clk, sb, bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra, tzero, tile, lane);
+      flux_tile_guarded<T, kSkip>(clk, &s_now, &sb, &bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra, tflag,
+                                  tile, lane);
   }
   pdl_trigger();  // no tile left for this warp
   if (kSkip && lane == 0 && skipped)  // spread over the slots: one address would serialize the atomics
     atomicAdd(&clk->skipped[0][(blockIdx.x * 4 + (threadIdx.x >> 5)) % kSkipSlots], (unsigned long long)skipped);
 }
 
-// ---------------------------------------------------------------------------
-// Sparse kernels (run on the destination buffer after k_flux_update).
-// 'order' lists the items of one conflict-free wave; items that touch the
-// same cell are in different waves, launched in the reference's index order.
-// ---------------------------------------------------------------------------
-template <typename T>
-__global__ void k_sources(DevClock* __restrict__ clk, StateBufs<T> sb, const int32_t* __restrict__ order,
-                          int count, int nsrc, const int32_t* __restrict__ cells, const double* __restrict__ hyg_t,
-                          const T* __restrict__ hyg_v, T dx) {
-  pdl_wait();
-  pdl_trigger();
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count || !clk->active) return;
-  const int id = order[k];
-  const int lo = clk->src_idx_low, hi = clk->src_idx_high;
-  const T dt = T(clk->global_dt);
-  const T simtime = T(clk->t_step);
-  T* h = sb.H(clk->dst);
-  const T flo = hyg_v[(size_t)lo * nsrc + id];
-  const T fhi = hyg_v[(size_t)hi * nsrc + id];
-  const T tlo = T(hyg_t[lo]), thi = T(hyg_t[hi]);
-  T flow;
-  if (lo == hi) {
-    flow = flo;
-  } else {
-    const T td = simtime - tlo;
-    const T td2 = thi - tlo;
-    flow = flo + (((fhi - flo) * td) / td2);
-  }
-  const int sid = cells[id];
-  T hij = h[sid];
-  const T hs = (flow * dt) / (dx * dx);
-  hij += hs;
-  h[sid] = hij;
-  atomicAdd(&clk->acc_step[kAccSources], (double)hs);
-}
-
-// Final values of copy_info_to_exterior_boundaries_west_east followed by
-// _north_south (kernels.h:437-512), item k of max(rows, cols): ghost columns
-// take the adjacent interior column (rows 1..rows-2), ghost rows take the
-// adjacent interior row, corners the diagonal interior cell.
-template <typename T>
-__device__ __forceinline__ void open_bc_item(const DevClock* __restrict__ clk, const StateBufs<T>& sb, int rows,
-                                             int cols, int k) {
-  const int d = clk->dst;
-  T* h = sb.H(d);
-  T* qx = sb.QX(d);
-  T* qy = sb.QY(d);
-  auto cp = [&](size_t g, size_t i) {
-    h[g] = h[i];
-    qx[g] = qx[i];
-    qy[g] = qy[i];
-  };
-  if (k < rows) {
-    const int r = k;
-    if (r >= 1 && r <= rows - 2) {
-      cp((size_t)r * cols, (size_t)r * cols + 1);
-      cp((size_t)r * cols + cols - 1, (size_t)r * cols + cols - 2);
-    }
-  }
-  if (k < cols) {
-    const int cc = k;
-    const int ci = cc == 0 ? 1 : (cc == cols - 1 ? cols - 2 : cc);
-    cp((size_t)cc, (size_t)cols + ci);
-    cp((size_t)(rows - 1) * cols + cc, (size_t)(rows - 2) * cols + ci);
-  }
-}
-
-template <typename T>
-__global__ void k_open_bc(const DevClock* __restrict__ clk, StateBufs<T> sb, int rows, int cols) {
-  pdl_wait();
-  pdl_trigger();
-  if (!clk->active) return;
-  open_bc_item<T>(clk, sb, rows, cols, blockIdx.x * blockDim.x + threadIdx.x);
-}
-
-// compute_extbc_values for one boundary cell (kernels.h:254-420), single rank.
-template <typename T>
-__device__ __forceinline__ void extbc_apply(DevClock* __restrict__ clk, const StateBufs<T>& sb, const BedMap<T>& bed,
-                                            const T* __restrict__ n2, int id, const int32_t* __restrict__ cells,
-                                            const int32_t* __restrict__ types, const int32_t* __restrict__ start,
-                                            const int32_t* __restrict__ nrowsv, const T* __restrict__ var1,
-                                            const T* __restrict__ var2, int rows, int cols) {
-  const int d = clk->dst;
-  T* h = sb.H(d);
-  T* qx = sb.QX(d);
-  T* qy = sb.QY(d);
-  const T dt = T(clk->global_dt);
-  const T simtime = T(clk->t_step);
-  const int ii = cells[id];
-  const int bt = types[id];
-  const int s0 = start[id];
-  const int ix = ii / cols, iy = ii % cols;
-  const bool top = (ix == 1), btm = (ix == rows - 2), lt = (iy == 1), rt = (iy == cols - 2);
-  if (!(top || lt || rt || btm)) return;
-  bool corner = false;
-  int ib = ii, ibc = ii;
-  T f0 = T(1), f1 = T(0), f2 = T(0);
-  if (lt) {
-    ib = ii - 1;
-    f1 = T(-1);
-    f2 = T(0);
-  }
-  if (rt) {
-    ib = ii + 1;
-    f1 = T(1);
-    f2 = T(0);
-  }
-  if (top) {
-    ib = ii - cols;
-    f1 = T(0);
-    f2 = T(1);
-    if (lt) {
-      corner = true;
-      ibc = ii - 1;
-      f2 = T(0);
-    }
-    if (rt) {
-      corner = true;
-      ibc = ii + 1;
-      f2 = T(0);
-    }
-  }
-  if (btm) {
-    ib = ii + cols;
-    f1 = T(0);
-    f2 = T(-1);
-    if (lt) {
-      corner = true;
-      ibc = ii - 1;
-      f2 = T(0);
-    }
-    if (rt) {
-      corner = true;
-      ibc = ii + 1;
-      f2 = T(0);
-    }
-  }
-  T hij = h[ii], qxij = qx[ii], qyij = qy[ii];
-  if (bt == 0) {
-    h[ib] = hij;
-    qx[ib] = qxij;
-    qy[ib] = qyij;
-    if (corner) {
-      h[ibc] = hij;
-      qx[ibc] = qxij;
-      qy[ibc] = qyij;
-    }
-    return;
-  }
-  if (bt == 1) {
-    const T lvar = T(0.5) * (simtime + simtime + dt);
-    int lo = 0, hi = nrowsv[id] - 1;
-    if (lvar < var1[s0]) {
-      lo = 0;
-      hi = 0;
-    } else if (lvar > var1[hi + s0]) {
-      lo = hi;
-    } else {
-      lo = 0;  // a non-monotone table leaves the reference's index unset; clamp to row 0
-      for (int i = 0; i < hi; i++) {
-        if (var1[i + s0] <= lvar && var1[i + 1 + s0] > lvar) {
-          lo = i;
-          hi = i + 1;
-          break;
-        }
-      }
-    }
-    T aux;
-    if (lo == hi) {
-      aux = var2[lo + s0];
-    } else {
-      const T td = lvar - var1[lo + s0];
-      const T td2 = var1[hi + s0] - var1[lo + s0];
-      aux = var2[lo + s0] + (((var2[hi + s0] - var2[lo + s0]) * td) / td2);
-    }
-    if (sizeof(T) == 8) {
-      hij = dev_fmax(aux - (T)bed.absolute(ii, ix, iy), T(0));
-    } else {  // FP32 form: level minus bed in FP64, then rounded
-      hij = (T)fmax((double)aux - bed.absolute(ii, ix, iy), 0.0);
-    }
-    atomicAdd(&clk->acc_step[kAccExtbc], (double)hij - (double)h[ii]);
-  } else {
-    const T aux = var1[s0];
-    T vel = T(0);
-    if (bt == 2) vel = dev_sqrt(aux * hij * dev_cbrt(hij) / dev_fmax(n2[ii], T(1e-6)));
-    if (bt == 3) vel = aux * dev_sqrt(T(kGravity) * hij);
-    qxij = hij * vel;
-    qyij = hij * vel;
-  }
-  h[ib] = hij * f0;
-  qx[ib] = qxij * f1;
-  qy[ib] = qyij * f2;
-  h[ii] = hij * f0;
-  qx[ii] = qxij * f1;
-  qy[ii] = qyij * f2;
-  if (corner) {
-    h[ibc] = hij * f0;
-    qx[ibc] = qxij * f1;
-    qy[ibc] = qyij * f2;
-  }
-}
-
-template <typename T>
-__global__ void k_extbc(DevClock* __restrict__ clk, StateBufs<T> sb, const BedMap<T> bed, const T* __restrict__ n2,
-                        const int32_t* __restrict__ order, int count, const int32_t* __restrict__ cells,
-                        const int32_t* __restrict__ types, const int32_t* __restrict__ start,
-                        const int32_t* __restrict__ nrowsv, const T* __restrict__ var1, const T* __restrict__ var2,
-                        int rows, int cols) {
-  pdl_wait();
-  pdl_trigger();
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count || !clk->active) return;
-  extbc_apply<T>(clk, sb, bed, n2, order[k], cells, types, start, nrowsv, var1, var2, rows, cols);
-}
-
-// ---------------------------------------------------------------------------
-// k_wetdry_dt: wet/dry masks and max depth on interior cells, then the CFL dt
-// of every cell (ghosts included, as compute_dt_and_sqrt runs over rows*cols)
-// reduced warp -> block -> one atomicMin on the ordered key of the slot the
-// next k_clock reads.  With WETDRY=false it is the initial dt pass.
-// Each thread walks one column down a band of rows, keeping h and the bed of
-// the rows above and below in registers and loading the next row one
-// iteration ahead; east/west neighbours come by shuffle (lanes 0 and 31 load
-// theirs).  Every value is read once, with several loads in flight.
-// ---------------------------------------------------------------------------
 // Kahan fold of the step's volume terms into the domain's totals.
 __device__ __forceinline__ void fold_accounts(DevClock* __restrict__ clk) {
   for (int k = 0; k < kAccTerms; k++) {
@@ -858,104 +921,21 @@ __device__ __forceinline__ void fold_accounts(DevClock* __restrict__ clk) {
   }
 }
 
-// One block's band: columns bx*128 .. +127, rows by*band .. +band-1.
-// Returns this thread's minimum dt key.
-template <typename T, bool WETDRY>
-__device__ __forceinline__ unsigned long long wetdry_band(const DevClock* __restrict__ clk, const StateBufs<T>& sb,
-                                                          const BedMap<T>& bed, T* __restrict__ maxh, int rows,
-                                                          int cols, int band, double dx, double cn, T hextra,
-                                                          float* __restrict__ arrival, float arrival_depth, int bx,
-                                                          int by) {
-  const int buf = WETDRY ? clk->dst : clk->cur;
-  const T* __restrict__ h = sb.H(buf);
-  T* __restrict__ qx = sb.QX(buf);
-  T* __restrict__ qy = sb.QY(buf);
-  const T E12 = eps12<T>();
-  const int lane = threadIdx.x & 31;
-  const int c = bx * kWetCols + threadIdx.x;
-  const int ra = by * band;
-  const int rz = min(ra + band - 1, rows - 1);
-  const bool incol = c < cols;
-  const bool intcol = c >= 1 && c <= cols - 2;
-  const double zref = bed.ref_of(ra, min(bx * kWetCols, cols - 1));
-  const float simtime_now = WETDRY ? (float)clk->simtime : 0.0f;
-
-  T hm = T(0), zm = T(0), h0 = T(0), z0 = T(0), hp = T(0), zp = T(0);
-  T qx0 = T(0), qy0 = T(0), mh0 = T(0), qxp = T(0), qyp = T(0), mhp = T(0);
-  auto load_row = [&](int r, T& hv, T& zv, T& qxv, T& qyv, T& mhv) {
-    if (incol && r >= 0 && r < rows) {
-      const size_t id = (size_t)r * cols + c;
-      hv = h[id];
-      zv = bed.local(id, r, c, zref);
-      qxv = qx[id];
-      qyv = qy[id];
-      if (WETDRY && intcol && r >= 1 && r <= rows - 2) mhv = maxh[id];
-    }
-  };
-  {
-    T a, b, e;
-    if (ra >= 1) load_row(ra - 1, hm, zm, a, b, e);
+// Wave speed of a wet cell (compute_dt_and_sqrt, kernels.h:167-187).  FP64:
+// the reference's denominator, bit for bit, straight-line where the cell's
+// values are in the range of those forms.  FP32 form: in FP32 (its maximum and
+// the dt are FP64).
+__device__ __forceinline__ double wave_speed(double h, double qx, double qy) {
+  const double q = fmax(fabs(qx), fabs(qy));
+  if (regular_cell(h, q, q)) {
+    const double y = rsqrt_line(h);
+    return div_line(q, h, recip_line(h, y * y)) + kSqrtG * sqrt_line(h, y);
   }
-  load_row(ra, h0, z0, qx0, qy0, mh0);
-  unsigned long long key = kDtKeyInf;
-  for (int r = ra; r <= rz; ++r) {
-    if (r + 1 <= rows - 1) load_row(r + 1, hp, zp, qxp, qyp, mhp);
-    // east / west neighbours of row r
-    T he = __shfl_down_sync(0xffffffffu, h0, 1), ze = __shfl_down_sync(0xffffffffu, z0, 1);
-    T hw = __shfl_up_sync(0xffffffffu, h0, 1), zw = __shfl_up_sync(0xffffffffu, z0, 1);
-    const size_t id = (size_t)r * cols + c;
-    const bool interior = WETDRY && intcol && r >= 1 && r <= rows - 2;
-    if (interior) {
-      if (lane == 31) {
-        he = h[id + 1];
-        ze = bed.local(id + 1, r, c + 1, zref);
-      }
-      if (lane == 0) {
-        hw = h[id - 1];
-        zw = bed.local(id - 1, r, c - 1, zref);
-      }
-    }
-    T qxv = qx0, qyv = qy0;
-    const T hij = h0;
-    if (interior) {
-      const T zij = z0;
-      if (hij > hextra) {
-        if ((hij + zij < ze && he < E12) || (hij + zij < zw && hw < E12)) {
-          qxv = T(0);
-          qx[id] = T(0);
-        }
-        if ((hij + zij < zm && hm < E12) || (hij + zij < zp && hp < E12)) {
-          qyv = T(0);
-          qy[id] = T(0);
-        }
-      }
-      if (hij > mh0) maxh[id] = hij;
-      if (arrival != nullptr && hij > arrival_depth && !(arrival[id] < 3.0e38f)) arrival[id] = simtime_now;
-    }
-    if (incol && hij > hextra) {  // wave speed of the CFL dt (reduced as its maximum)
-      double d;
-      if (sizeof(T) == 8) {  // FP64: the reference's denominator, bit for bit
-        const double hd = (double)hij;
-        const double sq = fmax(sqrt(hd), 0.0);
-        const double maxu = fmax(fabs((double)qxv), fabs((double)qyv)) / hd;
-        d = maxu + kSqrtG * sq;
-      } else {  // FP32 form: speed in FP32, maximum and dt in FP64
-        const T sq = dev_fmax(dev_sqrt(hij), T(0));
-        const T maxu = fdiv(dev_fmax(dev_fabs(qxv), dev_fabs(qyv)), hij);
-        d = (double)(maxu + T(kSqrtG) * sq);
-      }
-      const unsigned long long k = speed_key(d);
-      key = k < key ? k : key;
-    }
-    hm = h0;
-    zm = z0;
-    h0 = hp;
-    z0 = zp;
-    qx0 = qxp;
-    qy0 = qyp;
-    mh0 = mhp;
-  }
-  return key;
+  return q / h + kSqrtG * fmax(sqrt(h), 0.0);
+}
+__device__ __forceinline__ float wave_speed(float h, float qx, float qy) {
+  const float maxu = fdiv(dev_fmax(dev_fabs(qx), dev_fabs(qy)), h);
+  return maxu + float(kSqrtG) * dev_fmax(dev_sqrt(h), 0.0f);
 }
 
 // ---------------------------------------------------------------------------
@@ -1006,9 +986,9 @@ static_assert(WetStage<float>::kBand + 2 <= 32, "staged rows span at most two be
 // once more on every group from 'from' on so no copy still writes this
 // block's shared memory when it exits.
 template <int kGroups>
-__device__ __forceinline__ void stage_abandon(DevClock* clk, uint64_t* bar, int from) {
+__device__ __forceinline__ void stage_abandon(DevClock* clk, uint64_t* bar, int from, uint32_t parity) {
   atomicExch(&clk->status, kStatusStageTimeout);
-  for (int g = from; g < kGroups; ++g) mbar_wait(&bar[g], 0);
+  for (int g = from; g < kGroups; ++g) mbar_wait(&bar[g], parity);
 }
 
 // Test hook (one thread of one block): a bounded wait on a barrier whose
@@ -1024,14 +1004,16 @@ static __device__ __noinline__ void wait_test(DevClock* clk) {
   if (!mbar_wait(&bar, 0, clk->wait_test)) atomicExch(&clk->status, kStatusTestWait);
 }
 
+// iter: how many bands this block has staged before (its barriers' phase).
 template <typename T>
 __device__ __forceinline__ unsigned long long wetdry_staged(DevClock* __restrict__ clk, const StateBufs<T>& sb,
                                                             const BedMap<T>& bed, T* __restrict__ maxh, int rows,
                                                             int cols, T hextra, float* __restrict__ arrival,
-                                                            float arrival_depth, int bx, int by, T* stage) {
+                                                            float arrival_depth, int bx, int by, T* stage,
+                                                            int iter = 0) {
   using S = WetStage<T>;
   constexpr bool kF32 = sizeof(T) == 4;
-  const int buf = clk->dst;
+  const int buf = clk->now.dst;
   T* __restrict__ qx = sb.QX(buf);
   T* __restrict__ qy = sb.QY(buf);
   const T E12 = eps12<T>();
@@ -1049,7 +1031,7 @@ __device__ __forceinline__ unsigned long long wetdry_staged(DevClock* __restrict
   float* tdel = reinterpret_cast<float*>(offs + S::kHRows);
   const int rlo = max(ra - 1, 0), rhi = min(rz + 1, rows - 1);
   const int tr0 = rlo >> 5, tc0 = cl >> 5;
-  if (tid < S::kGroups) mbar_init(&bar[tid], 1);
+  if (iter == 0 && tid < S::kGroups) mbar_init(&bar[tid], 1);
   if (tid < S::kHRows) {
     const int64_t r = (int64_t)(ra - 1 + tid);
     offs[tid] = (int)(r * cols - ((r * cols + cl) & ~(int64_t)(S::kVec - 1)));
@@ -1131,7 +1113,7 @@ __device__ __forceinline__ unsigned long long wetdry_staged(DevClock* __restrict
       de1 = (T)tdel[S::kTileCols + te];
     }
   }
-  const float simtime_now = (float)clk->simtime;
+  const float simtime_now = (float)clk->now.t_end;
   // largest wave speed of the thread's cells (NaN speeds left out, as
   // speed_key does); one key at the end equals the minimum of per-cell keys
   T dmax = T(-1);
@@ -1148,8 +1130,8 @@ __device__ __forceinline__ unsigned long long wetdry_staged(DevClock* __restrict
     for (int jq = 0; jq < S::kBand; ++jq) {
       const int r = ra + jq;
       if (r > rz) break;
-      if (jq % S::kGR == 0 && !mbar_wait(&bar[jq / S::kGR], 0)) {
-        stage_abandon<S::kGroups>(clk, bar, jq / S::kGR);
+      if (jq % S::kGR == 0 && !mbar_wait(&bar[jq / S::kGR], (uint32_t)iter & 1)) {
+        stage_abandon<S::kGroups>(clk, bar, jq / S::kGR, (uint32_t)iter & 1);
         return kDtKeyInf;
       }
       const int j = jq + 1;
@@ -1187,20 +1169,7 @@ __device__ __forceinline__ unsigned long long wetdry_staged(DevClock* __restrict
         if (hij > smh[jq * S::kCap + c + o]) maxh[id] = hij;
         if (arrival != nullptr && hij > arrival_depth && !(arrival[id] < 3.0e38f)) arrival[id] = simtime_now;
       }
-      if (hij > hextra) {  // wave speed of the CFL dt (reduced as its maximum)
-        T d;
-        if (sizeof(T) == 8) {  // FP64: the reference's denominator, bit for bit
-          const double hd = (double)hij;
-          const double sq = fmax(sqrt(hd), 0.0);
-          const double maxu = fmax(fabs((double)qxv), fabs((double)qyv)) / hd;
-          d = (T)(maxu + kSqrtG * sq);
-        } else {  // FP32 form: speed in FP32, maximum and dt in FP64
-          const T sq = dev_fmax(dev_sqrt(hij), T(0));
-          const T maxu = fdiv(dev_fmax(dev_fabs(qxv), dev_fabs(qyv)), hij);
-          d = maxu + T(kSqrtG) * sq;
-        }
-        dmax = dev_fmax(dmax, d);
-      }
+      if (hij > hextra) dmax = dev_fmax(dmax, wave_speed(hij, qxv, qyv));
       zm = z0;
       z0 = zp;
       om = o;
@@ -1229,69 +1198,214 @@ __device__ __forceinline__ void block_min_into(unsigned long long key, unsigned 
   }
 }
 
-template <typename T, bool WETDRY>
-__global__ void __launch_bounds__(kWetCols) k_wetdry_dt(DevClock* __restrict__ clk, StateBufs<T> sb,
-                                                        const BedMap<T> bed, T* __restrict__ maxh, int rows,
-                                                        int cols, int band, double dx, double cn, T hextra,
-                                                        float* __restrict__ arrival, float arrival_depth) {
-  if (WETDRY && !clk->active) return;
-  if (WETDRY && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) fold_accounts(clk);
-  const unsigned long long key = wetdry_band<T, WETDRY>(clk, sb, bed, maxh, rows, cols, band, dx, cn, hextra,
-                                                        arrival, arrival_depth, blockIdx.x, blockIdx.y);
-  block_min_into(key, &clk->dt_key[WETDRY ? clk->wr : clk->rd]);
+// The CFL dt of the current state, ghosts included (compute_dt_and_sqrt runs
+// over rows*cols), into the slot the next step reads.
+template <typename T>
+__global__ void __launch_bounds__(kWetCols) k_initial_dt(DevClock* __restrict__ clk, StateBufs<T> sb, int64_t n,
+                                                         T hextra) {
+  const T* __restrict__ h = sb.H(clk->cur);
+  const T* __restrict__ qx = sb.QX(clk->cur);
+  const T* __restrict__ qy = sb.QY(clk->cur);
+  T dmax = T(-1);
+  for (int64_t i = (int64_t)blockIdx.x * kWetCols + threadIdx.x; i < n; i += (int64_t)gridDim.x * kWetCols) {
+    const T hv = h[i];
+    if (hv > hextra) dmax = dev_fmax(dmax, wave_speed(hv, qx[i], qy[i]));
+  }
+  block_min_into(dmax >= T(0) ? speed_key((double)dmax) : kDtKeyInf, &clk->dt_key[clk->rd]);
 }
 
-// True when every flux tile covering this block's band holds only +0 in the
-// step's destination buffer (tzero: the flux kernel's [2][tiles] flags).  A
-// band without a wet cell has nothing to mask and no wave speed, and it
-// records no max depth or arrival while no max depth is negative (a device
-// flag set by max depth uploads) and the arrival depth is not (the host
-// passes no flags then).  Cell (r, c) belongs to tile row max(r-1,0)/rb and
-// strip max(c-1,0)/kStripCols, clamped: ghost rows and columns belong to the
-// edge tiles that copy them.  Uniform over the block.
+// ---------------------------------------------------------------------------
+// The post kernel: wet/dry masks, max depth and the CFL dt, tile by tile of the
+// flux kernel's tiles; the end of the step.
+//
+// A warp walks a tile as the flux kernel does: lane l holds column c0-1+l, the
+// rows come one after the other with the next row's loads in flight, east and
+// west neighbours by shuffle.  Ghost cells belong to the tiles at the grid's
+// edge (the reference's dt covers rows*cols).  It is a stream of 40 B (FP64) or
+// 20 B a cell read and 8 or 4 written where a max depth rises, so what counts is
+// loads in flight: no staging through shared memory, no block barrier, and as
+// many warps as registers allow.
+// A dry tile (flagged all +0 by the flux kernel in the step's destination
+// buffer) has no wet cell: nothing to mask and no wave speed, and nothing to
+// record while no max depth is negative and the arrival depth is not.
+// ---------------------------------------------------------------------------
 template <typename T>
-__device__ __forceinline__ bool band_all_zero(const DevClock* clk, const uint8_t* __restrict__ tzero, int rows,
-                                              int cols, int rb, int bx, int by) {
-  const int ns = (cols - 2 + kStripCols - 1) / kStripCols, nty = (rows - 2 + rb - 1) / rb;
-  const uint8_t* tz = tzero + (size_t)clk->dst * ((size_t)ns * nty);
-  const int ra = by * WetStage<T>::kBand, rz = min(ra + WetStage<T>::kBand - 1, rows - 1);
-  const int c0 = bx * kWetCols, c1 = min(c0 + kWetCols - 1, cols - 1);
-  const int t0 = min(max(ra - 1, 0) / rb, nty - 1), t1 = min(max(rz - 1, 0) / rb, nty - 1);
-  const int s0 = min(max(c0 - 1, 0) / kStripCols, ns - 1), s1 = min(max(c1 - 1, 0) / kStripCols, ns - 1);
-  const int nsx = s1 - s0 + 1, count = (t1 - t0 + 1) * nsx;
-  int nz = 0;
-  for (int i = threadIdx.x; i < count; i += blockDim.x) nz |= !tz[(size_t)(t0 + i / nsx) * ns + s0 + i % nsx];
-  return !__syncthreads_or(nz);
-}
+struct PostArgs {
+  const T* h;
+  T* qx;
+  T* qy;
+  const T* z;  // FP32 form: offsets from the bed tiles' bases
+  BedMap<T> bed;
+  T* maxh;
+  float* arrival;
+  float arrival_depth, t_end;
+  int rows, cols, rb;
+  T hextra;
+};
 
 template <typename T>
-__global__ void __launch_bounds__(kWetCols) k_wetdry_staged(DevClock* __restrict__ clk, StateBufs<T> sb,
-                                                            const BedMap<T> bed, T* __restrict__ maxh, int rows,
-                                                            int cols, T hextra, float* __restrict__ arrival,
-                                                            float arrival_depth, const uint8_t* __restrict__ tzero,
-                                                            int rb, const int32_t* __restrict__ maxh_neg) {
-  extern __shared__ __align__(128) unsigned char wet_smem[];
+__device__ __forceinline__ PostArgs<T> post_args(const StepNow& now, const StateBufs<T>& sb, const BedMap<T>& bed,
+                                                 T* maxh, float* arrival, float arrival_depth, int rows, int cols,
+                                                 int rb, T hextra) {
+  PostArgs<T> P;
+  P.h = sb.H(now.dst);
+  P.qx = sb.QX(now.dst);
+  P.qy = sb.QY(now.dst);
+  P.z = bed.z;
+  P.bed = bed;
+  P.maxh = maxh;
+  P.arrival = arrival;
+  P.arrival_depth = arrival_depth;
+  P.t_end = (float)now.t_end;
+  P.rows = rows;
+  P.cols = cols;
+  P.rb = rb;
+  P.hextra = hextra;
+  return P;
+}
+
+// One tile (whole warp): returns the largest wave speed of dmax and the lane's
+// cells.
+template <typename T>
+__device__ __forceinline__ T post_tile(const PostArgs<T>& P, unsigned tile, int lane, T dmax) {
+  constexpr bool kF32 = sizeof(T) == 4;
+  const T E12 = eps12<T>();
+  const int rows = P.rows, cols = P.cols;
+  const unsigned ns = (unsigned)(cols - 2 + kStripCols - 1) / kStripCols;
+  const int sx = (int)(tile % ns), ry = (int)(tile / ns);
+  const int c = sx * kStripCols + lane;
+  const bool incol = c < cols;
+  const bool upd = lane >= 1 && lane <= kStripCols && c <= cols - 2;  // an interior column of this tile
+  const bool own = upd || (incol && (c == 0 || c == cols - 1));       // or a ghost column
+  const int r0 = 1 + ry * P.rb, r1 = min(r0 + P.rb - 1, rows - 2);
+  const int ra = r0 == 1 ? 0 : r0, rz = r1 == rows - 2 ? rows - 1 : r1;
+  // FP32 form: bed levels relative to a reference per 128 columns and bed tile
+  // row (deltas of the bed tiles of columns c-1, c, c+1), so that a difference
+  // of levels keeps FP32 accuracy on high terrain
+  T dw = T(0), dc = T(0), de = T(0);
+  double ref = 0.0;
+  auto deltas = [&](int r) {
+    if (kF32 && upd) {
+      ref = P.bed.base_at(r, c & ~(kWetCols - 1));
+      dw = (T)(P.bed.base_at(r, c - 1) - ref);
+      dc = (T)(P.bed.base_at(r, c) - ref);
+      de = (T)(P.bed.base_at(r, c + 1) - ref);
+    }
+  };
+  struct Row {
+    T h, z, qx, qy, m;
+  };
+  const T* __restrict__ hp = P.h;
+  const T* __restrict__ zp = P.z;
+  const T* __restrict__ mp = P.maxh;
+  // row r's values; of the row below the tile only the depth and the bed
+  auto load = [&](int r) {
+    Row w;
+    w.h = w.z = w.qx = w.qy = w.m = T(0);
+    const size_t id = (size_t)r * cols + c;
+    if (incol && r <= rz + 1 && r < rows) {
+      w.h = hp[id];
+      w.z = zp[id];
+    }
+    if (own && r <= rz) {
+      w.qx = P.qx[id];
+      w.qy = P.qy[id];
+      if (upd && r >= 1 && r <= rows - 2) w.m = mp[id];
+    }
+    return w;
+  };
+  T hn = T(0), zn = T(0);  // the row above
+  if (ra > 0 && incol) {
+    const size_t id = (size_t)(ra - 1) * cols + c;
+    hn = hp[id];
+    zn = zp[id];
+  }
+  // two rows of loads in flight
+  Row cur = load(ra), nxt = load(ra + 1);
+  deltas(ra);
+  for (int r = ra; r <= rz; ++r) {
+    const Row nx2 = load(r + 2);
+    if (kF32 && r > ra && (r & 31) == 0) deltas(r);
+    const T he = __shfl_down_sync(0xffffffffu, cur.h, 1), hw = __shfl_up_sync(0xffffffffu, cur.h, 1);
+    T ze = __shfl_down_sync(0xffffffffu, cur.z, 1), zw = __shfl_up_sync(0xffffffffu, cur.z, 1);
+    const size_t id = (size_t)r * cols + c;
+    const bool wet = cur.h > P.hextra;
+    T qx = cur.qx, qy = cur.qy;
+    if (upd && r >= 1 && r <= rows - 2) {
+      if (wet && (he < E12 || hw < E12 || hn < E12 || nxt.h < E12)) {  // a dry neighbour may stop the flow
+        T zc = cur.z, zu = zn, zd = nxt.z;
+        if (kF32) {
+          zc += dc;
+          ze += de;
+          zw += dw;
+          zu += (r & 31) == 0 ? (T)(P.bed.base_at(r - 1, c) - ref) : dc;
+          zd += (r & 31) == 31 ? (T)(P.bed.base_at(r + 1, c) - ref) : dc;
+        }
+        const T level = cur.h + zc;
+        if ((level < ze && he < E12) || (level < zw && hw < E12)) {
+          qx = T(0);
+          P.qx[id] = T(0);
+        }
+        if ((level < zu && hn < E12) || (level < zd && nxt.h < E12)) {
+          qy = T(0);
+          P.qy[id] = T(0);
+        }
+      }
+      if (cur.h > cur.m) P.maxh[id] = cur.h;
+      if (P.arrival != nullptr && cur.h > P.arrival_depth && !(P.arrival[id] < 3.0e38f)) P.arrival[id] = P.t_end;
+    }
+    if (own && wet) dmax = dev_fmax(dmax, wave_speed(cur.h, qx, qy));
+    hn = cur.h;
+    zn = cur.z;
+    cur = nxt;
+    nxt = nx2;
+  }
+  return dmax;
+}
+
+// Interior cells of a tile.
+__device__ __forceinline__ unsigned tile_cells(unsigned tile, int rows, int cols, int rb) {
+  const unsigned ns = (unsigned)(cols - 2 + kStripCols - 1) / kStripCols;
+  const int sx = (int)(tile % ns), r0 = 1 + (int)(tile / ns) * rb;
+  return (unsigned)((min(r0 + rb - 1, rows - 2) - r0 + 1) * min(kStripCols, cols - 2 - sx * kStripCols));
+}
+
+// tflag: the flux kernel's tile flags where dry tiles are skipped, else null.
+template <typename T>
+__global__ void __launch_bounds__(kWetCols, PostBlocks<T>::v)
+    k_post(DevClock* __restrict__ clk, const __grid_constant__ StateBufs<T> sb, const __grid_constant__ BedMap<T> bed,
+           T* __restrict__ maxh, int rows, int cols, T hextra, float* __restrict__ arrival, float arrival_depth,
+           const uint8_t* __restrict__ tflag, int rb, unsigned ntiles) {
   pdl_wait();
   pdl_trigger();
-  if (!clk->active) return;
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
-    fold_accounts(clk);
-    if (clk->wait_test) wait_test(clk);
-  }
-  if (tzero != nullptr && *maxh_neg == 0 && band_all_zero<T>(clk, tzero, rows, cols, rb, blockIdx.x, blockIdx.y)) {
-    if (threadIdx.x == 0) {  // interior cells of the skipped band
-      const int ra = max((int)blockIdx.y * WetStage<T>::kBand, 1);
-      const int rz = min((int)blockIdx.y * WetStage<T>::kBand + WetStage<T>::kBand - 1, rows - 2);
-      const int ca = max((int)blockIdx.x * kWetCols, 1), cz = min((int)blockIdx.x * kWetCols + kWetCols - 1, cols - 2);
-      if (rz >= ra && cz >= ca)
-        atomicAdd(&clk->skipped[1][(blockIdx.x + blockIdx.y * 7) % kSkipSlots],
-                  (unsigned long long)(rz - ra + 1) * (cz - ca + 1));
+  if (!clk->now.active) return;
+  const int lane = threadIdx.x & 31;
+  const unsigned warps = gridDim.x * (kWetCols / 32);
+  const PostArgs<T> P = post_args<T>(clk->now, sb, bed, maxh, arrival, arrival_depth, rows, cols, rb, hextra);
+  const uint8_t* flags = nullptr;
+  if (tflag != nullptr && *clk->maxh_neg == 0) flags = tflag + (size_t)clk->now.dst * ntiles;
+  T dmax = T(-1);
+  unsigned skipped = 0;  // interior cells of the tiles this lane found dry
+  // the warp's tiles are t, t + warps, ...; 32 of them are looked at at once
+  for (unsigned t = blockIdx.x * (kWetCols / 32) + (threadIdx.x >> 5); t < ntiles; t += 32 * warps) {
+    const uint64_t mine = t + (uint64_t)lane * warps;
+    bool todo = mine < ntiles;
+    if (todo && flags != nullptr && flags[mine]) {
+      todo = false;
+      skipped += tile_cells((unsigned)mine, rows, cols, rb);
     }
-    return;
+    for (unsigned left = __ballot_sync(0xffffffffu, todo); left != 0; left &= left - 1)
+      dmax = post_tile<T>(P, t + (unsigned)(__ffs(left) - 1) * warps, lane, dmax);
   }
-  const unsigned long long key = wetdry_staged<T>(clk, sb, bed, maxh, rows, cols, hextra, arrival, arrival_depth,
-                                                  blockIdx.x, blockIdx.y, reinterpret_cast<T*>(wet_smem));
-  block_min_into(key, &clk->dt_key[clk->wr]);
+  skipped = __reduce_add_sync(0xffffffffu, skipped);
+  if (lane == 0 && skipped)
+    atomicAdd(&clk->skipped[1][(blockIdx.x * 4 + (threadIdx.x >> 5)) % kSkipSlots], (unsigned long long)skipped);
+  block_min_into(dmax >= T(0) ? speed_key((double)dmax) : kDtKeyInf, &clk->dt_key[clk->now.wr]);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (clk->wait_test) wait_test(clk);
+    fold_accounts(clk);
+    end_step(clk);  // writes nothing that the other blocks read
+  }
 }
 
 // ===========================================================================
@@ -1301,11 +1415,17 @@ __global__ void __launch_bounds__(kWetCols) k_wetdry_staged(DevClock* __restrict
 // take tiles from one queue over all members' tiles, the wet-dry kernel's
 // blocks are a concatenation of every member's bands.
 // ===========================================================================
+// The first step's clocks of an advance; later ones are run by the post kernel.
 template <typename T>
 __global__ void k_batch_clock(const MemberDev<T>* __restrict__ mem, int nm, BatchCtl* __restrict__ ctl) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m == 0) ctl->tile_next = 0;
-  if (m < nm && clock_step(mem[m].clk)) atomicAdd(&ctl->halted, 1);
+  if (m < nm) mem[m].clk->now = begin_step(mem[m].clk);
+}
+
+template <typename T>
+__device__ __forceinline__ FluxCtx<T> member_ctx(const MemberDev<T>& M) {
+  return flux_ctx<T>(M.clk, M.clk->now, M.sb, M.bed, M.n2, M.zone, M.rates, M.rows, M.cols, M.rb, M.dx, M.rdx, M.hextra);
 }
 
 template <typename T, int MINB>
@@ -1314,89 +1434,54 @@ __global__ void __launch_bounds__(128, MINB) k_batch_flux(const MemberDev<T>* __
                                                           BatchCtl* __restrict__ ctl, uint32_t ntiles) {
   __shared__ FluxCtx<T> s_ctx[4];  // the member context of each warp's tile
   const int lane = threadIdx.x & 31;
+  pdl_wait();
   while (true) {
     unsigned tile = 0;
     if (lane == 0) tile = atomicAdd(&ctl->tile_next, 1u);
     tile = __shfl_sync(0xffffffffu, tile, 0);
     if (tile >= ntiles) break;
     const MemberDev<T>& M = mem[tile_member[tile]];
-    if (!M.clk->active) continue;
+    if (!M.clk->now.active) continue;
     __syncwarp();  // the warp's previous tile no longer reads its context
-    if (lane == 0)
-      s_ctx[threadIdx.x >> 5] = flux_ctx<T>(M.clk, M.sb, M.bed, M.n2, M.zone, M.rates, M.rows, M.cols, M.rb, M.dx,
-                                            M.rdx, M.hextra);
+    FluxCtx<T>& X = s_ctx[threadIdx.x >> 5];
+    if (lane == 0) X = member_ctx<T>(M);
     __syncwarp();
-    flux_tile_member<T>(s_ctx[threadIdx.x >> 5], tile - M.tile_begin, lane);
+    flux_tile_member<T>(X, tile - M.tile_begin, lane);
   }
+  pdl_trigger();
 }
 
+// The post kernel of every member: block b serves member post_member[b], whose
+// warps share the member's tiles.  A member's last block folds its volume
+// accounts and runs its clock for the next step, which the other members'
+// blocks hide (a kernel for all clocks took 6 to 7 us a step).
 template <typename T>
-__global__ void __launch_bounds__(kWetCols) k_batch_wetdry(const MemberDev<T>* __restrict__ mem,
-                                                            const int32_t* __restrict__ wet_member) {
-  extern __shared__ __align__(128) unsigned char wet_smem[];
-  const MemberDev<T>& M = mem[wet_member[blockIdx.x]];
+__global__ void __launch_bounds__(kWetCols, PostBlocks<T>::batch)
+    k_batch_post(const MemberDev<T>* __restrict__ mem, const int32_t* __restrict__ post_member,
+                 BatchCtl* __restrict__ ctl) {
+  pdl_wait();
+  pdl_trigger();
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctl->tile_next = 0;  // this step's flux launch is done
+  const MemberDev<T>& M = mem[post_member[blockIdx.x]];
   DevClock* clk = M.clk;
-  if (!clk->active) return;
-  const uint32_t local = blockIdx.x - M.wet_begin;
-  if (local == 0 && threadIdx.x == 0) fold_accounts(clk);
-  const unsigned long long key =
-      wetdry_staged<T>(clk, M.sb, M.bed, M.maxh, M.rows, M.cols, M.hextra, M.arrival, M.arrival_depth,
-                       (int)(local % M.wet_nbx), (int)(local / M.wet_nbx), reinterpret_cast<T*>(wet_smem));
-  block_min_into(key, &clk->dt_key[clk->wr]);
-}
-
-// Open-boundary ghosts of the batch members that have open edges: block row
-// y serves member open_members[y].
-template <typename T>
-__global__ void k_batch_open_bc(const MemberDev<T>* __restrict__ mem, const int32_t* __restrict__ open_members) {
-  const MemberDev<T>& M = mem[open_members[blockIdx.y]];
-  if (!M.clk->active) return;
-  open_bc_item<T>(M.clk, M.sb, M.rows, M.cols, blockIdx.x * blockDim.x + threadIdx.x);
-}
-
-// Point source `id` of member M (compute_flow, kernels.h:51-84).
-template <typename T>
-__device__ __forceinline__ void source_apply(const MemberDev<T>& M, int id) {
-  DevClock* clk = M.clk;
-  const int lo = clk->src_idx_low, hi = clk->src_idx_high;
-  const T dt = T(clk->global_dt), simtime = T(clk->t_step);
-  T* h = M.sb.H(clk->dst);
-  const T flo = M.hyg_v[(size_t)lo * M.nsrc + id], fhi = M.hyg_v[(size_t)hi * M.nsrc + id];
-  const T tlo = T(M.hyg_t[lo]), thi = T(M.hyg_t[hi]);
-  T flow;
-  if (lo == hi) {
-    flow = flo;
-  } else {
-    const T td = simtime - tlo, td2 = thi - tlo;
-    flow = flo + (((fhi - flo) * td) / td2);
+  if (!clk->now.active) return;
+  const PostArgs<T> P = post_args<T>(clk->now, M.sb, M.bed, M.maxh, M.arrival, M.arrival_depth, M.rows, M.cols, M.rb,
+                                     M.hextra);
+  const unsigned warps = M.post_count * (kWetCols / 32), ntiles = M.tile_end - M.tile_begin;
+  T dmax = T(-1);
+  for (unsigned t = (blockIdx.x - M.post_begin) * (kWetCols / 32) + (threadIdx.x >> 5); t < ntiles; t += warps)
+    dmax = post_tile<T>(P, t, threadIdx.x & 31, dmax);
+  block_min_into(dmax >= T(0) ? speed_key((double)dmax) : kDtKeyInf, &clk->dt_key[clk->now.wr]);
+  if (threadIdx.x == 0) {  // block_min_into's atomic was this thread's
+    __threadfence();
+    if (atomicAdd(&clk->post_done, 1u) == M.post_count - 1) {
+      __threadfence();
+      clk->post_done = 0;
+      fold_accounts(clk);
+      if (end_step(clk)) atomicAdd(&ctl->halted, 1);
+      clk->now = begin_step(clk);
+    }
   }
-  const int sid = M.src_cells[id];
-  T hij = h[sid];
-  const T hs = (flow * dt) / (M.dx * M.dx);
-  hij += hs;
-  h[sid] = hij;
-  atomicAdd(&clk->acc_step[kAccSources], (double)hs);
-}
-
-// Sparse forcing of a batch: items are (member, index) pairs of one
-// conflict-free wave (a member's own waves keep its index order).
-template <typename T>
-__global__ void k_batch_sources(const MemberDev<T>* __restrict__ mem, const int2* __restrict__ items, int count) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  const MemberDev<T>& M = mem[items[k].x];
-  if (!M.clk->active) return;
-  source_apply<T>(M, items[k].y);
-}
-
-template <typename T>
-__global__ void k_batch_extbc(const MemberDev<T>* __restrict__ mem, const int2* __restrict__ items, int count) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  const MemberDev<T>& M = mem[items[k].x];
-  if (!M.clk->active) return;
-  extbc_apply<T>(M.clk, M.sb, M.bed, M.n2, items[k].y, M.bc_cells, M.bc_types, M.bc_start, M.bc_nrows, M.bc_v1,
-                 M.bc_v2, M.rows, M.cols);
 }
 
 // ===========================================================================
@@ -1428,18 +1513,17 @@ __device__ __forceinline__ void forcing_block(const MemberDev<T>& M) {
   DevClock* clk = M.clk;
   for (int w = 0; w < M.src_nw; ++w) {
     for (int i = M.src_woff[w] + (int)threadIdx.x; i < M.src_woff[w + 1]; i += blockDim.x)
-      source_apply<T>(M, M.src_order[i]);
+      source_apply<T>(clk, clk->now, M.sb, M.f, M.dx, M.src_order[i]);
     __syncthreads();
   }
   if (M.open) {
     const int n = max(M.rows, M.cols);
-    for (int k = threadIdx.x; k < n; k += blockDim.x) open_bc_item<T>(clk, M.sb, M.rows, M.cols, k);
+    for (int k = threadIdx.x; k < n; k += blockDim.x) open_bc_item<T>(clk->now.dst, M.sb, M.rows, M.cols, k);
     __syncthreads();
   }
   for (int w = 0; w < M.bc_nw; ++w) {
     for (int i = M.bc_woff[w] + (int)threadIdx.x; i < M.bc_woff[w + 1]; i += blockDim.x)
-      extbc_apply<T>(clk, M.sb, M.bed, M.n2, M.bc_order[i], M.bc_cells, M.bc_types, M.bc_start, M.bc_nrows,
-                     M.bc_v1, M.bc_v2, M.rows, M.cols);
+      extbc_apply<T>(clk, clk->now, M.sb, M.bed, M.n2, M.bc_order[i], M.f, M.rows, M.cols);
     __syncthreads();
   }
 }
@@ -1497,11 +1581,10 @@ __device__ __forceinline__ void steps_flux_item(const MemberDev<T>* __restrict__
     *seen_m = (uint32_t)m;
     *seen_s = s;
   }
-  if (M.clk->active) {
+  if (M.clk->now.active) {
     __shared__ FluxCtx<T> s_ctx[4];  // the member context of each warp's tile, reread every row
     if (lane == 0)
-      s_ctx[warp] = flux_ctx<T>(M.clk, M.sb, M.bed, M.n2, M.zone, M.rates, M.rows, M.cols, M.rb, M.dx, M.rdx,
-                                M.hextra);
+      s_ctx[warp] = member_ctx<T>(M);
     __syncwarp();
     flux_tile_member<T>(s_ctx[warp], tile - M.tile_begin, lane);
   }
@@ -1520,7 +1603,8 @@ __device__ __noinline__ void steps_clock_item(const MemberDev<T>& M, uint32_t m,
   // handling of a wait that gave up can be tested with nothing else wrong
   if (ctl->wait_test != 0 && m == 0 && s == 0) steps_wait(&prog[0].clock, 0xFFFFFFFFu, ctl, ctl->wait_test);
   steps_wait(&prog[m].wet, s * M.wet_count, ctl);
-  if (clock_step(M.clk)) atomicAdd(&ctl->halted, 1);
+  M.clk->now = begin_step(M.clk);
+  if (M.clk->now.active && end_step(M.clk)) atomicAdd(&ctl->halted, 1);
   __threadfence();
   atomicAdd(&prog[m].clock, 1u);
 }
@@ -1529,7 +1613,7 @@ template <typename T>
 __device__ __noinline__ void steps_forcing_item(const MemberDev<T>& M, uint32_t m, uint32_t s,
                                                 BatchCtl* __restrict__ ctl, MemberProgress* __restrict__ prog) {
   acquire_block(&prog[m].flux, (s + 1) * (M.tile_end - M.tile_begin), ctl);
-  if (M.clk->active) forcing_block<T>(M);
+  if (M.clk->now.active) forcing_block<T>(M);
   publish_block(&prog[m].forcing);
 }
 
@@ -1552,14 +1636,14 @@ __device__ __noinline__ bool steps_wet_item(const MemberDev<T>* __restrict__ mem
   }
   DevClock* clk = M.clk;
   bool broken = false;
-  if (clk->active) {
+  if (clk->now.active) {
     fence_proxy_async_global();  // the bulk copies read what other blocks wrote
     const uint32_t local = r - M.wet_begin;
     if (local == 0 && threadIdx.x == 0) fold_accounts(clk);
     const unsigned long long key =
         wetdry_staged<T>(clk, M.sb, M.bed, M.maxh, M.rows, M.cols, M.hextra, M.arrival, M.arrival_depth,
                          (int)(local % M.wet_nbx), (int)(local / M.wet_nbx), reinterpret_cast<T*>(smem));
-    block_min_into(key, &clk->dt_key[clk->wr]);
+    block_min_into(key, &clk->dt_key[clk->now.wr]);
     broken = __syncthreads_or(clk->status == kStatusStageTimeout) != 0;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + S::kData);
     if (!broken && threadIdx.x < S::kGroups) mbar_inval(&bar[threadIdx.x]);

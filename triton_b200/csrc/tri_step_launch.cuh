@@ -79,36 +79,33 @@ template <typename T>
 int launch_step(const StepArgs& a, cudaStream_t s, cudaEvent_t* ev) {
   const int rows = a.rows, cols = a.cols;
   const T dx = (T)a.dx, hx = (T)a.hextra, rdx = (T)(1.0 / a.dx);
-  StateBufs<T> sb = bufs_of<T>(a);
+  const StateBufs<T> sb = bufs_of<T>(a);
   const BedMap<T> bed = bed_of<T>(a);
-  TRI_CUDA_TRY(launch_pdl(k_clock, 1, 32, 0, s, a.clk));
+  ForcingDev<T> f;
+  f.nsrc = a.nsrc;
+  f.src_cells = a.src_cells;
+  f.hyg_t = a.hyg_t;
+  f.hyg_v = (const T*)a.hyg_v;
+  f.bc_cells = a.bc_cells;
+  f.bc_types = a.bc_types;
+  f.bc_start = a.bc_start;
+  f.bc_nrows = a.bc_nrows;
+  f.bc_v1 = (const T*)a.bc_v1;
+  f.bc_v2 = (const T*)a.bc_v2;
   if (ev) cudaEventRecord(ev[0], s);
-  if (a.tzero != nullptr)  // dry-tile skipping
-    TRI_CUDA_TRY(launch_pdl(flux_kernel<T, true>(a.flux_variant), a.flux_blocks, 128, 0, s, a.clk, sb, bed,
-                            (const T*)a.n2, a.zone, (const T*)a.rates, rows, cols, a.rb, dx, rdx, hx, a.tzero));
-  else
-    TRI_CUDA_TRY(launch_pdl(flux_kernel<T, false>(a.flux_variant), a.flux_blocks, 128, 0, s, a.clk, sb, bed,
-                            (const T*)a.n2, a.zone, (const T*)a.rates, rows, cols, a.rb, dx, rdx, hx, a.tzero));
+  const auto k = a.skip_dry ? flux_kernel<T, true>(a.flux_variant) : flux_kernel<T, false>(a.flux_variant);
+  TRI_CUDA_TRY(launch_pdl(k, a.flux_blocks, 128, 0, s, a.clk, sb, bed, (const T*)a.n2, a.zone, (const T*)a.rates,
+                          rows, cols, a.rb, dx, rdx, hx, a.tflag));
   if (ev) cudaEventRecord(ev[1], s);
-  for (int w = 0; a.nsrc > 0 && w < a.n_src_waves; w++) {
-    const int off = a.src_waves[w], cnt = a.src_waves[w + 1] - off;
-    TRI_CUDA_TRY(launch_pdl(k_sources<T>, (cnt + 127) / 128, 128, 0, s, a.clk, sb, a.src_order + off, cnt, a.nsrc,
-                            a.src_cells, a.hyg_t, (const T*)a.hyg_v, dx));
-  }
-  if (a.open_boundaries) {
-    const int n = std::max(rows, cols);
-    TRI_CUDA_TRY(launch_pdl(k_open_bc<T>, (n + 255) / 256, 256, 0, s, a.clk, sb, rows, cols));
-  }
-  for (int w = 0; a.nbc > 0 && w < a.n_bc_waves; w++) {
-    const int off = a.bc_waves[w], cnt = a.bc_waves[w + 1] - off;
-    TRI_CUDA_TRY(launch_pdl(k_extbc<T>, (cnt + 127) / 128, 128, 0, s, a.clk, sb, bed, (const T*)a.n2,
-                            a.bc_order + off, cnt, a.bc_cells, a.bc_types, a.bc_start, a.bc_nrows, (const T*)a.bc_v1,
-                            (const T*)a.bc_v2, rows, cols));
-  }
-  dim3 g2((cols + kWetCols - 1) / kWetCols, (rows + WetStage<T>::kBand - 1) / WetStage<T>::kBand);
+  if (a.tf.count > 0)
+    TRI_CUDA_TRY(launch_pdl(k_forcing<T>, (a.tf.count + 3) / 4, 128, 0, s, a.clk, sb, bed, (const T*)a.n2, f, a.tf,
+                            a.open_boundaries != 0, dx, rows, cols, a.rb));
   if (ev) cudaEventRecord(ev[2], s);
-  TRI_CUDA_TRY(launch_pdl(k_wetdry_staged<T>, g2, kWetCols, WetStage<T>::kBytes, s, a.clk, sb, bed, (T*)a.maxh,
-                          rows, cols, hx, a.arrival, a.arrival_depth, a.tzero_wet, a.rb, a.maxh_neg));
+  // with arrival tracking of a negative depth dry cells count, too
+  const bool skip_dry = a.skip_dry && (a.arrival == nullptr || a.arrival_depth >= 0.0f);
+  TRI_CUDA_TRY(launch_pdl(k_post<T>, post_blocks(a.ntiles, a.ntiles, PostBlocks<T>::v), kWetCols, 0, s, a.clk, sb, bed, (T*)a.maxh,
+                          rows, cols, hx, a.arrival, a.arrival_depth, (const uint8_t*)(skip_dry ? a.tflag : nullptr),
+                          a.rb, a.ntiles));
   if (ev) cudaEventRecord(ev[3], s);
   TRI_CUDA_TRY(cudaGetLastError());
   return TRI_OK;
@@ -116,9 +113,9 @@ int launch_step(const StepArgs& a, cudaStream_t s, cudaEvent_t* ev) {
 
 template <typename T>
 int launch_initial_dt(const StepArgs& a, cudaStream_t s) {
-  dim3 g2((a.cols + kWetCols - 1) / kWetCols, (a.rows + kWetBand - 1) / kWetBand);
-  k_wetdry_dt<T, false><<<g2, kWetCols, 0, s>>>(a.clk, bufs_of<T>(a), bed_of<T>(a), (T*)a.maxh, a.rows, a.cols,
-                                                kWetBand, a.dx, a.courant, (T)a.hextra, nullptr, 0.0f);
+  const int64_t n = (int64_t)a.rows * a.cols;
+  const unsigned blocks = (unsigned)std::min<int64_t>((n + 4 * kWetCols - 1) / (4 * kWetCols), 148 * 16);
+  k_initial_dt<T><<<blocks, kWetCols, 0, s>>>(a.clk, bufs_of<T>(a), n, (T)a.hextra);
   TRI_CUDA_TRY(cudaGetLastError());
   return TRI_OK;
 }
@@ -129,22 +126,20 @@ void batch_flux_occupancy(int variant, int* per_sm) {
 }
 
 template <typename T>
+int launch_batch_clock(const BatchArgs& a, cudaStream_t s) {
+  k_batch_clock<T><<<(a.nm + 127) / 128, 128, 0, s>>>((const MemberDev<T>*)a.mem, a.nm, a.ctl);
+  TRI_CUDA_TRY(cudaGetLastError());
+  return TRI_OK;
+}
+
+template <typename T>
 int launch_batch_step(const BatchArgs& a, cudaStream_t s) {
   const MemberDev<T>* mem = (const MemberDev<T>*)a.mem;
-  k_batch_clock<T><<<(a.nm + 127) / 128, 128, 0, s>>>(mem, a.nm, a.ctl);
-  batch_flux_kernel<T>(a.flux_variant)<<<a.flux_blocks, 128, 0, s>>>(mem, a.tile_member, a.ctl, a.ntiles);
-  for (int w = 0; w < a.n_src_waves; w++) {
-    const int off = a.src_waves[w], cnt = a.src_waves[w + 1] - off;
-    k_batch_sources<T><<<(cnt + 127) / 128, 128, 0, s>>>(mem, a.src_items + off, cnt);
-  }
-  if (a.n_open > 0)
-    k_batch_open_bc<T><<<dim3((unsigned)((a.open_dim + 255) / 256), (unsigned)a.n_open), 256, 0, s>>>(
-        mem, a.open_members);
-  for (int w = 0; w < a.n_bc_waves; w++) {
-    const int off = a.bc_waves[w], cnt = a.bc_waves[w + 1] - off;
-    k_batch_extbc<T><<<(cnt + 127) / 128, 128, 0, s>>>(mem, a.bc_items + off, cnt);
-  }
-  k_batch_wetdry<T><<<a.nwet_blocks, kWetCols, WetStage<T>::kBytes, s>>>(mem, a.wet_member);
+  TRI_CUDA_TRY(launch_pdl(batch_flux_kernel<T>(a.flux_variant), a.flux_blocks, 128, 0, s, mem, a.tile_member, a.ctl,
+                          a.ntiles));
+  if (a.tf.count > 0)
+    TRI_CUDA_TRY(launch_pdl(k_batch_forcing<T>, (a.tf.count + 3) / 4, 128, 0, s, mem, a.tile_member, a.tf));
+  TRI_CUDA_TRY(launch_pdl(k_batch_post<T>, a.npost_blocks, kWetCols, 0, s, mem, a.post_member, a.ctl));
   TRI_CUDA_TRY(cudaGetLastError());
   return TRI_OK;
 }
@@ -177,10 +172,6 @@ int prepare_kernels() {
   for (int v = 0; v < 2; v++)
     TRI_CUDA_TRY(cudaFuncSetAttribute(steps_kernel<T>(v), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)WetStage<T>::kBytes));
-  TRI_CUDA_TRY(cudaFuncSetAttribute(k_wetdry_staged<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)WetStage<T>::kBytes));
-  TRI_CUDA_TRY(cudaFuncSetAttribute(k_batch_wetdry<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)WetStage<T>::kBytes));
   return TRI_OK;
 }
 

@@ -15,7 +15,6 @@ namespace tri {
 constexpr int kStripCols = 30;   // interior columns per warp tile of the flux kernel
 constexpr int kFluxVariants = 5; // register budgets (FluxBudget)
 constexpr int kWetCols = 128;    // columns per block of the wet-dry/dt kernel
-constexpr int kWetBand = 16;     // rows per block of the initial-dt kernel
 // Blocks of 128 threads per SM that the flux kernel's register-budget
 // variants are compiled for (__launch_bounds__ minimum).  FP64: 122, 96, 80,
 // 72 and 64 registers a thread (from 96 down they spill to L1, 8 to 300
@@ -62,7 +61,24 @@ FluxShape flux_shape(bool fp64, double share, F tiles) {
     if (share * (double)tiles(rb) >= 4 * slots) best = rb;
   return {fp64 ? 0 : 2, best};
 }
-// rows per block of the staged wet-dry/dt kernel (its shared-memory tile),
+// Blocks of 128 threads per SM that the post kernels are compiled for: a stream
+// with two rows of loads in flight per warp, so as many as its registers allow
+// without spills (the batched one reads its parameters from memory and needs
+// more).  FP64 at 8, 6 and 5: bowl 2048^2 33.2, 29.9 and 33.1 us with 4 us of
+// timing, a 10-member ensemble step 110, 107.5 and 103.5 us; FP32 at 10, 8 and
+// 7: rain on 4096^2 96, 110 and 127 us, a 24-member ensemble step 299, 247 and
+// 253 us.
+template <typename T>
+struct PostBlocks;
+template <>
+struct PostBlocks<double> {
+  static constexpr int v = 6, batch = 5;
+};
+template <>
+struct PostBlocks<float> {
+  static constexpr int v = 10, batch = 8;
+};
+// rows per block of the staged wet-dry/dt pass (its shared-memory tile),
 // and output rows per group of its copies (each group on its own mbarrier)
 template <typename T>
 constexpr int kStageBand = sizeof(T) == 8 ? 4 : 8;
@@ -84,34 +100,33 @@ struct StepArgs {
   int rows, cols;
   int rb, flux_blocks, flux_variant;
   double dx, courant, hextra;
-  int open_boundaries;
   int nsrc;
   const int32_t* src_cells;
-  const int32_t* src_order;
   const double* hyg_t;
   const void* hyg_v;
-  const int32_t* src_waves;  // host array, n_src_waves + 1 offsets
-  int n_src_waves;
-  int nbc;
-  const int32_t *bc_cells, *bc_types, *bc_start, *bc_nrows, *bc_order;
+  const int32_t *bc_cells, *bc_types, *bc_start, *bc_nrows;
   const void *bc_v1, *bc_v2;
-  const int32_t* bc_waves;  // host array, n_bc_waves + 1 offsets
-  int n_bc_waves;
   float* arrival;
   float arrival_depth;
-  // dry-tile flags of the flux kernel ([2][tiles] by buffer + [tiles]
-  // pinned), or null to compute every tile; the same for the wet-dry kernel
-  // (null also while the arrival depth is negative), which skips bands only
-  // while *maxh_neg (an uploaded max depth is negative) is 0
-  uint8_t* tzero;
-  const uint8_t* tzero_wet;
-  const int32_t* maxh_neg;
+  // tile flags of the flux kernel ([2][tiles] by buffer + [tiles] pinned),
+  // forcing by tile; skip_dry: dry tiles are skipped
+  uint8_t* tflag;
+  uint32_t ntiles;
+  TileForcing tf;
+  int open_boundaries;
+  bool skip_dry;
 };
 
-// One time step (clock, flux/update, sources, open ghosts, boundary cells,
-// wet-dry/dt).  ev: optional 4 events around the flux and wet-dry launches.
+// One time step (flux/update, forcing, post kernel).  ev: optional 4
+// events around the two launches.
 template <typename T>
 int launch_step(const StepArgs& a, cudaStream_t s, cudaEvent_t* ev);
+// Blocks of the post kernel (4 warps each, `per_sm` resident on an SM) for
+// `tiles` flux tiles, `all` of them in the launch.
+inline uint32_t post_blocks(uint32_t tiles, uint32_t all, uint32_t per_sm) {
+  const uint32_t per = (all + 148 * 4 * per_sm - 1) / (148 * 4 * per_sm);  // tiles per warp
+  return (tiles + 4 * per - 1) / (4 * per);
+}
 // CFL dt of the current state into the slot the next step reads.
 template <typename T>
 int launch_initial_dt(const StepArgs& a, cudaStream_t s);
@@ -128,15 +143,13 @@ struct BatchArgs {
   BatchCtl* ctl;
   uint32_t ntiles, nwet_blocks;
   int flux_blocks, flux_variant;
-  const int2* src_items;
-  const int32_t* src_waves;
-  int n_src_waves;
-  const int2* bc_items;
-  const int32_t* bc_waves;
-  int n_bc_waves;
-  const int32_t* open_members;  // members with open edges (device), their count and largest max(rows, cols)
-  int n_open, open_dim;
+  const int32_t* post_member;  // member of every post kernel block
+  uint32_t npost_blocks;
+  TileForcing tf;
 };
+// The members' clocks of the first batched step of an advance.
+template <typename T>
+int launch_batch_clock(const BatchArgs& a, cudaStream_t s);
 template <typename T>
 int launch_batch_step(const BatchArgs& a, cudaStream_t s);
 // Single-launch mode: nsteps batched steps in one launch of k_batch_steps
@@ -163,6 +176,8 @@ extern template int launch_initial_dt<double>(const StepArgs&, cudaStream_t);
 extern template int launch_initial_dt<float>(const StepArgs&, cudaStream_t);
 extern template void flux_occupancy<double>(int, int*);
 extern template void flux_occupancy<float>(int, int*);
+extern template int launch_batch_clock<double>(const BatchArgs&, cudaStream_t);
+extern template int launch_batch_clock<float>(const BatchArgs&, cudaStream_t);
 extern template int launch_batch_step<double>(const BatchArgs&, cudaStream_t);
 extern template int launch_batch_step<float>(const BatchArgs&, cudaStream_t);
 extern template int launch_batch_steps<double>(const BatchArgs&, MemberProgress*, int, int, cudaStream_t);

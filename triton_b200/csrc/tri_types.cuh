@@ -20,27 +20,43 @@ enum { kAccBoundary = 0, kAccSources = 1, kAccRunoff = 2, kAccExtbc = 3, kAccCli
 // Slots of the skipped-cell counters in DevClock.
 constexpr int kSkipSlots = 32;
 
+// The parameters of the running time step, formed from the loop state
+// (begin_step): the dt policy's outcome, table rows, buffers.
+struct StepNow {
+  double dt, rdt;      // time step, RN(1/dt)
+  double t_step, t_end;  // simtime at its start and end
+  int32_t src, dst;    // state buffers
+  int32_t wr;          // dt slot its wave speeds go to
+  int32_t runoff_row, src_idx_low, src_idx_high;
+  int32_t step;        // it_count including this step
+  int32_t events;      // TRI_EV_* it raises
+  int32_t active;      // 0: halted or past the limit, nothing runs
+};
+
 // Device-resident loop state.  Host mirror: tri_clock plus the bookkeeping
-// fields below.
+// fields below.  It stands still during a step (every block of the flux kernel
+// forms 'now' from it by itself) and moves on when the step ends (end_step).
 struct DevClock {
   double simtime, sim_duration, print_interval, print_observation, last_obs_time;
   double init_dt, time_step, average_dt, global_dt;
-  double t_step;  // simtime at the start of the running step
-  double rdt;     // RN(1/global_dt)
   double cfl_a;   // RN(courant * dx): the CFL dt is cfl_a / (largest wave speed)
   int32_t print_id, it_count, it_print, time_series, time_increment_fixed;
-  int32_t runoff_row, src_idx_low, src_idx_high;
-  int32_t active, halt, events, steps;
-  int32_t cur, src, dst, rd, wr;  // ping-pong state buffers and dt slots
+  int32_t runoff_row, src_idx_low;
+  int32_t halt, events, steps;
+  int32_t cur, rd;  // state buffer and dt slot of the current state; the other slot is empty
+  int32_t limit;    // steps the running advance call may take (the clock then stands still)
   int32_t nroff, roff_rows, nsrc, hyg_rows;
   int32_t status;  // nonzero: a device-side check failed (value = reason)
   uint32_t tile_next;  // work counter of the flux kernel's dynamic tiles, reset every step
+  uint32_t post_done;  // batches: blocks of the running step's post kernel that are done
   uint32_t wait_test;  // test hook: nonzero = polls of a wait nothing completes (tri_domain_set_wait_test)
   unsigned long long dt_key[2];
   const double* roff_t;
   const double* hyg_t;
+  const int32_t* maxh_neg;  // nonzero: a max depth that was uploaded is negative or NaN
+  StepNow now;
   // FP64 volume accounting in depth units (multiply by dx^2), both forms.
-  // acc_step collects the running step (atomics), the wet-dry kernel folds it
+  // acc_step collects the running step (atomics), the post kernel folds it
   // into the Kahan-compensated totals acc_sum/acc_comp.
   double acc_step[kAccTerms];
   double acc_sum[kAccTerms];
@@ -102,6 +118,29 @@ struct BedMap<float> {
   }
 };
 
+// The forcing that writes into cells after their flux update, sorted by the
+// flux tile that holds the cell (an external boundary cell's ghosts belong to
+// its tile, too).  Entry k is tile tiles[k] with the groups group_of[k] ..
+// group_of[k+1]; group g has the items item_of[g] .. item_of[g+1]; an item is
+// a source index, or -1 - j for external boundary cell j.  Items of one group
+// touch different cells; groups keep the reference's order (sources, then
+// boundary cells; the ghosts of open edges between the two).
+struct TileForcing {
+  const int32_t *tiles, *group_of, *item_of, *items;
+  int count;
+};
+
+// Forcing tables of one domain (device arrays).
+template <typename T>
+struct ForcingDev {
+  int nsrc;
+  const int32_t* src_cells;
+  const double* hyg_t;
+  const T* hyg_v;
+  const int32_t *bc_cells, *bc_types, *bc_start, *bc_nrows;
+  const T *bc_v1, *bc_v2;
+};
+
 template <typename T>
 struct MemberDev {
   DevClock* clk;
@@ -118,13 +157,8 @@ struct MemberDev {
   double dxd, courant;
   uint32_t tile_begin, tile_end;  // this member's tiles in the flux queue
   uint32_t wet_begin, wet_nbx;    // first wet-dry block, blocks per band row
-  // sparse forcing (device arrays of the member)
-  int nsrc;
-  const int32_t* src_cells;
-  const double* hyg_t;
-  const T* hyg_v;
-  const int32_t *bc_cells, *bc_types, *bc_start, *bc_nrows;
-  const T *bc_v1, *bc_v2;
+  uint32_t post_begin, post_count;  // blocks of the post kernel
+  ForcingDev<T> f;
   // single-launch mode (k_batch_steps): the member's wet-dry block count and
   // its forcing as conflict-free waves of its own items (order: device item
   // indices wave after wave, woff: nw+1 wave offsets), open edges
