@@ -316,18 +316,19 @@ int tri_kernel_copy_info_to_exterior_boundaries_north_south_f64(int size, int nr
                                                                 int total_process, void* stream);
 /* compute_extbc_values: cells that touch the same cell (corners shared by two
  * segments, repeated cells) are applied in index order, as the reference's
- * serial build does; to schedule them the entry reads the cell list back to
- * the host, so it synchronizes 'stream'.  The order is cached per host thread
- * and device, in device memory allocated on first use and grown for longer
- * lists (freed when the thread exits). */
+ * serial build does.  Up to 8192 cells the device finds that order itself and
+ * the call does not synchronize; for longer lists the entry reads the cell
+ * list back to the host, so it synchronizes 'stream', and the order is cached
+ * per host thread and device, in device memory allocated on first use and
+ * grown for longer lists (freed when the thread exits). */
 int tri_kernel_compute_extbc_values_f64(int size, int nrows, int ncols, double dt, double* h, double* qx, double* qy,
                                         const double* dem, const double* n, const int32_t* relative_index,
                                         const int32_t* extbctype, const int32_t* start_index,
                                         const int32_t* nrows_vars, const double* extbcvar1, const double* extbcvar2,
                                         double simtime, int rank, int total_process, void* stream);
 /* No-alloc variant of tri_kernel_compute_extbc_values_f64; it has no
- * counterpart in the reference.  Same arguments, same results, and it also
- * synchronizes 'stream'.  It allocates no device memory: the application
+ * counterpart in the reference.  Same arguments, same results; beyond 8192
+ * cells it, too, synchronizes 'stream'.  It allocates no device memory: the application
  * order is kept in a fixed array inside the library of
  * TRI_NOALLOC_EXTBC_MAX_CELLS entries (256 KiB), and a longer cell list is
  * rejected with TRI_E_INVALID.  For callers that cannot allocate device

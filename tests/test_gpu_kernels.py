@@ -153,3 +153,57 @@ def test_kernel_entry_points_match_oracle(oracle):
     _abi.check(L.tri_kernel_copy_observation_points_f64(obs.size, _p(dh), _p(dout), _p(dobs), None))
     torch.cuda.synchronize()
     assert np.array_equal(dout.cpu().numpy(), out_o)
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 1025, 9000])
+@pytest.mark.parametrize("odd", [False, True])
+def test_extbc_list_order_matches_oracle(oracle, n, odd):
+    """Boundary cells listed several times with different types, in any order
+    (each cell's items apply in list order), around the sizes of a block, of
+    the scan's chunk and beyond the scan's limit; a list with a ghost cell in
+    it is applied serially.  Types without a cube root: equal in every bit."""
+    import torch
+    from triton_b200 import _abi
+    L, O = _abi.lib(), oracle.lib()
+    O.tor_compute_extbc_values.restype = None
+    R, Cc = 43, 61
+    rng = np.random.default_rng(n)
+    edge = [r * Cc + c for r in range(1, R - 1) for c in range(1, Cc - 1) if r in (1, R - 2) or c in (1, Cc - 2)]
+    cells = rng.choice(np.array(edge, np.int32), n).astype(np.int32)
+    if odd:
+        cells[n // 2] = 1  # ghost (0, 1): its column has a western ghost
+    types = rng.choice(np.array([0, 1, 3], np.int32), n).astype(np.int32)
+    start = np.where(types == 1, 0, 4).astype(np.int32)
+    nrows = np.where(types == 1, 4, 1).astype(np.int32)
+    v1, v2 = np.array([0.0, 5.0, 9.0, 30.0, 0.7]), np.array([6.0, 7.0, 6.5, 6.5, 0.7])
+    h = rng.random(R * Cc) * 2.0
+    qx, qy = rng.standard_normal(R * Cc), rng.standard_normal(R * Cc)
+    z, n2 = 5.0 + rng.random(R * Cc), np.full(R * Cc, 1e-3)
+    dev = [_dev(torch, a.copy()) for a in (h, qx, qy, z, n2, cells, types, start, nrows, v1, v2)]
+    O.tor_compute_extbc_values(n, R, Cc, C.c_double(0.1), *[a.ctypes.data_as(_dp) for a in (h, qx, qy, z, n2)],
+                               *[a.ctypes.data_as(_ip) for a in (cells, types, start, nrows)],
+                               v1.ctypes.data_as(_dp), v2.ctypes.data_as(_dp), C.c_double(7.0))
+    _abi.check(L.tri_kernel_compute_extbc_values_f64(n, R, Cc, 0.1, *[_p(t) for t in dev], 7.0, 0, 1, None))
+    torch.cuda.synchronize()
+    for a, t in zip((h, qx, qy), dev):
+        assert np.array_equal(t.cpu().numpy(), a)
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 100])
+def test_flow_of_sources_in_shared_cells_matches_oracle(oracle, n):
+    """Sources that share cells add up in source order, within a warp's 32
+    sources and across them."""
+    import torch
+    from triton_b200 import _abi
+    L, O = _abi.lib(), oracle.lib()
+    O.tor_compute_flow.restype = None
+    rng = np.random.default_rng(n)
+    h = rng.random(50)
+    pos = rng.choice(np.array([3, 17, 44], np.int32), n).astype(np.int32)
+    ht, hv = np.array([0.0, 4.0, 9.0]), rng.random(3 * n)
+    dh, dpos, dht, dhv = (_dev(torch, a.copy()) for a in (h, pos, ht, hv))
+    O.tor_compute_flow(n, ht.ctypes.data_as(_dp), hv.ctypes.data_as(_dp), C.c_double(3.0), C.c_double(0.07),
+                       C.c_double(3.0), 0, 1, h.ctypes.data_as(_dp), pos.ctypes.data_as(_ip))
+    _abi.check(L.tri_kernel_compute_flow_f64(n, _p(dht), _p(dhv), 3.0, 0.07, 3.0, 0, 1, _p(dh), _p(dpos), None))
+    torch.cuda.synchronize()
+    assert np.array_equal(dh.cpu().numpy(), h)
