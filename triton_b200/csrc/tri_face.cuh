@@ -28,38 +28,8 @@ namespace tri {
 template <typename T>
 struct CellQ {
   T h, qx, qy, z, sq, u, v;
+  T hd;  // h*dx/2/dt, the limiter's bound: the same for the cell's four faces
 };
-
-// LINE: the FP64 straight-line forms, for cells that regular_cell() accepts.
-template <typename T, bool LINE = false>
-__device__ __forceinline__ CellQ<T> make_cell(T h, T qx, T qy, T z, T hextra) {
-  CellQ<T> c;
-  c.h = h;
-  c.qx = qx;
-  c.qy = qy;
-  c.z = z;
-  if constexpr (LINE && sizeof(T) == 8) {
-    const double hs = h > 0.0 ? h : 1.0;
-    const double y = rsqrt_line(hs);
-    const double s = sqrt_line(hs, y);
-    const double rh = recip_line(hs, y * y);
-    const bool flows = h >= hextra;
-    c.sq = h > 0.0 ? s : 0.0;
-    c.u = flows ? div_line(qx, hs, rh) : 0.0;
-    c.v = flows ? div_line(qy, hs, rh) : 0.0;
-    return c;
-  }
-  c.sq = dev_fmax(dev_sqrt(h), T(0));
-  if (h >= hextra) {
-    const T rh = recip(h);
-    c.u = div_shared(qx, h, rh);
-    c.v = div_shared(qy, h, rh);
-  } else {
-    c.u = T(0);
-    c.v = T(0);
-  }
-  return c;
-}
 
 // Result of one face: contributions to the owner (a) and to the neighbour (b),
 // already scaled as rhs = dt*d/dx (kernels_flux.h:267-273).  'wet' is false for
@@ -101,6 +71,45 @@ __host__ __device__ inline StepK<T> step_k(T dx, T dt, T rdx, T rdt, T hextra) {
   return K;
 }
 
+// LINE: the FP64 straight-line forms, for cells that regular_cell() accepts.
+template <typename T, bool LINE = false>
+__device__ __forceinline__ CellQ<T> make_cell(T h, T qx, T qy, T z, const StepK<T>& K) {
+  const T hextra = K.hextra;
+  CellQ<T> c;
+  c.h = h;
+  c.qx = qx;
+  c.qy = qy;
+  c.z = z;
+  c.hd = div_nz(h * K.dx * T(0.5), K.dt, K.rdt);
+  if constexpr (LINE && sizeof(T) == 8) {
+    const double hs = h > 0.0 ? h : 1.0;
+    const double y = rsqrt_line(hs);
+    const double s = sqrt_line(hs, y);
+    const double rh = recip_line(hs, y * y);
+    const bool flows = h >= hextra;
+    c.sq = h > 0.0 ? s : 0.0;
+    c.u = flows ? div_line(qx, hs, rh) : 0.0;
+    c.v = flows ? div_line(qy, hs, rh) : 0.0;
+    return c;
+  }
+  c.sq = dev_fmax(dev_sqrt(h), T(0));
+  if constexpr (sizeof(T) == 4) {
+    const T rh = recip(h);
+    c.u = h >= hextra ? div_shared(qx, h, rh) : T(0);
+    c.v = h >= hextra ? div_shared(qy, h, rh) : T(0);
+    return c;
+  }
+  if (h >= hextra) {
+    const T rh = recip(h);
+    c.u = div_shared(qx, h, rh);
+    c.v = div_shared(qy, h, rh);
+  } else {
+    c.u = T(0);
+    c.v = T(0);
+  }
+  return c;
+}
+
 // Products with the face normal (nx, ny) = (1,0) or (0,1): the component
 // itself (the product with the zero component is a zero term).
 template <typename T, bool XFACE>
@@ -122,12 +131,13 @@ __device__ __forceinline__ float quot(float a, float b, float y) {
   return div_shared(a, b, y);
 }
 
-// dzb (FP32 form): base level of c2's bed tile minus that of c1's.
+// cross, dzb (FP32 form): the cells lie in different bed tiles; base level of
+// c2's minus that of c1's.
 // LINE (FP64): both cells are regular (regular_cell), so square roots,
 // reciprocals and shared quotients take their straight-line forms.
 template <typename T, bool XFACE, bool LINE = false>
 __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<T>& c2, const StepK<T>& K,
-                                                double dzb = 0.0) {
+                                                bool cross = false, double dzb = 0.0) {
   constexpr bool L64 = LINE && sizeof(T) == 8;
   const T dx = K.dx, dt = K.dt, hextra = K.hextra;
   const T G = T(kGravity), SG = T(kSqrtG), E12 = eps12<T>();
@@ -135,7 +145,8 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
   out.a0 = out.a1 = out.a2 = out.b0 = out.b1 = out.b2 = T(0);
 
   const T h1 = c1.h, h2 = c2.h;
-  if (!(h1 > T(0) || h2 > T(0))) return out;
+  const bool brink = h1 < E12 || h2 < E12;  // next to a dry cell
+  if (brink && !(h1 > T(0) || h2 > T(0))) return out;
 
   const T u1 = c1.u, v1 = c1.v, u2 = c2.u, v2 = c2.v;
   const T sqh1 = c1.sq, sqh2 = c2.sq;
@@ -161,6 +172,7 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
   const T un = n_dot<T, XFACE>(u12, v12);
   T lam0 = un - c12, lam1 = un, lam2 = un + c12;
   T lamE0 = T(0), lamE2 = T(0);  // lamE1 is always zero
+  bool fixed = false;
 
   // Harten-Hyman style entropy fix on the acoustic waves (rare: one branch)
   {
@@ -168,7 +180,8 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
     const T g1 = SG * sqh1, g2 = SG * sqh2;
     const T a1 = un1 - g1, a2 = un2 - g2, b1 = un1 + g1, b2 = un2 + g2;
     const bool fix0 = a1 < T(0) && a2 > T(0), fix2 = b1 < T(0) && b2 > T(0);
-    if (fix0 || fix2) {
+    fixed = fix0 || fix2;
+    if (fixed) {
       if (fix0) {
         const T t = div_rare(a1 * (a2 - lam0), a2 - a1);
         lamE0 = lam0 - t;
@@ -206,7 +219,8 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
     // FP32 form: the bed step from both cells' bases and offsets, so
     // every evaluation of a face gets the same value (a face on a tile edge
     // is evaluated by both tiles, and mass is conserved only if both agree)
-    dz = dzb == 0.0 ? c2.z - c1.z : (T)(dzb + ((double)c2.z - (double)c1.z));
+    dz = c2.z - c1.z;
+    if (cross) dz = (T)(dzb + ((double)c2.z - (double)c1.z));
     above1 = h1 < dz;
     above2 = h2 < -dz;
   }
@@ -220,133 +234,143 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
   }
   T be0 = quot<L64>(T(0.5) * G * (hp - T(0.5) * dev_fabs(dzp)) * dzp, c12, rc12);
 
-  // positivity limiter on subcritical wet-wet faces
-  hp = h1 + al0;
-  if (lam0 * lam2 < T(0) && hp > T(0) && h1 > T(0) && h2 > T(0)) {
-    // lam/(lam + lamE) is exactly 1 without an entropy-fix part (lam != 0 here)
-    const T f0 = lamE2 == T(0) ? T(1) : div_rare(lam0, lam0 + lamE2);
-    const T f2 = lamE0 == T(0) ? T(1) : div_rare(lam2, lam2 + lamE0);
-    const T lo = f0 * (al0 * lam0 - div_nz(h1 * dx * T(0.5), dt, K.rdt) + lamE2 * h2);
-    const T hi = f2 * (-al2 * lam2 + div_nz(h2 * dx * T(0.5), dt, K.rdt) + lamE0 * h1);
-    if constexpr (L64) {  // no NaN here: plain selections
-      be0 = lo > be0 ? lo : be0;
-      be0 = hi < be0 ? hi : be0;
-    } else {
-      be0 = dev_fmax(be0, lo);
-      be0 = dev_fmin(be0, hi);
-    }
-  }
-  const T be2 = -be0;
-
-  // waves 0, 1 and 2 with eigenvectors (1, r01, r02), (0, -c12 ny, c12 nx) and
+  // Waves 0, 1 and 2 with eigenvectors (1, r01, r02), (0, -c12 ny, c12 nx) and
   // (1, r21, r22) go to the neighbour's side (q) where their speed is
-  // positive, else to the owner's (p).  Subcritical faces away from a dry cell
-  // (nearly all of them) send one acoustic wave each way: assigned at once.
-  // The rest forms intermediate states, which decide whether mass is
-  // redirected from a dry side, and sorts wave by wave: by branches in FP64,
-  // by selections in FP32, where a selection is one instruction (the other
-  // way round each measured slower: rain on 1531x2049, FP64 flux launch 152
-  // us against 163; on 4096^2, FP32 445 against 452).
+  // positive, else to the owner's (p).  Plain faces - subcritical, no entropy
+  // fix, no dry cell - are nearly all: they send one acoustic wave each way and
+  // are done in one short block without the terms that are zero there (flux
+  // launch of rain on 1531x2049, FP64: 157 -> 148 us; on 4096^2, FP32: 448 ->
+  // 404 us).
   T p0, p1, p2, q0, q1, q2;
-  const T w0 = lam0 * al0 - be0, w1 = lam1 * al1, w2 = lam2 * al2 - be2;
-  const bool brink = h1 < E12 || h2 < E12;
-  if ((sizeof(T) == 4 || !brink) && !(lam0 > T(0)) && lam2 > T(0)) {
-    const T t = XFACE ? w1 * c12 : w1 * -c12;
-    p0 = w0;
-    q0 = w2;
-    p1 = w0 * r01;
-    p2 = w0 * r02;
-    q1 = w2 * r21;
-    q2 = w2 * r22;
+  hp = h1 + al0;
+  if (!brink && !fixed && lam0 < T(0) && lam2 > T(0)) {
+    {  // positivity limiter
+      const T lo = al0 * lam0 - c1.hd, hi = -al2 * lam2 + c2.hd;
+      const bool limit = hp > T(0);
+      if constexpr (L64) {  // no NaN here: plain selections
+        be0 = limit && lo > be0 ? lo : be0;
+        be0 = limit && hi < be0 ? hi : be0;
+      } else {
+        const T b = dev_fmin(dev_fmax(be0, lo), hi);
+        be0 = limit ? b : be0;
+      }
+    }
+    const T w1 = lam1 * al1, t = XFACE ? w1 * c12 : w1 * -c12;
+    p0 = lam0 * al0 - be0;
+    q0 = lam2 * al2 + be0;
+    p1 = p0 * r01;
+    p2 = p0 * r02;
+    q1 = q0 * r21;
+    q2 = q0 * r22;
     if (lam1 > T(0)) {
       if (XFACE) q2 = t + q2; else q1 = t + q1;
     } else {
       if (XFACE) p2 = p2 + t; else p1 = p1 + t;
     }
-  } else if (sizeof(T) == 4) {
-    const bool right0 = lam0 > T(0), right2 = lam2 > T(0);
-    const T x1 = w0 * r01, x2 = w0 * r02, y1 = w2 * r21, y2 = w2 * r22;
-    const T t = XFACE ? w1 * c12 : w1 * -c12;
-    p0 = (right0 ? T(0) : w0) + (right2 ? T(0) : w2);
-    q0 = (right0 ? w0 : T(0)) + (right2 ? w2 : T(0));
-    p1 = right0 ? T(0) : x1;
-    p2 = right0 ? T(0) : x2;
-    q1 = right0 ? x1 : T(0);
-    q2 = right0 ? x2 : T(0);
-    if (lam1 > T(0)) {
-      if (XFACE) q2 += t; else q1 += t;
-    } else {
-      if (XFACE) p2 += t; else p1 += t;
-    }
-    p1 += right2 ? T(0) : y1;
-    p2 += right2 ? T(0) : y2;
-    q1 += right2 ? y1 : T(0);
-    q2 += right2 ? y2 : T(0);
   } else {
-    p0 = p1 = p2 = q0 = q1 = q2 = T(0);
-    if (h2 < E12 && hp + div_rare(be2, lam2) < -E12) {
-      p0 += w0 + w2;
-    } else if (h1 < E12 && hp - div_rare(be0, lam0) < -E12) {
-      q0 += w0 + w2;
-    } else {
-      if (lam0 > T(0)) {
-        q0 += w0;
-        q1 += w0 * r01;
-        q2 += w0 * r02;
-      } else {
-        p0 += w0;
-        p1 += w0 * r01;
-        p2 += w0 * r02;
+    if (lam0 * lam2 < T(0) && hp > T(0) && h1 > T(0) && h2 > T(0)) {
+      T lo = al0 * lam0 - c1.hd, hi = -al2 * lam2 + c2.hd;
+      if (fixed) {
+        // lam/(lam + lamE) is exactly 1 without an entropy-fix part (lam != 0 here)
+        const T f0 = lamE2 == T(0) ? T(1) : div_rare(lam0, lam0 + lamE2);
+        const T f2 = lamE0 == T(0) ? T(1) : div_rare(lam2, lam2 + lamE0);
+        lo = f0 * (lo + lamE2 * h2);
+        hi = f2 * (hi + lamE0 * h1);
       }
+      be0 = dev_fmax(be0, lo);
+      be0 = dev_fmin(be0, hi);
+    }
+    const T be2 = -be0;
+    const T w0 = lam0 * al0 - be0, w1 = lam1 * al1, w2 = lam2 * al2 - be2;
+    // intermediate states decide whether mass is redirected from a dry side;
+    // they only matter next to a dry cell, so they are formed only there.  The
+    // rest is sorted wave by wave: by branches in FP64, by selections in FP32,
+    // where a selection is one instruction.
+    if (sizeof(T) == 4) {
+      const bool right0 = lam0 > T(0), right2 = lam2 > T(0);
+      const T x1 = w0 * r01, x2 = w0 * r02, y1 = w2 * r21, y2 = w2 * r22;
+      const T t = XFACE ? w1 * c12 : w1 * -c12;
+      p0 = (right0 ? T(0) : w0) + (right2 ? T(0) : w2);
+      q0 = (right0 ? w0 : T(0)) + (right2 ? w2 : T(0));
+      p1 = right0 ? T(0) : x1;
+      p2 = right0 ? T(0) : x2;
+      q1 = right0 ? x1 : T(0);
+      q2 = right0 ? x2 : T(0);
       if (lam1 > T(0)) {
-        if (XFACE) q2 += w1 * c12; else q1 += w1 * -c12;
+        if (XFACE) q2 += t; else q1 += t;
       } else {
-        if (XFACE) p2 += w1 * c12; else p1 += w1 * -c12;
+        if (XFACE) p2 += t; else p1 += t;
       }
-      if (lam2 > T(0)) {
-        q0 += w2;
-        q1 += w2 * r21;
-        q2 += w2 * r22;
+      p1 += right2 ? T(0) : y1;
+      p2 += right2 ? T(0) : y2;
+      q1 += right2 ? y1 : T(0);
+      q2 += right2 ? y2 : T(0);
+    if (brink) {
+      const bool dry2 = h2 < E12 && hp + div_rare(be2, lam2) < -E12;
+      const bool dry1 = !dry2 && h1 < E12 && hp - div_rare(be0, lam0) < -E12;
+      if (dry1 || dry2) {
+        const T m = w0 + w2;
+        p0 = dry2 ? m : T(0);
+        q0 = dry2 ? T(0) : m;
+        p1 = p2 = q1 = q2 = T(0);
+      }
+    }
+    } else {
+      p0 = p1 = p2 = q0 = q1 = q2 = T(0);
+      if (h2 < E12 && hp + div_rare(be2, lam2) < -E12) {
+        p0 += w0 + w2;
+      } else if (h1 < E12 && hp - div_rare(be0, lam0) < -E12) {
+        q0 += w0 + w2;
       } else {
-        p0 += w2;
-        p1 += w2 * r21;
-        p2 += w2 * r22;
+        if (lam0 > T(0)) {
+          q0 += w0;
+          q1 += w0 * r01;
+          q2 += w0 * r02;
+        } else {
+          p0 += w0;
+          p1 += w0 * r01;
+          p2 += w0 * r02;
+        }
+        if (lam1 > T(0)) {
+          if (XFACE) q2 += w1 * c12; else q1 += w1 * -c12;
+        } else {
+          if (XFACE) p2 += w1 * c12; else p1 += w1 * -c12;
+        }
+        if (lam2 > T(0)) {
+          q0 += w2;
+          q1 += w2 * r21;
+          q2 += w2 * r22;
+        } else {
+          p0 += w2;
+          p1 += w2 * r21;
+          p2 += w2 * r22;
+        }
       }
     }
-  }
-  if (sizeof(T) == 4 && brink) {
-    const bool dry2 = h2 < E12 && hp + div_rare(be2, lam2) < -E12;
-    const bool dry1 = !dry2 && h1 < E12 && hp - div_rare(be0, lam0) < -E12;
-    if (dry1 || dry2) {
-      const T m = w0 + w2;
-      p0 = dry2 ? m : T(0);
-      q0 = dry2 ? T(0) : m;
-      p1 = p2 = q1 = q2 = T(0);
+    // entropy-fix parts (a wave without a fix contributes zeros; lamE1 is zero)
+    if (lamE0 != T(0)) {
+      const T w = lamE0 * al0;
+      if (lamE0 > T(0)) {
+        q0 += w * T(1);
+        q1 += w * r01;
+        q2 += w * r02;
+      } else {
+        p0 += w * T(1);
+        p1 += w * r01;
+        p2 += w * r02;
+      }
     }
-  }
-  // entropy-fix parts (a wave without a fix contributes zeros; lamE1 is zero)
-  if (lamE0 != T(0)) {
-    const T w = lamE0 * al0;
-    if (lamE0 > T(0)) {
-      q0 += w * T(1);
-      q1 += w * r01;
-      q2 += w * r02;
-    } else {
-      p0 += w * T(1);
-      p1 += w * r01;
-      p2 += w * r02;
-    }
-  }
-  if (lamE2 != T(0)) {
-    const T w = lamE2 * al2;
-    if (lamE2 > T(0)) {
-      q0 += w * T(1);
-      q1 += w * r21;
-      q2 += w * r22;
-    } else {
-      p0 += w * T(1);
-      p1 += w * r21;
-      p2 += w * r22;
+    if (lamE2 != T(0)) {
+      const T w = lamE2 * al2;
+      if (lamE2 > T(0)) {
+        q0 += w * T(1);
+        q1 += w * r21;
+        q2 += w * r22;
+      } else {
+        p0 += w * T(1);
+        p1 += w * r21;
+        p2 += w * r22;
+      }
     }
   }
   // flush tiny contributions, then scale to depth/discharge increments
@@ -361,8 +385,8 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
     // contributions keep the absolute threshold only: zeroing those below
     // the noise of their terms deleted slow flows out of deep water every
     // step, and the FP32 run drained 2-5x further from FP64 in volume.)
-    const T s0 = dev_fabs(lam0 * al0) + dev_fabs(be0) + dev_fabs(lam2 * al2) + dev_fabs(lamE0 * al0) +
-                 dev_fabs(lamE2 * al2);
+    T s0 = dev_fabs(lam0 * al0) + dev_fabs(be0) + dev_fabs(lam2 * al2);
+    if (fixed) s0 = s0 + dev_fabs(lamE0 * al0) + dev_fabs(lamE2 * al2);
     th0 = dev_fmax(E12, T(kNoise32) * s0);
   }
   if (sizeof(T) == 4 && th0 > E12) {

@@ -115,24 +115,26 @@ template <bool XFACE>
 __device__ __noinline__ FaceOut<double> face_guarded(double h1, double qx1, double qy1, double z1, double s1, double h2,
                                                      double qx2, double qy2, double z2, double s2, double dx,
                                                      double dt, double hextra) {
-  CellQ<double> a = make_cell<double>(h1, qx1, qy1, z1, hextra);
-  CellQ<double> b = make_cell<double>(h2, qx2, qy2, z2, hextra);
+  const StepK<double> K = step_k<double>(dx, dt, 1.0 / dx, 1.0 / dt, hextra);
+  CellQ<double> a = make_cell<double>(h1, qx1, qy1, z1, K);
+  CellQ<double> b = make_cell<double>(h2, qx2, qy2, z2, K);
   a.sq = s1;  // the kernels read the SQRTH array, not sqrt(h)
   b.sq = s2;
-  return face_flux<double, XFACE>(a, b, step_k<double>(dx, dt, 1.0 / dx, 1.0 / dt, hextra));
+  return face_flux<double, XFACE>(a, b, K);
 }
 
 // Velocity of a regular cell (make_cell without its square root, which comes
 // from the SQRTH array here).
 __device__ __forceinline__ CellQ<double> cell_line(double h, double qx, double qy, double z, double sq,
-                                                   double hextra) {
+                                                   const StepK<double>& K) {
   CellQ<double> c;
   c.h = h;
   c.qx = qx;
   c.qy = qy;
   c.z = z;
   c.sq = sq;
-  const bool flows = h >= hextra;
+  c.hd = div_nz(h * K.dx * 0.5, K.dt, K.rdt);
+  const bool flows = h >= K.hextra;
   const double hs = flows ? h : 1.0;
   const double y = rsqrt_line(hs), rh = recip_line(hs, y * y);
   c.u = flows ? div_line(qx, hs, rh) : 0.0;
@@ -183,8 +185,8 @@ __global__ void __launch_bounds__(kThreads)
     // the sum of the square roots divides: it must be in range, too
     if (regular_cell(h1, qx1, qy1) && regular_cell(h2, qx2, qy2) && K.hextra >= 0x1p-100 && s1 >= 0.0 && s2 >= 0.0 &&
         s1 + s2 >= 0x1p-151 && s1 + s2 <= 0x1p51)
-      f = face_flux<double, XFACE, true>(cell_line(h1, qx1, qy1, z1, s1, K.hextra),
-                                         cell_line(h2, qx2, qy2, z2, s2, K.hextra), K);
+      f = face_flux<double, XFACE, true>(cell_line(h1, qx1, qy1, z1, s1, K),
+                                         cell_line(h2, qx2, qy2, z2, s2, K), K);
     else
       f = face_guarded<XFACE>(h1, qx1, qy1, z1, s1, h2, qx2, qy2, z2, s2, K.dx, K.dt, K.hextra);
   }
