@@ -209,7 +209,7 @@ int rebuild(tri_batch* b) { return b->prec == TRI_FP64 ? build_table<double>(b) 
 // The default shape for the present members (batched steps compute every tile).
 void choose_shape(tri_batch* b) {
   if (b->shape_set || b->members.empty()) return;
-  const FluxShape s = flux_shape(b->prec == TRI_FP64, 1.0, [&](int rb) {
+  const FluxShape s = flux_shape(b->prec == TRI_FP64, true, 1.0, [&](int rb) {
     int64_t n = 0;
     for (const tri_domain* d : b->members)
       n += (int64_t)((d->desc.cols - 2 + kStripCols - 1) / kStripCols) * ((d->desc.rows - 2 + rb - 1) / rb);

@@ -233,6 +233,7 @@ StepArgs step_args(tri_domain* d) {
   a.ntiles = (uint32_t)d->tz_tiles;
   a.tf = d->tf;
   a.open_boundaries = d->desc.open_boundaries;
+  a.maxh_neg = d->maxh_neg;
   a.skip_dry = d->nroff == 0;  // runoff reaches every cell
   return a;
 }
@@ -305,7 +306,7 @@ void size_flux_grid(tri_domain* d) {
 // every tile, one without about half of them.
 void choose_shape(tri_domain* d) {
   const int64_t rows = d->desc.rows - 2, strips = (d->desc.cols - 2 + kStripCols - 1) / kStripCols;
-  const FluxShape s = flux_shape(d->prec == TRI_FP64, d->nroff > 0 ? 1.0 : 0.5,
+  const FluxShape s = flux_shape(d->prec == TRI_FP64, false, d->nroff > 0 ? 1.0 : 0.5,
                                  [&](int rb) { return strips * ((rows + rb - 1) / rb); });
   d->flux_variant = s.variant;
   d->rb = s.rb;
@@ -531,7 +532,6 @@ int tri_domain_create(const tri_grid_desc* desc, void* stream, tri_domain** out)
   if (cudaMalloc((void**)&d->maxh_neg, sizeof(int32_t)) != cudaSuccess)
     return fail(set_error(TRI_E_CUDA, "flag allocation failed"));
   cudaMemsetAsync(d->maxh_neg, 0, sizeof(int32_t), d->stream);
-  d->mirror->maxh_neg = d->maxh_neg;
   d->vol_blocks = 296;
   if (cudaMalloc((void**)&d->vol_part, d->vol_blocks * sizeof(double)) != cudaSuccess ||
       cudaMalloc((void**)&d->vol_out, sizeof(double)) != cudaSuccess)

@@ -45,7 +45,8 @@ __device__ __forceinline__ StepNow begin_step(const DevClock* __restrict__ c) {
   double dt;
   if (!c->time_increment_fixed) {
     // compute_global_dt: dry fallback, then clamp to the next print time
-    dt = dt_of_key(c->dt_key[c->rd], c->cfl_a);
+    const unsigned long long key0 = c->dt_key[0], key1 = c->dt_key[1];  // both, not one behind rd
+    dt = dt_of_key(c->rd ? key1 : key0, c->cfl_a);
     if (dt >= kMaxValue - 1.0) dt = c->init_dt;
     const double tp = c->print_interval * (c->print_id + 1);
     if (t0 + dt > tp) dt = tp - t0;
@@ -640,6 +641,44 @@ __device__ __forceinline__ const P* launder_ptr(const P* p) {
   return q;
 }
 
+// A piece of work of one warp: rows r0..r1 of strip sx, tile 'tile' or part of it.
+struct FluxUnit {
+  unsigned tile;
+  int sx, r0, r1;
+};
+__device__ __forceinline__ FluxUnit whole_tile(unsigned tile, int rows, int nstrips, int rb) {
+  FluxUnit u;
+  u.tile = tile;
+  u.sx = (int)(tile % (unsigned)nstrips);
+  u.r0 = 1 + (int)(tile / (unsigned)nstrips) * rb;
+  u.r1 = min(u.r0 + rb - 1, rows - 2);
+  return u;
+}
+
+// The last tiles of a launch, as many as it has warps (`split`), are taken in
+// parts of 4 or (tiles above 8 rows) 8 rows, so that the warps end together: unit
+// n of tiles - split + split * parts.  Rain on 1531x2049, FP64: step 181 -> 175
+// us (8 rows, parts of 4); a 24-member FP32 ensemble 239 -> 232 us (16 rows,
+// parts of 8; 235 with parts of 4, which repeat more rows of faces).
+__device__ __forceinline__ int part_rows(int rb) { return rb > 8 ? 8 : 4; }
+__device__ __forceinline__ unsigned tile_parts(int rb) { return (unsigned)((rb + part_rows(rb) - 1) / part_rows(rb)); }
+// Tile of unit n; *part: which part of it (-1: all).
+__device__ __forceinline__ unsigned unit_tile(unsigned n, unsigned ntiles, unsigned split, int rb, int* part) {
+  const unsigned whole = ntiles - split, parts = tile_parts(rb);
+  if (n < whole) {
+    *part = -1;
+    return n;
+  }
+  const unsigned v = n - whole;
+  *part = (int)(v % parts);
+  return whole + v / parts;
+}
+__device__ __forceinline__ void take_part(FluxUnit* u, int part, int rb) {
+  if (part < 0) return;
+  u->r0 += part * part_rows(rb);
+  u->r1 = min(u->r1, u->r0 + part_rows(rb) - 1);
+}
+
 // One warp tile: strip sx (30 interior columns), rows r0..r1.  kTrack:
 // record in X.tz_dst whether the tile wrote only +0 (dry-tile skipping; the
 // kernels of domains that cannot skip are built without it).  kReload: the
@@ -657,15 +696,13 @@ __device__ __forceinline__ const P* launder_ptr(const P* p) {
 // the caller computes it again with the guarded forms (the tile only reads
 // the source buffer, so it can be repeated).
 template <typename T, bool kTrack, bool kReload, bool kLine>
-__device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, unsigned tile, int lane) {
+__device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, FluxUnit u, int lane) {
   bool odd = false;  // this lane met a cell that is not regular
   const FluxCtx<T>& X = kReload ? *launder_ptr(&X0) : X0;
-  const int rows = X.rows, cols = X.cols, rb = X.rb;
+  const int rows = X.rows, cols = X.cols;
   const T hextra = X.K.hextra;
-  const int sx = (int)(tile % X.nstrips), ry = (int)(tile / X.nstrips);
-  const int c = sx * kStripCols + lane;  // = c0 - 1 + lane with c0 = 1 + 30*sx
-  const int r0 = 1 + ry * rb;
-  const int r1 = min(r0 + rb - 1, rows - 2);
+  const int c = u.sx * kStripCols + lane;  // = c0 - 1 + lane with c0 = 1 + 30*sx
+  const int r0 = u.r0, r1 = u.r1;
   const bool incol = c < cols;
   const bool mid = (lane >= 1 && lane <= kStripCols);
   const bool upd = mid && c >= 1 && c <= cols - 2;
@@ -843,7 +880,7 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, unsigned ti
   }
   if (kTrack) {
     const bool nz = __any_sync(0xffffffffu, wrote_nonzero);
-    if (lane == 0) X.tz_dst[tile] = (!nz && !X.tpin[tile]) ? 1 : 0;
+    if (lane == 0) X.tz_dst[u.tile] = (!nz && !X.tpin[u.tile]) ? 1 : 0;
   }
   return true;
 }
@@ -852,23 +889,23 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, unsigned ti
 // single-domain kernel's context is formed again from the kernel parameters
 // (a context that the call took by reference would live in local memory).
 template <typename T>
-__device__ __noinline__ void flux_tile_guarded_ctx(const FluxCtx<T>* X, unsigned tile, int lane) {
-  flux_tile_form<T, false, true, false>(*X, tile, lane);
+__device__ __noinline__ void flux_tile_guarded_ctx(const FluxCtx<T>* X, FluxUnit u, int lane) {
+  flux_tile_form<T, false, true, false>(*X, u, lane);
 }
 template <typename T, bool kSkip>
 __device__ __noinline__ void flux_tile_guarded(DevClock* clk, const StepNow* now, const StateBufs<T>* sb,
                                                const BedMap<T>* bed, const T* n2, const int32_t* zone, const T* rates,
                                                int rows, int cols, int rb, T dx, T rdx, T hextra, uint8_t* tflag,
-                                               unsigned tile, int lane) {
+                                               FluxUnit u, int lane) {
   flux_tile_form<T, kSkip, false, false>(
-      flux_ctx_tiles<T, kSkip>(clk, *now, *sb, *bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra, tflag), tile,
+      flux_ctx_tiles<T, kSkip>(clk, *now, *sb, *bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra, tflag), u,
       lane);
 }
 
-// One tile of a batch member, its context in shared memory.
+// A unit of a batch member, its context in shared memory.
 template <typename T>
-__device__ __forceinline__ void flux_tile_member(const FluxCtx<T>& X, unsigned tile, int lane) {
-  if (!flux_tile_form<T, false, true, sizeof(T) == 8>(X, tile, lane)) flux_tile_guarded_ctx<T>(&X, tile, lane);
+__device__ __forceinline__ void flux_tile_member(const FluxCtx<T>& X, FluxUnit u, int lane) {
+  if (!flux_tile_form<T, false, true, sizeof(T) == 8>(X, u, lane)) flux_tile_guarded_ctx<T>(&X, u, lane);
 }
 
 // kSkip: the domain can have dry tiles (no runoff) and skips them.
@@ -890,23 +927,31 @@ __global__ void __launch_bounds__(128, MINB)
                                                 tflag);
   const int lane = threadIdx.x & 31;
   const unsigned ntiles = (unsigned)X.nstrips * (unsigned)((rows - 2 + rb - 1) / rb);
+  // a dry-tile flag has one writer: where dry tiles are skipped, tiles stay whole
+  const unsigned split = kSkip ? 0u : min(ntiles, gridDim.x * 4u);
+  const unsigned nunits = ntiles - split + split * tile_parts(rb);
   unsigned skipped = 0;  // interior cells of the tiles this warp skipped (lane 0)
   while (true) {
-    unsigned tile = 0;  // lane 0 takes the next tile; bit 31: skip it (tiles < 2^31)
+    unsigned n = 0;  // lane 0 takes the next unit; bit 31: skip it (tiles < 2^31)
     if (lane == 0) {
-      tile = atomicAdd(&clk->tile_next, 1u);
-      if (kSkip && tile < ntiles && tile_skippable<T>(X, tile)) {
-        const int sx = (int)(tile % X.nstrips), r0 = 1 + (int)(tile / X.nstrips) * rb;
-        skipped += (unsigned)((min(r0 + rb - 1, rows - 2) - r0 + 1) * min(kStripCols, cols - 2 - sx * kStripCols));
-        tile |= 0x80000000u;
+      n = atomicAdd(&clk->tile_next, 1u);
+      if (kSkip && n < ntiles && tile_skippable<T>(X, n)) {
+        const FluxUnit u = whole_tile(n, rows, X.nstrips, rb);
+        skipped += (unsigned)((u.r1 - u.r0 + 1) * min(kStripCols, cols - 2 - u.sx * kStripCols));
+        n |= 0x80000000u;
       }
     }
-    tile = __shfl_sync(0xffffffffu, tile, 0);
-    if ((tile & 0x7FFFFFFFu) >= ntiles) break;
-    if (kSkip && (tile >> 31)) continue;
-    if (!flux_tile_form<T, kSkip, false, sizeof(T) == 8>(X, tile, lane))
-      flux_tile_guarded<T, kSkip>(clk, &s_now, &sb, &bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra, tflag,
-                                  tile, lane);
+    n = __shfl_sync(0xffffffffu, n, 0);
+    if ((n & 0x7FFFFFFFu) >= nunits) break;
+    if (kSkip && (n >> 31)) continue;
+    int part = -1;
+    const unsigned tile = kSkip ? n : unit_tile(n, ntiles, split, rb, &part);
+    FluxUnit u = whole_tile(tile, rows, X.nstrips, rb);
+    take_part(&u, part, rb);
+    if (u.r0 > u.r1) continue;  // the grid's last tile row can be short
+    if (!flux_tile_form<T, kSkip, false, sizeof(T) == 8>(X, u, lane))
+      flux_tile_guarded<T, kSkip>(clk, &s_now, &sb, &bed, n2, zone, rates, rows, cols, rb, dx, rdx, hextra, tflag, u,
+                                  lane);
   }
   pdl_trigger();  // no tile left for this warp
   if (kSkip && lane == 0 && skipped)  // spread over the slots: one address would serialize the atomics
@@ -1380,15 +1425,16 @@ template <typename T>
 __global__ void __launch_bounds__(kWetCols, PostBlocks<T>::v)
     k_post(DevClock* __restrict__ clk, const __grid_constant__ StateBufs<T> sb, const __grid_constant__ BedMap<T> bed,
            T* __restrict__ maxh, int rows, int cols, T hextra, float* __restrict__ arrival, float arrival_depth,
-           const uint8_t* __restrict__ tflag, int rb, unsigned ntiles) {
+           const uint8_t* __restrict__ tflag, const int32_t* __restrict__ maxh_neg, int rb, unsigned ntiles) {
   pdl_wait();
   pdl_trigger();
+  const bool skips = tflag != nullptr && *maxh_neg == 0;
   if (!clk->now.active) return;
   const int lane = threadIdx.x & 31;
   const unsigned warps = gridDim.x * (kWetCols / 32);
   const PostArgs<T> P = post_args<T>(clk->now, sb, bed, maxh, arrival, arrival_depth, rows, cols, rb, hextra);
   const uint8_t* flags = nullptr;
-  if (tflag != nullptr && *clk->maxh_neg == 0) flags = tflag + (size_t)clk->now.dst * ntiles;
+  if (skips) flags = tflag + (size_t)clk->now.dst * ntiles;
   T dmax = T(-1);
   unsigned skipped = 0;  // interior cells of the tiles this lane found dry
   // the warp's tiles are t, t + warps, ...; 32 of them are looked at at once
@@ -1440,18 +1486,25 @@ __global__ void __launch_bounds__(128, MINB) k_batch_flux(const MemberDev<T>* __
   __shared__ FluxCtx<T> s_ctx[4];  // the member context of each warp's tile
   const int lane = threadIdx.x & 31;
   pdl_wait();
+  const int rb = mem[0].rb;
+  const unsigned split = min(ntiles, gridDim.x * 4u), nunits = ntiles - split + split * tile_parts(rb);
   while (true) {
-    unsigned tile = 0;
-    if (lane == 0) tile = atomicAdd(&ctl->tile_next, 1u);
-    tile = __shfl_sync(0xffffffffu, tile, 0);
-    if (tile >= ntiles) break;
+    unsigned n = 0;
+    if (lane == 0) n = atomicAdd(&ctl->tile_next, 1u);
+    n = __shfl_sync(0xffffffffu, n, 0);
+    if (n >= nunits) break;
+    int part;
+    const unsigned tile = unit_tile(n, ntiles, split, rb, &part);
     const MemberDev<T>& M = mem[tile_member[tile]];
     if (!M.clk->now.active) continue;
-    __syncwarp();  // the warp's previous tile no longer reads its context
+    FluxUnit u = whole_tile(tile - M.tile_begin, M.rows, (M.cols - 2 + kStripCols - 1) / kStripCols, rb);
+    take_part(&u, part, rb);
+    if (u.r0 > u.r1) continue;
+    __syncwarp();  // the warp's previous unit no longer reads its context
     FluxCtx<T>& X = s_ctx[threadIdx.x >> 5];
     if (lane == 0) X = member_ctx<T>(M);
     __syncwarp();
-    flux_tile_member<T>(X, tile - M.tile_begin, lane);
+    flux_tile_member<T>(X, u, lane);
   }
   pdl_trigger();
 }
@@ -1592,7 +1645,9 @@ __device__ __forceinline__ void steps_flux_item(const MemberDev<T>* __restrict__
     if (lane == 0)
       s_ctx[warp] = member_ctx<T>(M);
     __syncwarp();
-    flux_tile_member<T>(s_ctx[warp], tile - M.tile_begin, lane);
+    flux_tile_member<T>(s_ctx[warp],
+                        whole_tile(tile - M.tile_begin, M.rows, (M.cols - 2 + kStripCols - 1) / kStripCols, M.rb),
+                        lane);
   }
   __syncwarp();
   if (lane == 0) {

@@ -105,7 +105,7 @@ int launch_step(const StepArgs& a, cudaStream_t s, cudaEvent_t* ev) {
   const bool skip_dry = a.skip_dry && (a.arrival == nullptr || a.arrival_depth >= 0.0f);
   TRI_CUDA_TRY(launch_pdl(k_post<T>, post_blocks(a.ntiles, a.ntiles, PostBlocks<T>::v), kWetCols, 0, s, a.clk, sb, bed, (T*)a.maxh,
                           rows, cols, hx, a.arrival, a.arrival_depth, (const uint8_t*)(skip_dry ? a.tflag : nullptr),
-                          a.rb, a.ntiles));
+                          a.maxh_neg, a.rb, a.ntiles));
   if (ev) cudaEventRecord(ev[3], s);
   TRI_CUDA_TRY(cudaGetLastError());
   return TRI_OK;

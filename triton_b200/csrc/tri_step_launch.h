@@ -47,19 +47,20 @@ struct FluxBudget<float> {
 // faster: bowl 2048^2 97.4 us at 4 blocks per SM, 100.0 at 5, 112 at 6).  FP32
 // is bound by issue and takes 8 blocks per SM (rain 2048^2 129 us, 137 at 5),
 // but where one round holds all tiles the largest budget (bowl 256^2 12.6 us,
-// 14.0).
+// 14.0), and a batch, which reads its context from shared memory, 6 (24 members
+// 230 us a step, 240 at 8).
 struct FluxShape {
   int variant, rb;
 };
 template <typename F>
-FluxShape flux_shape(bool fp64, double share, F tiles) {
+FluxShape flux_shape(bool fp64, bool batch, double share, F tiles) {
   constexpr double slots = 148 * 16;
   for (int rb = 1; rb <= 4; rb++)
     if (share * (double)tiles(rb) <= slots) return {0, rb};
   int best = 4;
   for (int rb : {6, 8, 12, 16, 24, 32})
     if (share * (double)tiles(rb) >= 4 * slots) best = rb;
-  return {fp64 ? 0 : 2, best};
+  return {fp64 ? 0 : (batch ? 1 : 2), best};
 }
 // Blocks of 128 threads per SM that the post kernels are compiled for: a stream
 // with two rows of loads in flight per warp, so as many as its registers allow
@@ -115,6 +116,7 @@ struct StepArgs {
   TileForcing tf;
   int open_boundaries;
   bool skip_dry;
+  const int32_t* maxh_neg;  // device flag: a max depth that was uploaded is negative or NaN
 };
 
 // One time step (flux/update, forcing, post kernel).  ev: optional 4

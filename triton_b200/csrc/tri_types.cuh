@@ -53,7 +53,6 @@ struct DevClock {
   unsigned long long dt_key[2];
   const double* roff_t;
   const double* hyg_t;
-  const int32_t* maxh_neg;  // nonzero: a max depth that was uploaded is negative or NaN
   StepNow now;
   // FP64 volume accounting in depth units (multiply by dx^2), both forms.
   // acc_step collects the running step (atomics), the post kernel folds it
