@@ -520,10 +520,11 @@ int tri_domain_create(const tri_grid_desc* desc, void* stream, tri_domain** out)
   }
   if (cudaMalloc((void**)&d->clk, sizeof(DevClock)) != cudaSuccess ||
       cudaMallocHost((void**)&d->mirror, sizeof(DevClock)) != cudaSuccess ||
-      cudaMallocHost((void**)&d->halt_host, 2 * sizeof(int32_t)) != cudaSuccess)
+      cudaMallocHost((void**)&d->halt_host, sizeof(int32_t)) != cudaSuccess)
     return fail(set_error(TRI_E_CUDA, "clock allocation failed"));
   memset(d->mirror, 0, sizeof(DevClock));
   d->mirror->dt_key[0] = d->mirror->dt_key[1] = kDtKeyInf;
+  d->mirror->host_halt = d->halt_host;
   d->mirror->cfl_a = desc->courant * desc->cell_size;
   d->mirror->sim_duration = 0;
   d->mirror->print_interval = 1e300;
@@ -898,22 +899,20 @@ int tri_domain_advance(tri_domain* d, int32_t max_steps, tri_progress* p) {
     if (rc != TRI_OK) return rc;
   }
   // Chunks of steps, two in flight: after launching chunk k the host waits
-  // for chunk k-1 and stops launching once a step has raised an event.
+  // for chunk k-1 and stops launching once a step has raised an event.  The
+  // step that does sets a pinned host word itself: a copy of the flag behind
+  // every chunk kept the GPU idle between two graphs.
   const int chunk = 8;
+  volatile int32_t* halted = d->halt_host;
+  *halted = 0;
   int left = max_steps, k = 0;
-  bool halted = false;
-  while (left > 0 && !halted) {
+  while (left > 0 && !*halted) {
     const int n = std::min(chunk, left);
     rc = launch_steps(d, n);
     if (rc != TRI_OK) return rc;
-    TRI_CUDA_TRY(cudaMemcpyAsync(&d->halt_host[k & 1], &d->clk->halt, sizeof(int32_t), cudaMemcpyDeviceToHost,
-                                 d->stream));
     TRI_CUDA_TRY(cudaEventRecord(d->chunk_ev[k & 1], d->stream));
     left -= n;
-    if (k > 0) {
-      TRI_CUDA_TRY(cudaEventSynchronize(d->chunk_ev[(k - 1) & 1]));
-      if (d->halt_host[(k - 1) & 1]) halted = true;
-    }
+    if (k > 0) TRI_CUDA_TRY(cudaEventSynchronize(d->chunk_ev[(k - 1) & 1]));
     k++;
   }
   rc = pull_clock(d);

@@ -56,7 +56,7 @@ struct tri_domain {
   // clock
   DevClock* clk = nullptr;  // device
   DevClock* mirror = nullptr;  // pinned host mirror
-  int32_t* halt_host = nullptr;  // pinned, one per chunk slot
+  int32_t* halt_host = nullptr;  // pinned: the running advance raised an event (DevClock::host_halt)
   bool dt_valid = false;
   // volume reduction scratch
   double* vol_part = nullptr;

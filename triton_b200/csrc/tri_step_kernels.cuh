@@ -114,6 +114,7 @@ __device__ __forceinline__ bool end_step(DevClock* __restrict__ c) {
   if (n.events) {
     c->halt = 1;
     c->events = n.events;
+    *c->host_halt = 1;  // the host reads it behind an event recorded after this kernel
     return true;
   }
   return false;

@@ -53,6 +53,7 @@ struct DevClock {
   unsigned long long dt_key[2];
   const double* roff_t;
   const double* hyg_t;
+  int32_t* host_halt;  // pinned host word that tells a host waiting for a chunk that the domain has halted
   StepNow now;
   // FP64 volume accounting in depth units (multiply by dx^2), both forms.
   // acc_step collects the running step (atomics), the post kernel folds it
