@@ -231,6 +231,25 @@ __device__ __forceinline__ float sr_add(float a, float b, uint32_t r, float* exa
   return u * fabsf(t - s) < fabsf(err) ? t : s;
 }
 
+// Two products.  FP32: one instruction for both, each rounded (and flushed) as
+// the single product is, since the FP32 flux kernel is bound by issue: rain on
+// 4096^2 403.5 -> 378.4 us a launch, bowl 2048^2 65.2 -> 63.0.  Products only:
+// of a paired product and a paired sum the assembler makes fused
+// multiply-adds, which round otherwise.
+__device__ __forceinline__ void mul2(float a0, float a1, float b0, float b1, float* r0, float* r1) {
+  float x, y;
+  asm("{\n.reg .b64 a, b, r;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\n"
+      "mul.rn.ftz.f32x2 r, a, b;\nmov.b64 {%0, %1}, r;\n}"
+      : "=f"(x), "=f"(y)
+      : "f"(b0), "f"(b1), "f"(a0), "f"(a1));
+  *r0 = x;
+  *r1 = y;
+}
+__device__ __forceinline__ void mul2(double a0, double a1, double b0, double b1, double* r0, double* r1) {
+  *r0 = a0 * b0;
+  *r1 = a1 * b1;
+}
+
 // Reciprocal of a divisor shared by several quotients.  FP64: RN(1/b), as
 // div_shared requires.  FP32 form: the hardware's approximate reciprocal
 // (within 2 ulp), written as an intrinsic so it is the same instruction in

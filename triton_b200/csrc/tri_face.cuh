@@ -95,8 +95,10 @@ __device__ __forceinline__ CellQ<T> make_cell(T h, T qx, T qy, T z, const StepK<
   c.sq = dev_fmax(dev_sqrt(h), T(0));
   if constexpr (sizeof(T) == 4) {
     const T rh = recip(h);
-    c.u = h >= hextra ? div_shared(qx, h, rh) : T(0);
-    c.v = h >= hextra ? div_shared(qy, h, rh) : T(0);
+    T u, v;
+    mul2(rh, rh, qx, qy, &u, &v);
+    c.u = h >= hextra ? u : T(0);
+    c.v = h >= hextra ? v : T(0);
     return c;
   }
   if (h >= hextra) {
@@ -129,6 +131,17 @@ __device__ __forceinline__ double quot(double a, double b, double y) {
 template <bool LINE>
 __device__ __forceinline__ float quot(float a, float b, float y) {
   return div_shared(a, b, y);
+}
+
+// Two quotients by the same divisor.
+template <bool LINE>
+__device__ __forceinline__ void quot2(double a0, double a1, double b, double y, double* r0, double* r1) {
+  *r0 = quot<LINE>(a0, b, y);
+  *r1 = quot<LINE>(a1, b, y);
+}
+template <bool LINE>
+__device__ __forceinline__ void quot2(float a0, float a1, float, float y, float* r0, float* r1) {
+  mul2(y, y, a0, a1, r0, r1);
 }
 
 // cross, dzb (FP32 form): the cells lie in different bed tiles; base level of
@@ -167,8 +180,11 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
     rc12 = recip(c12);
     rssq = recip(ssq);
   }
-  const T u12 = quot<L64>(u1 * sqh1 + u2 * sqh2, ssq, rssq);
-  const T v12 = quot<L64>(v1 * sqh1 + v2 * sqh2, ssq, rssq);
+  T u12, v12;
+  T us1, vs1, us2, vs2;
+  mul2(sqh1, sqh1, u1, v1, &us1, &vs1);
+  mul2(sqh2, sqh2, u2, v2, &us2, &vs2);
+  quot2<L64>(us1 + us2, vs1 + vs2, ssq, rssq, &u12, &v12);
   const T un = n_dot<T, XFACE>(u12, v12);
   T lam0 = un - c12, lam1 = un, lam2 = un + c12;
   T lamE0 = T(0), lamE2 = T(0);  // lamE1 is always zero
@@ -177,7 +193,8 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
   // Harten-Hyman style entropy fix on the acoustic waves (rare: one branch)
   {
     const T un1 = n_dot<T, XFACE>(u1, v1), un2 = n_dot<T, XFACE>(u2, v2);
-    const T g1 = SG * sqh1, g2 = SG * sqh2;
+    T g1, g2;
+    mul2(SG, SG, sqh1, sqh2, &g1, &g2);
     const T a1 = un1 - g1, a2 = un2 - g2, b1 = un1 + g1, b2 = un2 + g2;
     const bool fix0 = a1 < T(0) && a2 > T(0), fix2 = b1 < T(0) && b2 > T(0);
     fixed = fix0 || fix2;
@@ -202,10 +219,12 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
 
   // wave strengths
   const T dqx = c2.qx - c1.qx, dqy = c2.qy - c1.qy;
-  const T aq = quot<L64>(n_dot<T, XFACE>(dqx, dqy) - un * dh, c12, rc12);
-  const T al0 = T(0.5) * (dh - aq);
-  const T al1 = quot<L64>(n_cross<T, XFACE>(dqx - u12 * dh, dqy - v12 * dh), c12, rc12);
-  const T al2 = T(0.5) * (dh + aq);
+  T udh, vdh, aq, al1;
+  mul2(dh, dh, u12, v12, &udh, &vdh);
+  const T dx1 = dqx - udh, dy1 = dqy - vdh;
+  quot2<L64>(n_dot<T, XFACE>(dx1, dy1), n_cross<T, XFACE>(dx1, dy1), c12, rc12, &aq, &al1);
+  T al0, al2;
+  mul2(T(0.5), T(0.5), dh - aq, dh + aq, &al0, &al2);
 
   // upwinded bed-step source, limited where the step is higher than the water
   T dz;
@@ -256,12 +275,12 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
       }
     }
     const T w1 = lam1 * al1, t = XFACE ? w1 * c12 : w1 * -c12;
-    p0 = lam0 * al0 - be0;
-    q0 = lam2 * al2 + be0;
-    p1 = p0 * r01;
-    p2 = p0 * r02;
-    q1 = q0 * r21;
-    q2 = q0 * r22;
+    T w0, w2;
+    mul2(lam0, lam2, al0, al2, &w0, &w2);
+    p0 = w0 - be0;
+    q0 = w2 + be0;
+    mul2(r01, r21, p0, q0, &p1, &q1);
+    mul2(r02, r22, p0, q0, &p2, &q2);
     if (lam1 > T(0)) {
       if (XFACE) q2 = t + q2; else q1 = t + q1;
     } else {
@@ -411,12 +430,12 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
   // rhs = dt*p/dx (kernels_flux.h:267-273); dt*p is +0 or at least dt*1e-12
   if (sizeof(T) == 4 || K.dx_pow2) {  // uniform over the launch; in FP32 a / dx is a * rdx for any dx
     const T s = K.rdx;
-    out.a0 = (dt * p0) * s;
-    out.a1 = (dt * p1) * s;
-    out.a2 = (dt * p2) * s;
-    out.b0 = (dt * q0) * s;
-    out.b1 = (dt * q1) * s;
-    out.b2 = (dt * q2) * s;
+    mul2(dt, dt, p0, q0, &p0, &q0);
+    mul2(dt, dt, p1, q1, &p1, &q1);
+    mul2(dt, dt, p2, q2, &p2, &q2);
+    mul2(s, s, p0, q0, &out.a0, &out.b0);
+    mul2(s, s, p1, q1, &out.a1, &out.b1);
+    mul2(s, s, p2, q2, &out.a2, &out.b2);
   } else {
     out.a0 = div_nz(dt * p0, dx, K.rdx);
     out.a1 = div_nz(dt * p1, dx, K.rdx);

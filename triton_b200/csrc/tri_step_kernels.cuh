@@ -476,7 +476,9 @@ __device__ __forceinline__ void update_cell(const CellQ<T>& c, const RowParts<T>
     const T ry1 = p.w2 + s2;
     const T mx = c.qx - p.r1 - rx1;
     const T my = c.qy - p.r2 - ry1;
-    const T mm = mx * mx + my * my;
+    T mxx, myy;
+    mul2(mx, my, mx, my, &mxx, &myy);
+    const T mm = mxx + myy;
     T modM;
     if constexpr (L64) {  // a square below 1e-30 is no flow either way
       odd |= ((uint32_t)__double2hiint(mm) & 0x7FFFFFFFu) > (1023u + 600u) << 20;
@@ -514,8 +516,9 @@ __device__ __forceinline__ void update_cell(const CellQ<T>& c, const RowParts<T>
         // 1e-3 of itself each step, one way (the 512^2 6 h watershed then
         // ponded up to 0.97 m away from the FP64 run).
         const T k = recip(T(1) + sq);
-        qxij = T(2) * mx * k;
-        qyij = T(2) * my * k;
+        T mx2, my2;
+        mul2(T(2), T(2), mx, my, &mx2, &my2);
+        mul2(k, k, mx2, my2, &qxij, &qyij);
       }
     } else {
       qxij = mx;
@@ -988,7 +991,7 @@ __device__ __forceinline__ float wave_speed(float h, float qx, float qy) {
 }
 
 // ---------------------------------------------------------------------------
-// Staged wet-dry/dt: one block per band of WetStage<T>::kBand rows x
+// Staged wet-dry/dt, the wet-dry item of the single-launch batch mode: one block per band of WetStage<T>::kBand rows x
 // kWetCols columns.  The block stages, in shared memory, its rows of h and
 // the bed with a halo row above and below, and its rows of qx, qy and the
 // maximum depth, each row from column c0-1 to c0+kWetCols (clipped to the
@@ -1464,8 +1467,8 @@ __global__ void __launch_bounds__(kWetCols, PostBlocks<T>::v)
 // Batched ensembles: one launch per kernel type advances every member of a
 // batch by one of its own steps (each member keeps its own clock and dt).
 // Members are described in device memory (MemberDev); the flux kernel's warps
-// take tiles from one queue over all members' tiles, the wet-dry kernel's
-// blocks are a concatenation of every member's bands.
+// take tiles from one queue over all members' tiles, the post kernel's
+// blocks are a concatenation of every member's blocks.
 // ===========================================================================
 // The first step's clocks of an advance; later ones are run by the post kernel.
 template <typename T>
