@@ -328,7 +328,7 @@ def _domain_window(sc, prec, stream, spinup, steps, warmup):
     """One domain of `sc` in `prec`, launch shape autotuned: `spinup` +
     `warmup` untimed steps, `steps` timed with CUDA events at the two ends,
     then the same number again with an event pair around every flux and
-    wet-dry launch for the per-kernel figures."""
+    post launch for the per-kernel figures."""
     d = sc.to_domain(prec, stream=stream.cuda_stream)
     try:
         d.set_clock(sim_duration=1e300, print_interval=1e300, print_observation=1e300, it_print=0, time_series=0)
@@ -594,7 +594,7 @@ def main():
     assert n == args.steps, (n, ev)
     ms = e0.elapsed_time(e1)
     # per-launch durations for the roofline: the same number of steps again
-    # with a CUDA event pair around every flux and wet-dry launch.  An event
+    # with a CUDA event pair around every flux and post launch.  An event
     # between two kernels costs a few microseconds of step time, so the
     # timed region above carries events only at its two ends.
     d.set_timing(True)

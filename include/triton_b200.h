@@ -182,19 +182,19 @@ int tri_domain_mass_balance(tri_domain* d, double* out6);
 int tri_domain_track_arrival(tri_domain* d, double depth);
 int tri_domain_download_arrival(tri_domain* d, double* host, int64_t n);
 /* Kernel timing with CUDA events on the domain's stream: when enabled,
- * advance() records the flux/update kernel and the wet-dry/dt kernel.
+ * advance() records the flux/update kernel and the post kernel (wet/dry, dt).
  * Reports total milliseconds and launch counts since the last reset. */
 int tri_domain_set_timing(tri_domain* d, int32_t enabled);
 int tri_domain_get_timing(tri_domain* d, double* flux_ms, int32_t* flux_launches, double* wetdry_ms,
                           int32_t* wetdry_launches);
-/* Interior cells of the flux tiles and wet-dry bands that advance() calls
- * computed since the last tri_domain_set_timing (steps run x interior cells,
+/* Interior cells of the flux tiles that advance() calls
+ * computed, in the flux kernel and in the post kernel, since the last tri_domain_set_timing (steps run x interior cells,
  * less the cells of tiles skipped as dry: tiles whose cells and neighbours
  * hold only zeros, whose update is exactly the identity).  No reference
  * counterpart (the reference updates every cell every step). */
 int tri_domain_get_work(tri_domain* d, int64_t* flux_cells, int64_t* wetdry_cells);
 /* Test hook for the bounded device waits (no reference counterpart; the
- * reference's kernels never wait).  While polls > 0, every step's wet-dry
+ * reference's kernels never wait).  While polls > 0, every step's post
  * launch also waits, at most 'polls' polls, on a barrier that nothing
  * completes; the wait gives up, the launch records a device status, and
  * tri_domain_advance returns TRI_E_TIMEOUT once the steps have run (the
@@ -214,7 +214,7 @@ typedef struct tri_tuning {
 } tri_tuning;
 int tri_domain_autotune(tri_domain* d, int32_t trial_steps, tri_tuning* out);
 int tri_domain_get_tuning(tri_domain* d, tri_tuning* out);
-/* Sets the flux kernel's launch shape directly (variant 0..2, rows per tile >= 1). */
+/* Sets the flux kernel's launch shape directly (variant 0..4, rows per tile >= 1). */
 int tri_domain_set_tuning(tri_domain* d, int32_t variant, int32_t rows_per_tile);
 
 /* Self-check of the exact divisions by a reused divisor used in the kernels:
@@ -264,7 +264,7 @@ int tri_batch_wait(tri_batch* b, tri_batch_progress* out);
 int tri_batch_autotune(tri_batch* b, int32_t trial_steps, tri_tuning* out);
 /* How batched steps are launched (no reference counterpart).
  * TRI_BATCH_GRAPHS (default): per batched step one launch per kernel type
- * (clock, flux, forcing waves, wet-dry/dt), 8 steps captured as a CUDA graph.
+ * (flux, forcing, post), 8 steps captured as a CUDA graph.
  * TRI_BATCH_SINGLE_LAUNCH: one persistent launch runs up to 32 batched
  * steps; its blocks take work items (a member's clock, four flux tiles, a
  * member's forcing, a wet-dry block) in a fixed order and each item waits,

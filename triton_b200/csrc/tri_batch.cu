@@ -3,12 +3,12 @@
 // The reference runs ensemble members as separate MPI rank groups (Ensify,
 // src/Ensify.h:43-72), one process group per member.  Here every member is a
 // tri_domain on one GPU and a batched step advances each member by one of its
-// own time steps with one launch per kernel type: a clock kernel over the
-// member table (per-member dt policy and events), one flux kernel whose warps
+// own time steps with one launch per kernel type: one flux kernel whose warps
 // take tiles from a single queue over all members' tiles (uneven sizes pack
-// without idle SMs), the sparse forcing in conflict-free waves of (member,
-// item) pairs, and one wet-dry/dt kernel over all members' bands, each member
-// folding its own dt minimum.  Steps are launched as CUDA graphs of 8 batched
+// without idle SMs), one forcing kernel with a warp per tile that has any, and
+// one post kernel (wet/dry, max depth, dt) over all members' tiles, whose last
+// block of a member folds its accounts and runs its clock (dt policy, events)
+// for the next step.  Steps are launched as CUDA graphs of 8 batched
 // steps; the host checks after each graph how many members have halted.  In
 // single-launch mode (tri_batch_set_mode) one persistent launch of
 // k_batch_steps runs a chunk of 32 batched steps instead: its blocks take the
@@ -33,7 +33,7 @@ struct tri_batch {
   std::vector<tri_domain*> members;
   void* d_mem = nullptr;
   int32_t* d_tile_mem = nullptr;  // member of every flux tile
-  int32_t* d_wet_mem = nullptr;   // member of every wet-dry block
+  int32_t* d_wet_mem = nullptr;   // single-launch mode: member of every wet-dry block
   BatchCtl* d_ctl = nullptr;
   BatchCtl* h_ctl = nullptr;  // pinned
   int32_t* h_seen = nullptr;  // pinned, one per chunk slot

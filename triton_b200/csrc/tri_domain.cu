@@ -617,7 +617,7 @@ int tri_domain_upload(tri_domain* d, int32_t field, const double* host, int64_t 
     k_from_f64<float><<<(unsigned)((n + 255) / 256), 256, 0, d->stream>>>(d->stage, (float*)p, n);
     TRI_CUDA_TRY(cudaGetLastError());
   }
-  if (field == TRI_FIELD_MAXH) {  // dry bands skip the wet-dry kernel only while no max depth is negative
+  if (field == TRI_FIELD_MAXH) {  // dry tiles skip the post kernel only while no max depth is negative
     TRI_CUDA_TRY(cudaMemsetAsync(d->maxh_neg, 0, sizeof(int32_t), d->stream));
     if (d->prec == TRI_FP64)
       k_flag_negative<double><<<(unsigned)((n + 255) / 256), 256, 0, d->stream>>>((const double*)p, n, d->maxh_neg);
@@ -644,7 +644,7 @@ int tri_domain_init_max_depth(tri_domain* d) {
   const int64_t n = d->ncells;
   void* h = d->h[d->mirror->cur];
   TRI_CUDA_TRY(cudaMemcpyAsync(d->maxh, h, (size_t)n * es, cudaMemcpyDeviceToDevice, d->stream));
-  // dry bands skip the wet-dry kernel only while no max depth is negative
+  // dry tiles skip the post kernel only while no max depth is negative
   TRI_CUDA_TRY(cudaMemsetAsync(d->maxh_neg, 0, sizeof(int32_t), d->stream));
   if (d->prec == TRI_FP64)
     k_flag_negative<double><<<(unsigned)((n + 255) / 256), 256, 0, d->stream>>>((const double*)d->maxh, n,

@@ -66,10 +66,10 @@ struct tri_domain {
   int rb = 16, flux_blocks = 1, flux_variant = 1;
   bool shape_set = false;  // tuned or set by the caller: the defaults no longer apply
   // tile flags of the flux kernel for the current tile shape: [2][tiles] (by
-  // state buffer) then [tiles] pinned, and the lists of the tiles' forcing.  Any change of state, forcing or shape outside the
-  // step kernels marks the flags dirty; they are reset (nothing known) before
-  // the next steps.  A change of forcing or shape (tile_lists_dirty) also
-  // rebuilds the pins and lists.
+  // state buffer) then [tiles] pinned, and the lists of the tiles' forcing.
+  // Any change of state, forcing or shape outside the step kernels marks the
+  // flags dirty; they are reset (nothing known) before the next steps.  A change
+  // of forcing or shape (tile_lists_dirty) also rebuilds the pins and lists.
   uint8_t* tflag = nullptr;
   int32_t* tlists = nullptr;
   tri::TileForcing tf{};
@@ -82,7 +82,7 @@ struct tri_domain {
   cudaGraphExec_t graph = nullptr;
   int graph_steps = 0;
   bool use_graphs = true;
-  // timing: CUDA event pairs around every flux and wet-dry launch, read once
+  // timing: CUDA event pairs around every flux and post launch, read once
   // the timed region is over so the stream is never stalled
   bool timing = false;
   std::vector<cudaEvent_t> tev;

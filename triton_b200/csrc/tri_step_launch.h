@@ -2,7 +2,7 @@
 // step needs (device pointers and sizes) and the launch functions.  The
 // kernels are instantiated in two translation units: tri_step_f64.cu (IEEE,
 // no contraction: bit-exact with the reference) and tri_step_f32.cu (FP32
-// precision form, contraction and fast division/sqrt allowed).
+// precision form, approximate division and square root).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -14,12 +14,12 @@ namespace tri {
 
 constexpr int kStripCols = 30;   // interior columns per warp tile of the flux kernel
 constexpr int kFluxVariants = 5; // register budgets (FluxBudget)
-constexpr int kWetCols = 128;    // columns per block of the wet-dry/dt kernel
+constexpr int kWetCols = 128;    // columns per block of the staged wet-dry/dt pass (single-launch batches)
 // Blocks of 128 threads per SM that the flux kernel's register-budget
-// variants are compiled for (__launch_bounds__ minimum).  FP64: 122, 96, 80,
-// 72 and 64 registers a thread (from 96 down they spill to L1, 8 to 300
-// bytes); FP32: 88, 80, 64, 48 and 40.  The kernel is latency bound, so
-// occupancy can pay for some spilling; the autotuner picks per domain.
+// variants are compiled for (__launch_bounds__ minimum), at most 128, 96, 80,
+// 72 and 64 registers a thread in FP64 (from 96 down they spill to L1), 96, 80,
+// 64, 48 and 40 in FP32.  flux_shape's comment has the default and what the
+// others measured; the autotuner times all on a domain's own state.
 template <typename T>
 struct FluxBudget;
 template <>
@@ -43,7 +43,7 @@ struct FluxBudget<float> {
 //    repeats one row of faces above it (rain on 2048^2, FP64: 199 us with 12
 //    rows, 214 with 4; FP32 4096^2: 442 with 32, 468 with 6) and the last
 //    round of tiles idles half the warps.
-// FP64 takes the largest register budget (no spills; more warps are not
+// FP64 takes the largest register budget (few spills; more warps are not
 // faster: bowl 2048^2 97.4 us at 4 blocks per SM, 100.0 at 5, 112 at 6).  FP32
 // is bound by issue and takes 8 blocks per SM (rain 2048^2 129 us, 137 at 5),
 // but where one round holds all tiles the largest budget (bowl 256^2 12.6 us,

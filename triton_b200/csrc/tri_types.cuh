@@ -61,8 +61,8 @@ struct DevClock {
   double acc_step[kAccTerms];
   double acc_sum[kAccTerms];
   double acc_comp[kAccTerms];
-  // interior cells of the flux tiles [0] and wet-dry bands [1] that dry-tile
-  // skipping left out, summed over slots (one address would serialize the
+  // interior cells of the tiles that dry-tile skipping left out in the flux
+  // kernel [0] and in the post kernel [1], summed over slots (one address would serialize the
   // atomics of a launch)
   unsigned long long skipped[2][kSkipSlots];
 };

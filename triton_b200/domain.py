@@ -176,7 +176,7 @@ class Domain:
         return a.value, na.value, b.value, nb.value
 
     def get_work(self):
-        """(flux cells, wet-dry cells) computed since set_timing: interior
+        """(flux cells, post-kernel cells) computed since set_timing: interior
         cells of the tiles that were not skipped as dry."""
         a, b = C.c_int64(), C.c_int64()
         check(lib().tri_domain_get_work(self._h, C.byref(a), C.byref(b)))
