@@ -172,9 +172,11 @@ int build_table(tri_batch* b) {
   // post kernel blocks and forcing of all members' tiles
   std::vector<int32_t> pm;
   TileLists lists;
+  const auto tiles_of = [&](size_t m) { return tab[m].tile_end - tab[m].tile_begin; };
+  const uint32_t per = post_tiles_per_warp(tab.size(), PostBlocks<T>::batch, tiles_of);
   for (size_t m = 0; m < tab.size(); m++) {
     tab[m].post_begin = (uint32_t)pm.size();
-    tab[m].post_count = post_blocks(tab[m].tile_end - tab[m].tile_begin, tiles, PostBlocks<T>::batch);
+    tab[m].post_count = post_blocks(tiles_of(m), per);
     pm.insert(pm.end(), tab[m].post_count, (int32_t)m);
     append_tile_lists(b->members[m], b->rb, (int32_t)tab[m].tile_begin, lists);
   }

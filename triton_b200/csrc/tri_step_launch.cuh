@@ -103,7 +103,8 @@ int launch_step(const StepArgs& a, cudaStream_t s, cudaEvent_t* ev) {
   if (ev) cudaEventRecord(ev[2], s);
   // with arrival tracking of a negative depth dry cells count, too
   const bool skip_dry = a.skip_dry && (a.arrival == nullptr || a.arrival_depth >= 0.0f);
-  TRI_CUDA_TRY(launch_pdl(k_post<T>, post_blocks(a.ntiles, a.ntiles, PostBlocks<T>::v), kWetCols, 0, s, a.clk, sb, bed, (T*)a.maxh,
+  const uint32_t per = post_tiles_per_warp(1, PostBlocks<T>::v, [&](size_t) { return a.ntiles; });
+  TRI_CUDA_TRY(launch_pdl(k_post<T>, post_blocks(a.ntiles, per), kWetCols, 0, s, a.clk, sb, bed, (T*)a.maxh,
                           rows, cols, hx, a.arrival, a.arrival_depth, (const uint8_t*)(skip_dry ? a.tflag : nullptr),
                           a.maxh_neg, a.rb, a.ntiles));
   if (ev) cudaEventRecord(ev[3], s);
