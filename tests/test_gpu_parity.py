@@ -170,3 +170,37 @@ def test_tile_heights_agree_with_boundary_cells(precision):
     for other in got[1:]:
         for a, b in zip(got[0], other):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("rb", [1 << 30, (1 << 31) - 1])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_any_tile_height_computes_every_tile(precision, rb):
+    """Heights far above the grid's: a tile is taken in as many parts as its
+    rows need (2^27 parts of 8 rows in each of 32 strips are 2^32, no part at
+    all in 32 bits), alone and in a batch; the height set is the one reported."""
+    from triton_b200 import _abi, scenarios
+    from triton_b200.batch import Batch
+    import ctypes as C
+    got = []
+    for mode in ("default", "domain", "batch"):
+        sc = scenarios.mixed(rows=20, cols=960, seed=47, duration=5.0)
+        d = sc.to_domain(precision)
+        try:
+            d.set_clock(sim_duration=1e300, print_interval=1e300, time_series=0, it_print=0)
+            if mode == "batch":
+                with Batch([d]) as b:
+                    b.set_shape(0, rb)
+                    assert b.advance(9).steps == 9
+            else:
+                if mode == "domain":
+                    d.set_shape(0, rb)
+                    t = _abi.Tuning()
+                    _abi.check(_abi.lib().tri_domain_get_tuning(d._h, C.byref(t)))
+                    assert t.rows_per_tile == rb
+                assert d.advance(9)[0] == 9
+            got.append([d.download(f) for f in ("h", "qx", "qy", "maxh")] + [np.array(d.get_clock().simtime)])
+        finally:
+            d.close()
+    for other in got[1:]:
+        for a, b in zip(got[0], other):
+            assert np.array_equal(a, b)

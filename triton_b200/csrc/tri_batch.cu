@@ -144,7 +144,11 @@ template <typename T>
 int build_table(tri_batch* b) {
   std::vector<MemberDev<T>> tab;
   uint32_t tiles = 0, wet = 0;
-  for (tri_domain* d : b->members) tab.push_back(member_dev<T>(d, b->rb, tiles, wet));
+  // a tile ends with its grid: no height above the tallest member's interior
+  int rb = 1;
+  for (const tri_domain* d : b->members) rb = std::max(rb, d->desc.rows - 2);
+  rb = std::min(rb, b->rb);
+  for (tri_domain* d : b->members) tab.push_back(member_dev<T>(d, rb, tiles, wet));
   b->ntiles = tiles;
   b->nwet = wet;
   free_tables(b);
@@ -178,7 +182,7 @@ int build_table(tri_batch* b) {
     tab[m].post_begin = (uint32_t)pm.size();
     tab[m].post_count = post_blocks(tiles_of(m), per);
     pm.insert(pm.end(), tab[m].post_count, (int32_t)m);
-    append_tile_lists(b->members[m], b->rb, (int32_t)tab[m].tile_begin, lists);
+    append_tile_lists(b->members[m], rb, (int32_t)tab[m].tile_begin, lists);
   }
   b->npost = (uint32_t)pm.size();
   int rc = upload(pm, &b->d_post_mem);

@@ -194,6 +194,11 @@ __global__ void k_flag_negative(const T* __restrict__ v, int64_t n, int32_t* __r
   if (__syncthreads_or(neg) && threadIdx.x == 0) atomicExch(flag, 1);
 }
 
+// Tile height in use: a tile ends with the grid, so a taller one than the
+// interior (set_tuning takes any) is the interior's.  It also bounds what the
+// kernels count in 32 bits, the parts of a tile above all.
+int tile_rows(const tri_domain* d) { return std::min(d->rb, d->desc.rows - 2); }
+
 StepArgs step_args(tri_domain* d) {
   StepArgs a{};
   a.clk = d->clk;
@@ -211,7 +216,7 @@ StepArgs step_args(tri_domain* d) {
   a.rates = d->rates;
   a.rows = d->desc.rows;
   a.cols = d->desc.cols;
-  a.rb = d->rb;
+  a.rb = tile_rows(d);
   a.flux_blocks = d->flux_blocks;
   a.flux_variant = d->flux_variant;
   a.dx = d->desc.cell_size;
@@ -247,9 +252,9 @@ int64_t flux_tiles(const tri_domain* d, int rb) {
 // hold a source or an external boundary cell, or lie on an open edge.  They
 // are never skipped nor flagged.  Called outside graph capture, before steps.
 int build_tile_lists(tri_domain* d) {
-  const int64_t nt = flux_tiles(d, d->rb);
+  const int64_t nt = flux_tiles(d, tile_rows(d));
   TileLists lists;
-  append_tile_lists(d, d->rb, 0, lists);
+  append_tile_lists(d, tile_rows(d), 0, lists);
   std::vector<uint8_t> pin((size_t)nt, 0);
   for (int32_t t : lists.tiles) pin[(size_t)t] = 1;
   drop_graph(d);  // the graphs hold the old pointers and lists
@@ -288,7 +293,7 @@ int reset_tiles(tri_domain* d) {
 // Grid of the flux kernel for the domain's variant and tile height: one
 // resident wave of blocks, each warp fetching tiles until none are left.
 void size_flux_grid(tri_domain* d) {
-  const int rows = d->desc.rows - 2, cols = d->desc.cols - 2;
+  const int rows = d->desc.rows - 2, cols = d->desc.cols - 2, rb = tile_rows(d);
   int sms = 148, dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   int per_sm = 0;
@@ -298,7 +303,7 @@ void size_flux_grid(tri_domain* d) {
     flux_occupancy<float>(d->flux_variant, &per_sm);
   if (per_sm < 1) per_sm = 1;
   const int64_t strips = (cols + kStripCols - 1) / kStripCols;
-  const int64_t tiles = strips * ((rows + d->rb - 1) / d->rb);
+  const int64_t tiles = strips * ((rows + rb - 1) / rb);
   d->flux_blocks = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)sms * per_sm, (tiles + 3) / 4));
 }
 
