@@ -207,3 +207,38 @@ def test_flow_of_sources_in_shared_cells_matches_oracle(oracle, n):
     _abi.check(L.tri_kernel_compute_flow_f64(n, _p(dht), _p(dhv), 3.0, 0.07, 3.0, 0, 1, _p(dh), _p(dpos), None))
     torch.cuda.synchronize()
     assert np.array_equal(dh.cpu().numpy(), h)
+
+
+def _flux_both(oracle, R, Cc, h, qx, qy, z, sq, hx, dx=3.0, dt=0.05):
+    """flux_x then flux_y by the oracle and by the entries: two lists of six arrays."""
+    import torch
+    from triton_b200 import _abi
+    L, O = _abi.lib(), oracle.lib()
+    O.tor_flux_x.restype = O.tor_flux_y.restype = None
+    want = [np.random.default_rng(k).standard_normal(R * Cc) for k in range(6)]
+    got = [_dev(torch, a.copy()) for a in want]
+    ins = [np.ascontiguousarray(a.reshape(-1)) for a in (h, qx, qy, z, sq)]
+    dev = [_dev(torch, a) for a in ins]
+    for name in ("x", "y"):
+        getattr(O, "tor_flux_" + name)(R, Cc, C.c_double(dx), C.c_double(dt), *[a.ctypes.data_as(_dp) for a in ins],
+                                       *[a.ctypes.data_as(_dp) for a in want], C.c_double(hx))
+        _abi.check(getattr(L, f"tri_kernel_flux_{name}_f64")(R * Cc, R, Cc, dx, dt, *[_p(t) for t in dev],
+                                                             *[_p(t) for t in got], hx, None))
+    torch.cuda.synchronize()
+    return want, [t.cpu().numpy() for t in got]
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+def test_flux_over_nonfinite_beds_matches_oracle(oracle, value):
+    """Deep water over beds that are no number: the limiter's fmax and fmin
+    replace the source term, so the contributions are finite."""
+    rng = np.random.default_rng(2)
+    R, Cc = 17, 40
+    h = 2.0 + 0.2 * rng.random((R, Cc))
+    z = 0.1 * rng.random((R, Cc))
+    for r, c in ((0, 3), (5, 5), (5, 6), (6, 5), (16, 39)):
+        z[r, c] = value
+    zero = np.zeros((R, Cc))
+    want, got = _flux_both(oracle, R, Cc, h, zero, zero, z, np.sqrt(h), 1e-3)
+    for a, b in zip(want, got):
+        assert np.isfinite(a).all() and np.array_equal(a, b)

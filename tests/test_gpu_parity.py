@@ -204,3 +204,27 @@ def test_any_tile_height_computes_every_tile(precision, rb):
     for other in got[1:]:
         for a, b in zip(got[0], other):
             assert np.array_equal(a, b)
+
+
+def test_bed_without_a_level_under_water_matches_oracle():
+    """Bed cells without a level (NaN) under water: the limiter replaces the
+    source term that is not a number, as the oracle's fmax does, so the first
+    step stays finite and equal in every bit."""
+    from tests._harness import compare_fields, oracle_from_scenario
+    from triton_b200 import scenarios
+    sc = scenarios.mixed(rows=40, cols=61, seed=5, friction=False, with_extbc=False, with_sources=False,
+                         with_runoff=False, duration=1e3)
+    rng = np.random.default_rng(5)
+    sc.h[1:-1, 1:-1] = 2.0 + 0.2 * rng.random((40, 61))
+    sc.qx[:], sc.qy[:] = 0.0, 0.0
+    sc.z[1:-1, 1:-1] = 0.1 * rng.random((40, 61))
+    for r, c in ((3, 3), (9, 31), (9, 32), (10, 30), (20, 30), (33, 7)):
+        sc.z[r, c] = np.nan
+    o, d = oracle_from_scenario(sc), sc.to_domain()
+    try:
+        assert o.advance(1) == d.advance(1) == (1, 0)
+        assert np.isfinite(o.grid("h")).all() and np.isfinite(o.grid("qx")).all()
+        compare_fields(o, d, True, sc.hextra)
+        assert d.get_clock().simtime == o.s.simtime
+    finally:
+        d.close()

@@ -266,7 +266,7 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
     {  // positivity limiter
       const T lo = al0 * lam0 - c1.hd, hi = -al2 * lam2 + c2.hd;
       const bool limit = hp > T(0);
-      if constexpr (L64) {  // no NaN here: plain selections
+      if constexpr (L64) {  // be0 is NaN only over beds that are no numbers, which the callers catch
         be0 = limit && lo > be0 ? lo : be0;
         be0 = limit && hi < be0 ? hi : be0;
       } else {

@@ -142,6 +142,14 @@ __device__ __forceinline__ CellQ<double> cell_line(double h, double qx, double q
   return c;
 }
 
+// A bed level that is a number.  The step between two others can be NaN, and so
+// the source term, which the straight-line limiter's selections would keep where
+// fmax and fmin replace it.  (The step kernel's tile finds it out by itself: the
+// cell's momentum is NaN then, which makes the tile odd.)
+__device__ __forceinline__ bool finite_bed(double z) {
+  return ((uint32_t)__double2hiint(z) & 0x7FFFFFFFu) < 0x7FF00000u;
+}
+
 // One face per thread (flux_x: 88 B a cell and one Roe face; flux_y: 136 B, as
 // it adds to what flux_x wrote).  The sums of flux_y are read before the face
 // is formed, so that their latency is hidden behind it; square roots and
@@ -183,8 +191,8 @@ __global__ void __launch_bounds__(kThreads)
     const double qx1 = qx[id], qy1 = qy[id], z1 = dem[id], s1 = sqrth[id];
     const double qx2 = qx[id2], qy2 = qy[id2], z2 = dem[id2], s2 = sqrth[id2];
     // the sum of the square roots divides: it must be in range, too
-    if (regular_cell(h1, qx1, qy1) && regular_cell(h2, qx2, qy2) && K.hextra >= 0x1p-100 && s1 >= 0.0 && s2 >= 0.0 &&
-        s1 + s2 >= 0x1p-151 && s1 + s2 <= 0x1p51)
+    if (regular_cell(h1, qx1, qy1) && regular_cell(h2, qx2, qy2) && finite_bed(z1) && finite_bed(z2) &&
+        K.hextra >= 0x1p-100 && s1 >= 0.0 && s2 >= 0.0 && s1 + s2 >= 0x1p-151 && s1 + s2 <= 0x1p51)
       f = face_flux<double, XFACE, true>(cell_line(h1, qx1, qy1, z1, s1, K),
                                          cell_line(h2, qx2, qy2, z2, s2, K), K);
     else
