@@ -228,3 +228,29 @@ def test_bed_without_a_level_under_water_matches_oracle():
         assert d.get_clock().simtime == o.s.simtime
     finally:
         d.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_cells_without_a_depth_stay_apart(precision):
+    """A block of cells without a depth (NaN) inside dry land: its faces have
+    no water on either side and add nothing, so its discharges stay zero and
+    nothing spreads, as in the oracle (FP64: every bit)."""
+    from tests._harness import compare_fields, oracle_from_scenario
+    from triton_b200 import scenarios
+    sc = scenarios.mixed(rows=40, cols=61, seed=5, friction=False, with_extbc=False, with_sources=False,
+                         with_runoff=False, duration=1e3)
+    for f in (sc.h, sc.qx, sc.qy):
+        f[:14, :34] = 0.0
+    sc.h[2:7, 3:30] = np.nan
+    d = sc.to_domain(precision)
+    try:
+        assert d.advance(3) == (3, 0)
+        if precision == "fp64":
+            o = oracle_from_scenario(sc)
+            assert o.advance(3) == (3, 0)
+            compare_fields(o, d, True, sc.hextra)
+        assert np.array_equal(np.isnan(d.download("h")), np.isnan(sc.h))
+        for f in ("qx", "qy"):
+            assert not d.download(f)[2:7, 3:30].any()
+    finally:
+        d.close()

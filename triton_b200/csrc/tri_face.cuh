@@ -158,7 +158,7 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
   out.a0 = out.a1 = out.a2 = out.b0 = out.b1 = out.b2 = T(0);
 
   const T h1 = c1.h, h2 = c2.h;
-  const bool brink = h1 < E12 || h2 < E12;  // next to a dry cell
+  const bool brink = !(h1 >= E12 && h2 >= E12);  // next to a dry cell, or one whose depth is no number
   if (brink && !(h1 > T(0) || h2 > T(0))) return out;
 
   const T u1 = c1.u, v1 = c1.v, u2 = c2.u, v2 = c2.v;
