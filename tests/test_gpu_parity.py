@@ -254,3 +254,55 @@ def test_cells_without_a_depth_stay_apart(precision):
             assert not d.download(f)[2:7, 3:30].any()
     finally:
         d.close()
+
+
+@pytest.mark.parametrize("hextra", [0.0, 1e-300, 1e-40])
+def test_any_depth_threshold_matches_oracle(hextra):
+    """Thresholds down to zero (all wet there: a dry cell's velocity is 0/0),
+    whose films and their velocities have any size."""
+    from triton_b200 import scenarios
+    sc = scenarios.mixed(rows=40, cols=61, seed=53, friction=False, with_extbc=False, open_boundaries=1, duration=4.0)
+    sc.hextra = hextra
+    if hextra == 0.0:
+        sc.h += 0.25
+    else:
+        sc.h[9:13, 25:35] = hextra * 1.5  # at rest: a discharge there would leave the range of doubles
+        sc.qx[9:13, 25:35] = sc.qy[9:13, 25:35] = 0.0
+    steps, _ = run_lockstep(sc, exact=True, max_events=2, chunk=8)
+    assert steps > 1
+
+
+def _flux_us(sc):
+    """Time of a flux launch of an FP64 domain, the shortest of three runs of 16 steps."""
+    d = sc.to_domain()
+    best = 1e30
+    try:
+        d.set_clock(sim_duration=1e300, print_interval=1e300, time_series=0, it_print=0)
+        d.advance(8)
+        for _ in range(3):
+            d.set_timing(True)
+            d.advance(16)
+            ms, n, _, _ = d.get_timing()
+            best = min(best, 1e3 * ms / n)
+        d.set_timing(False)
+    finally:
+        d.close()
+    return best
+
+
+def _wet_square(n=700):
+    from triton_b200 import scenarios
+    sc = scenarios.mixed(rows=n, cols=n, seed=59, with_extbc=False, with_sources=False, duration=1e3)
+    rng = np.random.default_rng(59)
+    sc.h[1:-1, 1:-1] = 1.0 + 0.2 * rng.random((n, n))
+    sc.qx[:], sc.qy[:] = 0.0, 0.0
+    return sc
+
+
+def test_small_depth_threshold_takes_the_straight_line_form():
+    """With a threshold below 2^-100 no tile is computed twice (2.5 times the
+    launch when each was)."""
+    sc = _wet_square()
+    usual = _flux_us(sc)
+    sc.hextra = 1e-40
+    assert _flux_us(sc) < 1.5 * usual

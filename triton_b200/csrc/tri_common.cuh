@@ -178,7 +178,8 @@ __device__ __forceinline__ double div_line(double a, double b, double y) {
 
 // True where the straight-line forms are exact on everything a face of this
 // cell computes: h is 0 or within 2^-300 .. 2^100 and the discharges are at
-// most 2^100 in magnitude.  A depth whose low word is all ones is left out
+// most 2^100 in magnitude, so velocities are at most 2^400 whatever depth they
+// begin at, and no quotient passes 2^900.  A depth whose low word is all ones is left out
 // (see recip_line; one depth in 2^32).  (Quotients of dividends below 2^-900 can then be
 // off by 2^-700 at most, far below the 1e-12 flush of the contributions they
 // enter.)  Tested on the high words: integer slots, which the FP64 tile has.

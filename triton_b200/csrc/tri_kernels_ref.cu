@@ -192,7 +192,8 @@ __global__ void __launch_bounds__(kThreads)
     const double qx2 = qx[id2], qy2 = qy[id2], z2 = dem[id2], s2 = sqrth[id2];
     // the sum of the square roots divides: it must be in range, too
     if (regular_cell(h1, qx1, qy1) && regular_cell(h2, qx2, qy2) && finite_bed(z1) && finite_bed(z2) &&
-        K.hextra >= 0x1p-100 && s1 >= 0.0 && s2 >= 0.0 && s1 + s2 >= 0x1p-151 && s1 + s2 <= 0x1p51)
+        (K.hextra > 0.0 || (h1 > 0.0 && h2 > 0.0)) && s1 >= 0.0 && s2 >= 0.0 && s1 + s2 >= 0x1p-151 &&
+        s1 + s2 <= 0x1p51)
       f = face_flux<double, XFACE, true>(cell_line(h1, qx1, qy1, z1, s1, K),
                                          cell_line(h2, qx2, qy2, z2, s2, K), K);
     else

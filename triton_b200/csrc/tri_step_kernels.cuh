@@ -426,10 +426,11 @@ struct RowParts {
 };
 
 // A friction quotient's dividend that div_line takes: 0 (of either sign) or at
-// least 2^-900 (a transverse discharge can decay to any size).
+// least 2^-200 (a transverse discharge can decay to any size), which over a
+// friction term of 2^760 at most leaves a normal quotient.
 __device__ __forceinline__ bool line_dividend(double a) {
   const uint32_t hi = (uint32_t)__double2hiint(a) & 0x7FFFFFFFu;
-  return hi >= (1023u - 900u) << 20 || (hi | (uint32_t)__double2loint(a)) == 0u;
+  return hi >= (1023u - 200u) << 20 || (hi | (uint32_t)__double2loint(a)) == 0u;
 }
 
 // LINE (FP64): the straight-line forms; *odd is set where they do not hold.
@@ -488,10 +489,10 @@ __device__ __forceinline__ void update_cell(const CellQ<T>& c, const RowParts<T>
       modM = dev_sqrt(mm);
     }
     if (L64 && n2v > E12 && hn >= hextra && modM > E12) {
-      // dividend of the friction term: 2^-300 .. 2^200 keeps it, its
-      // reciprocal and its square root normal for every regular depth
+      // dividend of the friction term: 2^-300 .. 2^60 keeps it, its reciprocal
+      // and its square root normal for every regular depth (2^-700 .. 2^234 as den)
       const double num = dt * G * n2v * modM, den = hn * hn * dev_cbrt(hn);
-      odd |= (uint32_t)__double2hiint(num) - ((1023u - 300u) << 20) > (500u << 20);
+      odd |= (uint32_t)__double2hiint(num) - ((1023u - 300u) << 20) > (360u << 20);
       const double tt = div_line(num, den, recip_line(den));
       const double t4 = T(1) + T(4) * tt;
       const double sq = sqrt_line(t4, rsqrt_line(t4));
@@ -740,6 +741,14 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, FluxUnit u,
     }
   };
 
+  // with a threshold of zero or less a dry cell has velocities, 0/0 (looked for
+  // here: a test in the row loop costs every other domain up to 1 %)
+  if (kLine && !(hextra > T(0))) {
+    bool dry = false;
+    for (int r = r0 - 1; r <= r1 + 1; ++r) dry |= incol && X.hi[(size_t)r * cols + c] == T(0);
+    if (__any_sync(0xffffffffu, dry)) return false;
+  }
+
   // raw values of the next row are loaded one iteration ahead
   T lh = T(0), lqx = T(0), lqy = T(0), lz = T(0);
   auto fetch = [&](const FluxCtx<T>& Z, int r) {
@@ -752,7 +761,7 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, FluxUnit u,
     }
   };
   fetch(X, r0 - 1);
-  if (kLine) odd = !regular_cell(lh, lqx, lqy) || !(hextra >= T(0x1p-100));  // bounds the velocities
+  if (kLine) odd = !regular_cell(lh, lqx, lqy);
   CellQ<T> prev = make_cell<T, kLine>(lh, lqx, lqy, lz, X.K);
   if (r0 - 1 == 0 && owner) copy_ghost(X, 0);
   fetch(X, r0);
