@@ -684,6 +684,14 @@ __device__ __forceinline__ void take_part(FluxUnit* u, int part, int rb) {
   u->r1 = min(u->r1, u->r0 + part_rows(rb) - 1);
 }
 
+// Whether any lane's column h (row stride `cols`) holds a 0 in rows r .. z.
+template <typename T>
+__device__ __noinline__ bool column_dry(const T* h, int cols, int r, int z) {
+  bool dry = false;
+  for (; r <= z; ++r) dry |= h[(size_t)r * cols] == T(0);
+  return __any_sync(0xffffffffu, dry);
+}
+
 // One warp tile: strip sx (30 interior columns), rows r0..r1.  kTrack:
 // record in X.tz_dst whether the tile wrote only +0 (dry-tile skipping; the
 // kernels of domains that cannot skip are built without it).  kReload: the
@@ -743,11 +751,7 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, FluxUnit u,
 
   // with a threshold of zero or less a dry cell has velocities, 0/0 (looked for
   // here: a test in the row loop costs every other domain up to 1 %)
-  if (kLine && !(hextra > T(0))) {
-    bool dry = false;
-    for (int r = r0 - 1; r <= r1 + 1; ++r) dry |= incol && X.hi[(size_t)r * cols + c] == T(0);
-    if (__any_sync(0xffffffffu, dry)) return false;
-  }
+  if (kLine && !(hextra > T(0)) && column_dry<T>(X.hi + c, cols, r0 - 1, incol ? r1 + 1 : r0 - 2)) return false;
 
   // raw values of the next row are loaded one iteration ahead
   T lh = T(0), lqx = T(0), lqy = T(0), lz = T(0);
