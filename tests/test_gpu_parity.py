@@ -306,3 +306,20 @@ def test_small_depth_threshold_takes_the_straight_line_form():
     usual = _flux_us(sc)
     sc.hextra = 1e-40
     assert _flux_us(sc) < 1.5 * usual
+
+
+def test_depths_of_minus_zero_are_dry_land():
+    """Depths of -0.0 equal the oracle's run bit for bit, and a tile with
+    them is computed once (1.5 times the launch when it was twice)."""
+    from triton_b200 import scenarios
+    sc = scenarios.mixed(rows=40, cols=61, seed=61, friction=False, duration=4.0)
+    sc.extbc = None
+    sc.h[sc.h == 0.0] = -0.0
+    run_lockstep(sc, exact=True, max_events=2, chunk=6)
+    times = []
+    for dry in (0.0, -0.0):
+        sc = _wet_square()
+        sc.runoff = None
+        sc.h[np.random.default_rng(67).random(sc.h.shape) < 0.5] = dry
+        times.append(_flux_us(sc))
+    assert times[1] < 1.25 * times[0], times

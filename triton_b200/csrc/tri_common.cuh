@@ -177,17 +177,18 @@ __device__ __forceinline__ double div_line(double a, double b, double y) {
 }
 
 // True where the straight-line forms are exact on everything a face of this
-// cell computes: h is 0 or within 2^-300 .. 2^100 and the discharges are at
-// most 2^100 in magnitude, so velocities are at most 2^400 whatever depth they
-// begin at, and no quotient passes 2^900.  A depth whose low word is all ones is left out
-// (see recip_line; one depth in 2^32).  (Quotients of dividends below 2^-900 can then be
-// off by 2^-700 at most, far below the 1e-12 flush of the contributions they
-// enter.)  Tested on the high words: integer slots, which the FP64 tile has.
+// cell computes: h is 0 (of either sign, as rasters hold it) or within 2^-300 ..
+// 2^100 and the discharges are at most 2^100 in magnitude, so velocities are at
+// most 2^400 whatever depth they begin at, and no quotient passes 2^900.  A
+// depth whose low word is all ones is left out (see recip_line; one depth in
+// 2^32).  (Quotients of dividends below 2^-900 can then be off by 2^-700 at
+// most, far below the 1e-12 flush of the contributions they enter.)  Tested on
+// the high words: integer slots, which the FP64 tile has.
 __device__ __forceinline__ bool regular_cell(double h, double qx, double qy) {
   constexpr uint32_t kLo = (1023u - 300u) << 20, kHi = (1023u + 100u) << 20;
   const uint32_t hh = (uint32_t)__double2hiint(h), hl = (uint32_t)__double2loint(h);
   const uint32_t ax = (uint32_t)__double2hiint(qx) & 0x7FFFFFFFu, ay = (uint32_t)__double2hiint(qy) & 0x7FFFFFFFu;
-  const bool hok = (hh - kLo <= kHi - kLo && hl != 0xFFFFFFFFu) || (hh | hl) == 0u;
+  const bool hok = (hh - kLo <= kHi - kLo && hl != 0xFFFFFFFFu) || ((hh & 0x7FFFFFFFu) | hl) == 0u;
   return hok && max(ax, ay) <= kHi;
 }
 __device__ __forceinline__ bool regular_cell(float, float, float) { return true; }
