@@ -242,3 +242,60 @@ def test_flux_over_nonfinite_beds_matches_oracle(oracle, value):
     want, got = _flux_both(oracle, R, Cc, h, zero, zero, z, np.sqrt(h), 1e-3)
     for a, b in zip(want, got):
         assert np.isfinite(a).all() and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("R,Cc", [(3, 3), (3, 9), (9, 3), (4, 4), (5, 7), (43, 61)])
+def test_extbc_lists_of_any_cells_match_oracle(oracle, R, Cc):
+    """Lists of cells of the whole grid, ghosts and corners among them, in any
+    order and repeated; some cells write into others' ghosts."""
+    import torch
+    from triton_b200 import _abi
+    L, O = _abi.lib(), oracle.lib()
+    O.tor_compute_extbc_values.restype = None
+    for n in (2, 5, 33, 700, 5000):
+        rng = np.random.default_rng(100 * R + Cc + n)
+        cells = rng.integers(0, R * Cc, n).astype(np.int32)
+        types = rng.choice(np.array([0, 1, 3], np.int32), n).astype(np.int32)
+        start, nrows = np.where(types == 1, 0, 4).astype(np.int32), np.where(types == 1, 4, 1).astype(np.int32)
+        v1, v2 = np.array([0.0, 5.0, 9.0, 30.0, 0.7]), np.array([6.0, 7.0, 6.5, 6.5, 0.7])
+        h, qx, qy = rng.random(R * Cc) * 2.0, rng.standard_normal(R * Cc), rng.standard_normal(R * Cc)
+        z, n2 = 5.0 + rng.random(R * Cc), np.full(R * Cc, 1e-3)
+        dev = [_dev(torch, a.copy()) for a in (h, qx, qy, z, n2, cells, types, start, nrows, v1, v2)]
+        O.tor_compute_extbc_values(n, R, Cc, C.c_double(0.1), *[a.ctypes.data_as(_dp) for a in (h, qx, qy, z, n2)],
+                                   *[a.ctypes.data_as(_ip) for a in (cells, types, start, nrows)],
+                                   v1.ctypes.data_as(_dp), v2.ctypes.data_as(_dp), C.c_double(7.0))
+        _abi.check(L.tri_kernel_compute_extbc_values_f64(n, R, Cc, 0.1, *[_p(t) for t in dev], 7.0, 0, 1, None))
+        torch.cuda.synchronize()
+        for a, t in zip((h, qx, qy), dev):
+            assert np.array_equal(t.cpu().numpy(), a)
+
+
+def test_extbc_lists_with_ghosts_or_repeats_stay_parallel():
+    """A list of 8192 cells with a ghost in it, or with cells listed twice, takes
+    no more than a few times a list of distinct interior cells (one thread for
+    all of it took a hundred times as long, a thread's search for a cell's later
+    items fifteen times)."""
+    import torch
+    from triton_b200 import _abi
+    L, R, n = _abi.lib(), 2052, 8192
+    edge = [r * R + c for r in (1, R - 2) for c in range(1, R - 1)] + [r * R + c for r in range(2, R - 2) for c in (1, R - 2)]
+    edge = np.random.default_rng(1).permutation(np.array(edge, np.int32))
+    f = [torch.rand(R * R, dtype=torch.float64, device="cuda") for _ in range(5)]
+    types, zero = torch.full((n,), 3, dtype=torch.int32, device="cuda"), torch.zeros(n, dtype=torch.int32, device="cuda")
+    one, v = torch.ones(n, dtype=torch.int32, device="cuda"), torch.full((1,), 0.3, dtype=torch.float64, device="cuda")
+    us = {}
+    for name, cells in (("plain", edge[:n]), ("ghost", np.append(edge[:n - 1], np.int32(1))), ("twice", np.tile(edge[:n // 2], 2))):
+        t = _dev(torch, cells.astype(np.int32))
+        best = 1e30
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(10):
+                _abi.check(L.tri_kernel_compute_extbc_values_f64(
+                    n, R, R, 0.1, *[_p(x) for x in f], _p(t), _p(types), _p(zero), _p(one), _p(v), _p(v), 1.0, 0, 1,
+                    C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b) * 100.0)
+        us[name] = best
+    assert us["ghost"] < 4 * us["plain"] and us["twice"] < 4 * us["plain"], us

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <mutex>
 #include <vector>
 
@@ -439,54 +440,126 @@ __global__ void kr_extbc(const int32_t* __restrict__ order, int count, int nrows
   extbc_item(order[k], nrows, ncols, dt, h, qx, qy, dem, n, rel, types, start, nvars, v1, v2, simtime, rank, nproc);
 }
 
+// Cells of one group are applied in list order; items of two groups touch
+// different cells.  An item writes its own cell and, next to an edge, ghosts
+// beside it.  A ghost off the corners belongs to one interior cell and is
+// inactive itself, so a cell is its own group but for the two by two at each
+// corner, which write into one another (checked against the touched cells of
+// every pair, grids of 3x3 to 8x8, first, inner and last ranks).  With three
+// rows or columns two corners are one; smaller grids are one group.
+__device__ __forceinline__ int extbc_group(int c, int nrows, int ncols) {
+  if (nrows < 3 || ncols < 3) return 0;
+  if (c < 0) return c;  // outside: nothing to apply
+  const int r = c / ncols, q = c - r * ncols;
+  const int a = r <= 1 || nrows == 3 ? 0 : (r >= nrows - 2 ? 1 : -1);
+  const int b = q <= 1 || ncols == 3 ? 0 : (q >= ncols - 2 ? 1 : -1);
+  return a < 0 || b < 0 ? c : INT_MIN + 2 * a + b;
+}
+
 // The whole list in one launch, in the reference's serial order where it
 // matters, without a look at it on the host (a copy back, a synchronization
-// and a comparison, about 25 us a call): items on different interior cells
-// touch different cells, so the first item of a cell runs at once and takes
-// the cell's later items after it.  A warp per item looks through the list
-// (1403 cells: 6.8 us; a thread per item took 31), which a block reads and
-// checks together.  A list with a cell that is not interior is applied by one thread.
+// and a comparison, about 25 us a call): the first item of a group runs at once
+// and takes the group's later items after it.  A warp looks through the list
+// for four items (a comparison each per cell it reads, which a block reads
+// together), then looks again for those with more than one later item.  A call
+// with 1403 cells 11 us, 4096 14, 8192 27 (with a ghost among them 26, each cell
+// twice 24, 227 cells 36 times each 118), against 24, 29 and 32 (38, 36, 177)
+// with the order found on the host; above 8192 the look, which grows with the
+// square, costs more.
 constexpr int kExtbcScan = 8192;
 constexpr int kScanThreads = 256;
+constexpr int kScanItems = 4;  // of a warp
 __global__ void __launch_bounds__(kScanThreads)
     kr_extbc_scan(int size, int nrows, int ncols, double dt, double* h, double* qx, double* qy,
                   const double* __restrict__ dem, const double* __restrict__ n, const int32_t* __restrict__ rel,
                   const int32_t* __restrict__ types, const int32_t* __restrict__ start,
                   const int32_t* __restrict__ nvars, const double* __restrict__ v1, const double* __restrict__ v2,
                   double simtime, int rank, int nproc) {
-  constexpr int kChunk = 2048;
-  __shared__ int32_t s_cell[kChunk];
-  const int lane = threadIdx.x & 31, k = blockIdx.x * (kScanThreads / 32) + (threadIdx.x >> 5);
-  const int mine = k < size ? rel[k] : -1;
-  bool earlier = k >= size, later = false, odd = false;
+  constexpr int kChunk = 4096;
+  constexpr int kNone = INT_MIN + 4;  // no group
+  __shared__ __align__(16) int32_t s_group[kChunk];
+  const int lane = threadIdx.x & 31;
+  const int k0 = (blockIdx.x * (kScanThreads / 32) + (int)(threadIdx.x >> 5)) * kScanItems;
+  int mine[kScanItems];
+  unsigned head[kScanItems], last[kScanItems], count[kScanItems];  // first, last and number of the group's items
+#pragma unroll
+  for (int i = 0; i < kScanItems; i++) {
+    mine[i] = k0 + i < size ? extbc_group(rel[k0 + i], nrows, ncols) : kNone;
+    head[i] = 0xFFFFFFFFu;
+    last[i] = count[i] = 0;
+  }
   for (int base = 0; base < size; base += kChunk) {
     const int m = min(kChunk, size - base);
     __syncthreads();
-    for (int j = threadIdx.x; j < m; j += kScanThreads) {
-      const int c = rel[base + j], r = c / ncols, q = c - r * ncols;
-      s_cell[j] = c;
-      odd |= c < 0 || r < 1 || r > nrows - 2 || q < 1 || q > ncols - 2;
-    }
+    for (int j = threadIdx.x; j < (m + 3) / 4 * 4; j += kScanThreads)
+      s_group[j] = j < m ? extbc_group(rel[base + j], nrows, ncols) : kNone;
     __syncthreads();
-    for (int j = lane; j < m; j += 32) {
-      const bool same = s_cell[j] == mine;
-      earlier |= same && base + j < k;
-      later |= same && base + j > k;
+    for (int j = 4 * lane; j < m; j += 128) {
+      const int4 v = *reinterpret_cast<const int4*>(&s_group[j]);
+      const int g[4] = {v.x, v.y, v.z, v.w};
+      bool hit = false;
+#pragma unroll
+      for (int i = 0; i < kScanItems; i++) hit |= v.x == mine[i] || v.y == mine[i] || v.z == mine[i] || v.w == mine[i];
+      if (!hit) continue;
+#pragma unroll
+      for (int i = 0; i < 4 * kScanItems; i++)
+        if (g[i & 3] == mine[i >> 2]) {
+          head[i >> 2] = min(head[i >> 2], (unsigned)(base + j + (i & 3)));
+          last[i >> 2] = (unsigned)(base + j + (i & 3));
+          count[i >> 2]++;
+        }
     }
   }
-  const bool first = !__any_sync(0xffffffffu, earlier) && lane == 0;
-  const bool more = __any_sync(0xffffffffu, later);
-  if (__syncthreads_or(odd)) {
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-      for (int j = 0; j < size; j++)
-        extbc_item(j, nrows, ncols, dt, h, qx, qy, dem, n, rel, types, start, nvars, v1, v2, simtime, rank, nproc);
-    return;
+  // lane i applies the group of item k0 + i if that is its first; last: of a
+  // group with more than one later item, which are looked for again below
+  unsigned my_last = 0, my_count = 0, end = 0;
+#pragma unroll
+  for (int i = 0; i < kScanItems; i++) {
+    const bool leads = __reduce_min_sync(0xffffffffu, head[i]) == (unsigned)(k0 + i) && k0 + i < size;
+    const unsigned l = __reduce_max_sync(0xffffffffu, last[i]), c = __reduce_add_sync(0xffffffffu, count[i]);
+    if (lane == i && leads) {
+      my_last = l;
+      my_count = c;
+    }
+    last[i] = leads && c > 2 ? l : 0;
+    end = max(end, last[i]);
   }
-  if (!first) return;
-  extbc_item(k, nrows, ncols, dt, h, qx, qy, dem, n, rel, types, start, nvars, v1, v2, simtime, rank, nproc);
-  for (int j = k + 1; more && j < size; j++)
-    if (rel[j] == mine)
-      extbc_item(j, nrows, ncols, dt, h, qx, qy, dem, n, rel, types, start, nvars, v1, v2, simtime, rank, nproc);
+  auto apply = [&](unsigned id) {
+    extbc_item((int)id, nrows, ncols, dt, h, qx, qy, dem, n, rel, types, start, nvars, v1, v2, simtime, rank, nproc);
+  };
+#pragma unroll 1
+  for (unsigned pass = 1; pass <= 2; pass++)  // the first item, then an only later one
+    if (pass == 1 ? my_count > 0 : my_count == 2) apply(pass == 1 ? (unsigned)(k0 + lane) : my_last);
+  if (end == 0) return;
+#pragma unroll 1
+  for (unsigned b = (unsigned)k0 & ~31u; b <= end; b += 128) {
+    int g[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const unsigned j = b + 32 * u + lane;
+      g[u] = j <= end ? extbc_group(rel[j], nrows, ncols) : kNone;
+    }
+#pragma unroll 1
+    for (unsigned at = b; at < b + 128; at += 32) {
+      unsigned todo = 0;
+#pragma unroll
+      for (int i = 0; i < kScanItems; i++) {
+        const unsigned j = at + lane;
+        const unsigned same = __ballot_sync(0xffffffffu, g[0] == mine[i] && j > (unsigned)(k0 + i) && j <= last[i]);
+        if (lane == i) todo = same;
+      }
+      for (; todo != 0; todo &= todo - 1) apply(at + (unsigned)__ffs(todo) - 1);
+      __syncwarp();
+      g[0] = g[1];
+      g[1] = g[2];
+      g[2] = g[3];
+    }
+  }
+}
+
+inline unsigned extbc_scan_blocks(int size) {
+  constexpr int per = kScanThreads / 32 * kScanItems;
+  return (unsigned)((size + per - 1) / per);
 }
 
 __global__ void kr_copy_obs(int size, const double* __restrict__ arr, double* __restrict__ out,
@@ -652,7 +725,7 @@ int tri_kernel_compute_extbc_values_f64(int size, int nrows, int ncols, double d
   if (size <= 0) return TRI_OK;
   TRI_CHECK_ARG(relative_index && extbctype && start_index && nrows_vars, "null device pointer");
   if (size <= kExtbcScan) {
-    kr_extbc_scan<<<(size + kScanThreads / 32 - 1) / (kScanThreads / 32), kScanThreads, 0, as_stream(stream)>>>(
+    kr_extbc_scan<<<extbc_scan_blocks(size), kScanThreads, 0, as_stream(stream)>>>(
         size, nrows, ncols, dt, h, qx, qy, dem, n, relative_index, extbctype, start_index, nrows_vars, extbcvar1,
         extbcvar2, simtime, rank, total_process);
     return launched();
@@ -757,7 +830,7 @@ extern "C" int tri_kernel_compute_extbc_values_noalloc_f64(
                 size, kNoAllocExtbcMaxCells);
   TRI_CHECK_ARG(relative_index && extbctype && start_index && nrows_vars, "null device pointer");
   if (size <= kExtbcScan) {
-    kr_extbc_scan<<<(size + kScanThreads / 32 - 1) / (kScanThreads / 32), kScanThreads, 0, as_stream(stream)>>>(
+    kr_extbc_scan<<<extbc_scan_blocks(size), kScanThreads, 0, as_stream(stream)>>>(
         size, nrows, ncols, dt, h, qx, qy, dem, n, relative_index, extbctype, start_index, nrows_vars, extbcvar1,
         extbcvar2, simtime, rank, total_process);
     return launched();
