@@ -97,3 +97,41 @@ def test_batch_rejects_bad_members():
     finally:
         a.close()
         b.close()
+
+
+@pytest.mark.parametrize("precision,small", [("fp64", 760), ("fp32", 1200)])
+def test_a_large_member_among_many_small_ones_keeps_its_blocks(precision, small):
+    """More members than the post kernel has resident blocks: a large one is not
+    left to one block (the step took ten times the parts' own steps)."""
+    import torch
+    from triton_b200.domain import Domain
+
+    def flat(rows, cols):
+        d = Domain(rows, cols, 1.0, 0.5, 1e-3, 0, precision)
+        d.upload("h", 1.0 + 0.1 * np.random.default_rng(rows).random((rows, cols)))
+        d.set_clock(sim_duration=1e300, print_interval=1e300, it_print=0)
+        return d
+
+    def step_us(members):
+        with Batch(members) as b:
+            b.launch(8)
+            b.wait()
+            best = 1e30
+            for _ in range(3):
+                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                torch.cuda.synchronize()
+                e0.record()
+                b.launch(32)
+                b.wait()
+                e1.record()
+                torch.cuda.synchronize()
+                best = min(best, e0.elapsed_time(e1) / 32 * 1e3)
+            return best
+
+    large, others = flat(1026, 1026), [flat(18, 20) for _ in range(small)]
+    try:
+        alone, rest, both = step_us([large]), step_us(others), step_us([large] + others)
+        assert both < 2.0 * (alone + rest), (alone, rest, both)
+    finally:
+        for d in [large] + others:
+            d.close()

@@ -131,17 +131,23 @@ inline uint32_t post_blocks(uint32_t tiles, uint32_t per) { return (tiles + 4 * 
 // fewest with which all blocks are resident, `per_sm` on an SM.  A member's last
 // block is rarely full, so the blocks' sum decides, not the tiles' total: a few
 // blocks above the places took a second round (48 members of 256^2 to 1024^2,
-// FP64, 8-row tiles: 1272 -> 1169 us a step; no change where they fit).
+// FP64, 8-row tiles: 1272 -> 1169 us a step; no change where they fit).  Up to
+// twice the even share: with nearly as many members as places, or more, a
+// second round of short blocks costs less than a large member in a few blocks
+// (760 members of 16x18 and one of 1024^2, FP64: 454 us a step, 5537 with one
+// block for each; 1200 in FP32 632 and 4493).
 template <typename F>
 uint32_t post_tiles_per_warp(size_t n, uint32_t per_sm, F tiles) {
-  const uint64_t places = std::max<uint64_t>(148 * per_sm, n);  // a member has one block at least
+  const uint64_t places = 148 * per_sm;
   uint64_t all = 0;
   for (size_t m = 0; m < n; m++) all += tiles(m);
-  for (uint32_t per = (uint32_t)std::max<uint64_t>((all + 4 * places - 1) / (4 * places), 1);; per++) {
+  const uint32_t share = (uint32_t)std::max<uint64_t>((all + 4 * places - 1) / (4 * places), 1);
+  for (uint32_t per = share; per <= 2 * share; per++) {
     uint64_t blocks = 0;
     for (size_t m = 0; m < n; m++) blocks += post_blocks(tiles(m), per);
     if (blocks <= places) return per;
   }
+  return share;
 }
 // CFL dt of the current state into the slot the next step reads.
 template <typename T>
