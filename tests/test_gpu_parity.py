@@ -323,3 +323,20 @@ def test_depths_of_minus_zero_are_dry_land():
         sc.h[np.random.default_rng(67).random(sc.h.shape) < 0.5] = dry
         times.append(_flux_us(sc))
     assert times[1] < 1.25 * times[0], times
+
+
+def test_autotune_tries_the_default_shape():
+    """The default height of this grid (3 rows) is not one of the heights that
+    every budget is tried at; the default is tried beside them, alone and in a
+    batch.  A default among them is not tried twice."""
+    from triton_b200 import scenarios
+    from triton_b200.batch import Batch
+    for cols, tried in ((1050, 31), (200, 30)):
+        sc = scenarios.mixed(rows=200, cols=cols, seed=73, with_extbc=False, duration=1e3)
+        d = sc.to_domain()
+        try:
+            assert d.autotune(2)["candidates"] == tried
+            with Batch([d]) as b:
+                assert b.autotune(2)["candidates"] == tried
+        finally:
+            d.close()

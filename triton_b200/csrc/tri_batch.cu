@@ -213,14 +213,17 @@ int build_table(tri_batch* b) {
 int rebuild(tri_batch* b) { return b->prec == TRI_FP64 ? build_table<double>(b) : build_table<float>(b); }
 
 // The default shape for the present members (batched steps compute every tile).
-void choose_shape(tri_batch* b) {
-  if (b->shape_set || b->members.empty()) return;
-  const FluxShape s = flux_shape(b->prec == TRI_FP64, true, 1.0, [&](int rb) {
+FluxShape default_shape(const tri_batch* b) {
+  return flux_shape(b->prec == TRI_FP64, true, 1.0, [&](int rb) {
     int64_t n = 0;
     for (const tri_domain* d : b->members)
       n += (int64_t)((d->desc.cols - 2 + kStripCols - 1) / kStripCols) * ((d->desc.rows - 2 + rb - 1) / rb);
     return n;
   });
+}
+void choose_shape(tri_batch* b) {
+  if (b->shape_set || b->members.empty()) return;
+  const FluxShape s = default_shape(b);
   b->variant = s.variant;
   b->rb = s.rb;
 }
@@ -586,41 +589,39 @@ int tri_batch_autotune(tri_batch* b, int32_t trial_steps, tri_tuning* out) {
     }
     return TRI_OK;
   };
-  const int heights[] = {1, 2, 4, 8, 16, 32};
   double best = 1e300;
   int best_v = b->variant, best_rb = b->rb, ncand = 0;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  for (int v = 0; v < kFluxVariants && rc == TRI_OK; v++) {
-    for (size_t hi = 0; hi < sizeof(heights) / sizeof(heights[0]) && rc == TRI_OK; hi++) {
-      b->variant = v;
-      b->rb = heights[hi];
-      rc = rebuild(b);
-      if (rc == TRI_OK) rc = restore();
-      for (tri_domain* d : b->members) {  // trials run without events
-        d->mirror->sim_duration = d->mirror->print_interval = d->mirror->print_observation = 1e300;
-        d->mirror->it_print = 0;
-        d->mirror->time_series = 0;
-      }
-      int runnable = 0;
-      if (rc == TRI_OK) rc = prepare_members(b, INT32_MAX, &runnable);
-      if (rc == TRI_OK) rc = reset_ctl(b);
-      if (rc == TRI_OK) rc = launch_clocks(b);
-      if (rc == TRI_OK) rc = launch_batch(b, 2);  // warm-up, also builds the graph
-      cudaEventRecord(e0, b->stream);
-      if (rc == TRI_OK) rc = launch_batch(b, trial_steps);
-      cudaEventRecord(e1, b->stream);
-      if (cudaEventSynchronize(e1) != cudaSuccess && rc == TRI_OK)
-        rc = set_error(TRI_E_CUDA, "batch autotune trial failed");
-      float ms = 0;
-      cudaEventElapsedTime(&ms, e0, e1);
-      ncand++;
-      if (rc == TRI_OK && ms / trial_steps < best) {
-        best = ms / trial_steps;
-        best_v = v;
-        best_rb = heights[hi];
-      }
+  for (const FluxShape& shape : tuning_shapes(default_shape(b))) {
+    if (rc != TRI_OK) break;
+    b->variant = shape.variant;
+    b->rb = shape.rb;
+    rc = rebuild(b);
+    if (rc == TRI_OK) rc = restore();
+    for (tri_domain* d : b->members) {  // trials run without events
+      d->mirror->sim_duration = d->mirror->print_interval = d->mirror->print_observation = 1e300;
+      d->mirror->it_print = 0;
+      d->mirror->time_series = 0;
+    }
+    int runnable = 0;
+    if (rc == TRI_OK) rc = prepare_members(b, INT32_MAX, &runnable);
+    if (rc == TRI_OK) rc = reset_ctl(b);
+    if (rc == TRI_OK) rc = launch_clocks(b);
+    if (rc == TRI_OK) rc = launch_batch(b, 2);  // warm-up, also builds the graph
+    cudaEventRecord(e0, b->stream);
+    if (rc == TRI_OK) rc = launch_batch(b, trial_steps);
+    cudaEventRecord(e1, b->stream);
+    if (cudaEventSynchronize(e1) != cudaSuccess && rc == TRI_OK)
+      rc = set_error(TRI_E_CUDA, "batch autotune trial failed");
+    float ms = 0;
+    cudaEventElapsedTime(&ms, e0, e1);
+    ncand++;
+    if (rc == TRI_OK && ms / trial_steps < best) {
+      best = ms / trial_steps;
+      best_v = shape.variant;
+      best_rb = shape.rb;
     }
   }
   cudaEventDestroy(e0);

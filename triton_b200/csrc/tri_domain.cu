@@ -309,10 +309,12 @@ void size_flux_grid(tri_domain* d) {
 
 // Default shape before any tuning (flux_shape); a domain with runoff computes
 // every tile, one without about half of them.
+FluxShape default_shape(const tri_domain* d) {
+  return flux_shape(d->prec == TRI_FP64, false, d->nroff > 0 ? 1.0 : 0.5,
+                    [&](int rb) { return flux_tiles(d, rb); });
+}
 void choose_shape(tri_domain* d) {
-  const int64_t rows = d->desc.rows - 2, strips = (d->desc.cols - 2 + kStripCols - 1) / kStripCols;
-  const FluxShape s = flux_shape(d->prec == TRI_FP64, false, d->nroff > 0 ? 1.0 : 0.5,
-                                 [&](int rb) { return strips * ((rows + rb - 1) / rb); });
+  const FluxShape s = default_shape(d);
   d->flux_variant = s.variant;
   d->rb = s.rb;
   d->tile_lists_dirty = true;
@@ -1004,7 +1006,6 @@ int tri_domain_autotune(tri_domain* d, int32_t trial_steps, tri_tuning* out) {
     return TRI_OK;
   };
   int rc = save_restore(true);
-  const int heights[] = {1, 2, 4, 8, 16, 32};
   double best = 1e300;
   int best_v = d->flux_variant, best_rb = d->rb, ncand = 0;
   cudaEvent_t e0, e1;
@@ -1012,40 +1013,39 @@ int tri_domain_autotune(tri_domain* d, int32_t trial_steps, tri_tuning* out) {
   cudaEventCreate(&e1);
   const bool timing = d->timing;
   d->timing = false;
-  for (int v = 0; v < kFluxVariants && rc == TRI_OK; v++) {
-    for (size_t hi = 0; hi < sizeof(heights) / sizeof(heights[0]) && rc == TRI_OK; hi++) {
-      if (heights[hi] > std::max(8, d->desc.rows - 2)) continue;
-      d->flux_variant = v;
-      d->rb = heights[hi];
-      d->tile_lists_dirty = true;
-      size_flux_grid(d);
-      drop_graph(d);
-      rc = save_restore(false);
-      if (rc == TRI_OK) rc = reset_tiles(d);  // the other buffer holds the last trial's state
-      if (rc != TRI_OK) break;
-      *m = saved;
-      m->sim_duration = m->print_interval = m->print_observation = 1e300;
-      m->it_print = 0;
-      m->time_series = 0;
-      m->halt = 0;
-      m->steps = 0;
-      m->limit = INT32_MAX;
-          m->dt_key[m->rd] = kDtKeyInf;
-      rc = push_clock(d);
-      if (rc == TRI_OK) rc = launch_dt(d);
-      if (rc == TRI_OK) rc = launch_steps(d, 2);  // warm-up (also builds the graph)
-      cudaEventRecord(e0, d->stream);
-      if (rc == TRI_OK) rc = launch_steps(d, trial_steps);
-      cudaEventRecord(e1, d->stream);
-      if (cudaEventSynchronize(e1) != cudaSuccess) rc = set_error(TRI_E_CUDA, "autotune trial failed");
-      float ms = 0;
-      cudaEventElapsedTime(&ms, e0, e1);
-      ncand++;
-      if (rc == TRI_OK && ms / trial_steps < best) {
-        best = ms / trial_steps;
-        best_v = v;
-        best_rb = heights[hi];
-      }
+  for (const FluxShape& shape : tuning_shapes(default_shape(d))) {
+    if (rc != TRI_OK) break;
+    if (shape.rb > std::max(8, d->desc.rows - 2)) continue;
+    d->flux_variant = shape.variant;
+    d->rb = shape.rb;
+    d->tile_lists_dirty = true;
+    size_flux_grid(d);
+    drop_graph(d);
+    rc = save_restore(false);
+    if (rc == TRI_OK) rc = reset_tiles(d);  // the other buffer holds the last trial's state
+    if (rc != TRI_OK) break;
+    *m = saved;
+    m->sim_duration = m->print_interval = m->print_observation = 1e300;
+    m->it_print = 0;
+    m->time_series = 0;
+    m->halt = 0;
+    m->steps = 0;
+    m->limit = INT32_MAX;
+    m->dt_key[m->rd] = kDtKeyInf;
+    rc = push_clock(d);
+    if (rc == TRI_OK) rc = launch_dt(d);
+    if (rc == TRI_OK) rc = launch_steps(d, 2);  // warm-up (also builds the graph)
+    cudaEventRecord(e0, d->stream);
+    if (rc == TRI_OK) rc = launch_steps(d, trial_steps);
+    cudaEventRecord(e1, d->stream);
+    if (cudaEventSynchronize(e1) != cudaSuccess) rc = set_error(TRI_E_CUDA, "autotune trial failed");
+    float ms = 0;
+    cudaEventElapsedTime(&ms, e0, e1);
+    ncand++;
+    if (rc == TRI_OK && ms / trial_steps < best) {
+      best = ms / trial_steps;
+      best_v = shape.variant;
+      best_rb = shape.rb;
     }
   }
   cudaEventDestroy(e0);
@@ -1066,6 +1066,7 @@ int tri_domain_autotune(tri_domain* d, int32_t trial_steps, tri_tuning* out) {
   if (rc != TRI_OK) return rc;
   if (rc2 != TRI_OK) return rc2;
   d->tuned_ms = best;
+  d->tuned_candidates = ncand;
   return tri_domain_get_tuning(d, out);
 }
 
@@ -1073,7 +1074,7 @@ int tri_domain_get_tuning(tri_domain* d, tri_tuning* out) {
   TRI_CHECK_ARG(d && out, "null argument");
   out->variant = d->flux_variant;
   out->rows_per_tile = d->rb;
-  out->candidates = kFluxVariants * 6;
+  out->candidates = d->tuned_candidates;
   out->flux_blocks = d->flux_blocks;
   out->ms_per_step = d->tuned_ms;
   return TRI_OK;

@@ -78,6 +78,7 @@ struct tri_domain {
   int32_t* maxh_neg = nullptr;  // device flag: an uploaded max depth is negative (or NaN)
   int64_t work_steps = 0;       // steps advance() ran since tri_domain_set_timing
   double tuned_ms = 0;
+  int tuned_candidates = tri::kFluxVariants * 6;  // shapes the autotuner tried
   // graph of 'graph_steps' steps
   cudaGraphExec_t graph = nullptr;
   int graph_steps = 0;

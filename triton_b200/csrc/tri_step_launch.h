@@ -9,6 +9,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <vector>
 
 #include "tri_types.cuh"
 
@@ -63,6 +64,19 @@ FluxShape flux_shape(bool fp64, bool batch, double share, F tiles) {
   for (int rb : {6, 8, 12, 16, 24, 32})
     if (share * (double)tiles(rb) >= 4 * slots) best = rb;
   return {fp64 ? 0 : (batch ? 1 : 2), best};
+}
+// What the autotuners time: every budget at heights 1 to 32, and the default
+// shape where its height is another.
+inline std::vector<FluxShape> tuning_shapes(FluxShape def) {
+  std::vector<FluxShape> v;
+  bool listed = false;
+  for (int variant = 0; variant < kFluxVariants; variant++)
+    for (int rb : {1, 2, 4, 8, 16, 32}) {
+      v.push_back({variant, rb});
+      listed |= variant == def.variant && rb == def.rb;
+    }
+  if (!listed) v.push_back(def);
+  return v;
 }
 // Blocks of 128 threads per SM that the post kernels are compiled for: a stream
 // with two rows of loads in flight per warp, so as many as its registers allow
