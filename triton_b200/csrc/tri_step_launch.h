@@ -50,8 +50,12 @@ struct FluxBudget<float> {
 // faster: bowl 2048^2 97.4 us at 4 blocks per SM, 100.0 at 5, 112 at 6).  FP32
 // is bound by issue and takes 8 blocks per SM (rain 2048^2 129 us, 137 at 5),
 // but where one round holds all tiles the largest budget (bowl 256^2 12.6 us,
-// 14.0), and a batch, which reads its context from shared memory, 6 (24 members
-// 230 us a step, 240 at 8).
+// 14.0).  A batch, which reads its context from shared memory and spills more,
+// takes 6 while its tiles are short (members, cells in all, height: 11, 1.0 M, 8
+// rows 58.9 us a step, 61.2 at 8 blocks; 9, 1.2 M, 8 rows 67.1 and 68.6; 24, 2.6
+// M, 8 rows 123.9 and 124.2), 8 from 12 rows on (16, 4.0 M 172.0 us at 6 and
+// 171.7 at 8; 24, 6.0 M 233.1 and 230.7; 24, 9.6 M 350.6 and 342.8; 48, 16.3 M
+// 558 and 548; 256, 263 M 8369 and 8168).
 struct FluxShape {
   int variant, rb;
 };
@@ -63,7 +67,7 @@ FluxShape flux_shape(bool fp64, bool batch, double share, F tiles) {
   int best = 4;
   for (int rb : {6, 8, 12, 16, 24, 32})
     if (share * (double)tiles(rb) >= 4 * slots) best = rb;
-  return {fp64 ? 0 : (batch ? 1 : 2), best};
+  return {fp64 ? 0 : (batch && best < 12 ? 1 : 2), best};
 }
 // What the autotuners time: every budget at heights 1 to 32, and the default
 // shape where its height is another.
