@@ -182,13 +182,15 @@ __device__ __forceinline__ double div_line(double a, double b, double y) {
 // most 2^400 whatever depth they begin at, and no quotient passes 2^900.  A
 // depth whose low word is all ones is left out (see recip_line; one depth in
 // 2^32).  (Quotients of dividends below 2^-900 can then be off by 2^-700 at
-// most, far below the 1e-12 flush of the contributions they enter.)  Tested on
-// the high words: integer slots, which the FP64 tile has.
+// most, far below the 1e-12 flush of the contributions they enter.)  Ranges are
+// tested on the high words, in integer slots; the zero in FP64, one instruction
+// for two (flood of 96x150 1187 -> 1177 us a pass, rain 1531x2049 18.82 -> 18.72
+// ms).
 __device__ __forceinline__ bool regular_cell(double h, double qx, double qy) {
   constexpr uint32_t kLo = (1023u - 300u) << 20, kHi = (1023u + 100u) << 20;
   const uint32_t hh = (uint32_t)__double2hiint(h), hl = (uint32_t)__double2loint(h);
   const uint32_t ax = (uint32_t)__double2hiint(qx) & 0x7FFFFFFFu, ay = (uint32_t)__double2hiint(qy) & 0x7FFFFFFFu;
-  const bool hok = (hh - kLo <= kHi - kLo && hl != 0xFFFFFFFFu) || ((hh & 0x7FFFFFFFu) | hl) == 0u;
+  const bool hok = (hh - kLo <= kHi - kLo && hl != 0xFFFFFFFFu) || h == 0.0;
   return hok && max(ax, ay) <= kHi;
 }
 __device__ __forceinline__ bool regular_cell(float, float, float) { return true; }
