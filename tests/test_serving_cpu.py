@@ -125,3 +125,16 @@ def test_deadline_leaves_requests_unfinished_and_frees_them(stand_ins):
     done = srv.run(reqs, deadline=0.05)
     assert all(r.finished is None for r in done)
     assert _Domain.live == 0 and srv.batches == {}
+
+
+def test_launch_shapes_of_the_module_and_of_a_server(stand_ins, monkeypatch):
+    """serving.SHAPES holds for every server, a server's own shapes come first,
+    and a precision in neither is left to the batch."""
+    set_shapes = []
+    monkeypatch.setattr(_Batch, "set_shape", lambda self, v, rb: set_shapes.append((v, rb)))
+    for module, own, want in (({}, None, []), ({"fp32": (1, 16)}, None, [(1, 16)]), ({"fp32": (1, 16)}, {"fp32": (2, 8)}, [(2, 8)]),
+                              ({"fp64": (1, 16)}, None, [])):
+        set_shapes.clear()
+        monkeypatch.setattr(serving, "SHAPES", module)
+        serving.Server(hbm_budget=1e12, chunk_steps=8, shapes=own).run(_requests(1))
+        assert set_shapes == want

@@ -31,6 +31,10 @@ import numpy as np
 from .batch import Batch
 from .domain import Domain
 
+# Launch shapes of the batched flux kernel (variant, rows per tile) by precision
+# for every server; a precision left out takes the batch's own rule.
+SHAPES: dict[str, tuple[int, int]] = {}
+
 
 @dataclass
 class Request:
@@ -68,7 +72,7 @@ class Server:
         self.budget = float(hbm_budget)
         self.chunk = int(chunk_steps)
         self.max_members = int(max_members)
-        self.shapes = dict(shapes or {})  # launch shapes (variant, rows per tile); else the batch's own rule
+        self.shapes = dict(SHAPES, **(shapes or {}))
         self.used = 0
         self.peak_used = 0
         self.batches: dict[str, Batch] = {}
