@@ -135,3 +135,46 @@ def test_a_large_member_among_many_small_ones_keeps_its_blocks(precision, small)
     finally:
         for d in [large] + others:
             d.close()
+
+
+_SOLO = {}
+
+
+def _advanced(precision, steps):
+    """Members whose tiles fill more than one round of the flux kernel's warps at
+    6 rows and of the post kernel's at one row, and each one's fields after
+    `steps` steps alone at its default shape."""
+    if precision not in _SOLO:
+        scs = _members()[4:] + scenarios.ensemble(members=2, seed=12, side_min=690, side_max=730, duration=600.0,
+                                                  rain_range=(50, 200))
+        got = []
+        for sc in scs:
+            d = sc.to_domain(precision)
+            d.set_clock(sim_duration=1e300, print_interval=1e300, time_series=0, it_print=0)
+            assert d.advance(steps)[0] == steps
+            got.append([d.download(f) for f in ("h", "qx", "qy", "maxh")] + [np.array(d.get_clock().simtime)])
+            d.close()
+        _SOLO[precision] = scs, got
+    return _SOLO[precision]
+
+
+@pytest.mark.parametrize("variant,rb", [(0, 1), (1, 6), (2, 12), (0, 32), (1, 100)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_batch_tile_heights_equal_solo_runs(precision, variant, rb):
+    """Heights that divide the members' rows and that leave short last rows,
+    whole tiles and the last ones in parts, several post tiles a warp."""
+    scs, solo = _advanced(precision, 21)
+    doms = [sc.to_domain(precision) for sc in scs]
+    try:
+        for d in doms:
+            d.set_clock(sim_duration=1e300, print_interval=1e300, time_series=0, it_print=0)
+        with Batch(doms) as b:
+            b.set_shape(variant, rb)
+            assert b.advance(21).steps == 21
+        for sc, d, want in zip(scs, doms, solo):
+            got = [d.download(f) for f in ("h", "qx", "qy", "maxh")] + [np.array(d.get_clock().simtime)]
+            for f, a, w in zip(("h", "qx", "qy", "maxh", "simtime"), got, want):
+                assert np.array_equal(a, w), f"{sc.name}: {f} differs in {int((a != w).sum())} values"
+    finally:
+        for d in doms:
+            d.close()
