@@ -299,3 +299,44 @@ def test_extbc_lists_with_ghosts_or_repeats_stay_parallel():
             best = min(best, a.elapsed_time(b) * 100.0)
         us[name] = best
     assert us["ghost"] < 4 * us["plain"] and us["twice"] < 4 * us["plain"], us
+
+
+_DEPTHS = [0.0, -0.0, 1e-310, 1e-95, 1e-12, 1e-3, 0.7, 0.9999999999999999, 3.0, 1e40]
+
+
+@pytest.mark.parametrize("hx", [1e-3, 1e-40, 0.0])
+def test_flux_of_values_past_the_straight_line_range_matches_oracle(oracle, hx):
+    """Faces between depths of any size, at rest and with large discharges in
+    ordinary depths; a threshold of zero with every cell wet."""
+    rng = np.random.default_rng(3)
+    R, Cc = 37, 53
+    h = rng.choice(np.array(_DEPTHS if hx else _DEPTHS[3:]), (R, Cc))
+    z = rng.random((R, Cc))
+    big = rng.choice(np.array([0.0, 0.3, -2.0, 1e31, -1e35]), (R, Cc))
+    qx = np.where((h > 1e-3) & (h < 4.0), big, 0.0)
+    qy = np.where((h > 1e-3) & (h < 4.0), rng.permutation(big), 0.0)
+    want, got = _flux_both(oracle, R, Cc, h, qx, qy, z, np.maximum(np.sqrt(h), 0.0), hx)
+    for a, b in zip(want, got):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("hx", [1e-3, 1e-40, 0.0])
+def test_dt_of_values_past_the_straight_line_range_matches_oracle(oracle, hx):
+    """Wave speeds of depths and discharges of any size, NaN and infinity among them."""
+    import torch
+    from triton_b200 import _abi
+    L, O = _abi.lib(), oracle.lib()
+    O.tor_compute_dt_and_sqrt.restype = None
+    hs = np.array(_DEPTHS + [np.nan, np.inf, -1.0, 1e300, 5e-324])
+    qs = np.array([0.0, -0.0, 5e-324, 1e-300, 0.3, -7.0, 1e31, 1e35, 1e300, np.nan, np.inf, -np.inf])
+    h, qx, qy = (np.ascontiguousarray(a.reshape(-1)) for a in np.meshgrid(hs, qs, qs, indexing="ij"))
+    n = h.size
+    sq, dt = np.zeros(n), np.zeros(n)
+    O.tor_compute_dt_and_sqrt(n, C.c_double(3.0), qx.ctypes.data_as(_dp), qy.ctypes.data_as(_dp), h.ctypes.data_as(_dp),
+                              sq.ctypes.data_as(_dp), dt.ctypes.data_as(_dp), C.c_double(0.5), C.c_double(hx))
+    dev = [_dev(torch, a) for a in (qx, qy, h)]
+    dsq, ddt = torch.zeros(n, dtype=torch.float64, device="cuda"), torch.zeros(n, dtype=torch.float64, device="cuda")
+    _abi.check(L.tri_kernel_compute_dt_and_sqrt_f64(n, 3.0, *[_p(t) for t in dev], _p(dsq), _p(ddt), 0.5, hx, None))
+    torch.cuda.synchronize()
+    assert np.array_equal(dsq.cpu().numpy(), sq, equal_nan=True)
+    assert np.array_equal(ddt.cpu().numpy(), dt, equal_nan=True)

@@ -340,3 +340,98 @@ def test_autotune_tries_the_default_shape():
                 assert b.autotune(2)["candidates"] == tried
         finally:
             d.close()
+
+
+def _odd_cells(sc, depth, discharge):
+    rows, cols = sc.rows - 2, sc.cols - 2
+    for r, c in ((1, 1), (8, 30), (9, 31 if cols > 31 else 5), (rows, cols)):
+        sc.h[r, c] = depth
+        sc.qx[r, c], sc.qy[r, c] = discharge, -discharge
+    return sc
+
+
+@pytest.mark.parametrize("depth,discharge,hextra,steps", [(1e40, 0.0, 1e-3, 6), (1e-95, 0.0, 1e-100, 4),
+                                                          (1.0, 1e35, 1e-3, 2), (1.0, 1e31, 1e-3, 4)])
+def test_values_past_the_straight_line_range_match_oracle(depth, discharge, hextra, steps):
+    """Depths above 2^100, wet ones below 2^-300 and discharges above 2^100 on
+    tile edges: those tiles, and the wave speeds of such cells, take the guarded
+    forms, bit for bit, alone and as a member of a batch."""
+    from tests._harness import compare_fields, oracle_from_scenario
+    from triton_b200 import scenarios
+    from triton_b200.batch import Batch
+    for batch in (False, True):
+        sc = scenarios.mixed(rows=40, cols=61, seed=31, friction=False, with_extbc=False, with_sources=False,
+                             with_runoff=False, duration=1e3)
+        sc.hextra = hextra
+        _odd_cells(sc, depth, discharge)
+        o, d = oracle_from_scenario(sc), sc.to_domain()
+        try:
+            o.advance(steps)
+            if batch:
+                with Batch([d]) as b:
+                    b.set_shape(0, 8)
+                    b.advance(steps)
+            else:
+                d.advance(steps)
+            assert all(np.isfinite(o.grid(f)).all() for f in ("h", "qx", "qy"))
+            assert d.get_clock().simtime == o.s.simtime
+            compare_fields(o, d, True, hextra)
+        finally:
+            d.close()
+
+
+def _uniform_flow(h, qx, qy, n2, hextra):
+    """A flat channel in uniform flow: one step changes its inner cells by
+    friction alone."""
+    from triton_b200 import scenarios
+    sc = scenarios.mixed(rows=40, cols=45, seed=1, with_extbc=False, with_sources=False, with_runoff=False, duration=1e3)
+    sc.hextra = hextra
+    sc.h[1:-1, 1:-1], sc.qx[1:-1, 1:-1], sc.qy[1:-1, 1:-1] = h, qx, qy
+    sc.z[1:-1, 1:-1], sc.n2[:] = 0.0, n2
+    return sc
+
+
+_FLOWS = [(1.0, 0.3, 0.2, 1e-3, 1e-3), (1.0, 0.3, 0.0, 1e-3, 1e-3), (1.0, 0.3, 1e-70, 1e-3, 1e-3),
+          (1.0, 0.3, 1e-250, 1e-3, 1e-3), (1.0, 0.3, 0.2, 1e19, 1e-3), (1.0, 1e-11, 0.0, 1e-3, 1e-3),
+          (1.0, 3e-13, 0.0, 1e-3, 1e-3), (1e-40, 2e-12, 1e-100, 1e-3, 1e-45), (1.0, 0.3, 0.2, 1e-11, 1e-3)]
+
+
+@pytest.mark.parametrize("h,qx,qy,n2,hextra", _FLOWS)
+def test_friction_over_its_range_matches_oracle(h, qx, qy, n2, hextra):
+    """Friction terms of any size, transverse discharges that have decayed, both
+    sides of the thresholds.  Tolerance: the cube root's last bits move the
+    friction term t by a few ulps, and the reference's -(m - m*s)/(2t) loses
+    1/t of its digits: 8 ulps times 1 + 1/t."""
+    from tests._harness import oracle_from_scenario
+    sc = _uniform_flow(h, qx, qy, n2, hextra)
+    o, d = oracle_from_scenario(sc), sc.to_domain()
+    try:
+        assert o.advance(1) == d.advance(1) == (1, 0)
+        inner = (slice(6, -6), slice(6, -6))
+        t = o.s.global_dt * 9.81 * n2 * np.hypot(qx, qy) / (h * h * np.cbrt(h))
+        for f in ("qx", "qy"):
+            a, w = d.download(f)[inner], o.grid(f)[inner]
+            assert np.abs(a - w).max() <= 8 * 2.0 ** -52 * (1 + 1 / t) * np.abs(w).max() + 5e-324, f
+        assert np.array_equal(d.download("h")[inner], o.grid("h")[inner])
+    finally:
+        d.close()
+
+
+@pytest.mark.parametrize("h,qx,qy,n2,hextra", _FLOWS)
+def test_friction_of_guarded_tiles_has_the_same_bits(h, qx, qy, n2, hextra):
+    """The same cells in a tile that holds a cell out of range (too far away to
+    reach them in a step) and in one that does not."""
+    got = []
+    for odd in (False, True):
+        sc = _uniform_flow(h, qx, qy, n2, hextra)
+        sc.h[1, 1], sc.qx[1, 1], sc.qy[1, 1] = 1e-310 if odd else 0.0, 0.0, 0.0
+        d = sc.to_domain()
+        try:
+            d.set_shape(0, 40)
+            d.set_clock(time_increment_fixed=1, time_step=1e-40 if h < 1 else 0.05)
+            assert d.advance(1)[0] == 1
+            got.append([d.download(f)[8:-1, 8:-1] for f in ("h", "qx", "qy")])
+        finally:
+            d.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
