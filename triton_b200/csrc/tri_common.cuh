@@ -63,28 +63,13 @@ __device__ __forceinline__ float div_rare(float a, float b) { return a / b; }
 // System/6000 processor", IBM J. Res. Dev. 34(1), 1990): q0 = RN(a*y) is within
 // one ulp of a/b, the residual r = a - b*q0 is exact in one fused
 // multiply-add, and RN(q0 + r*y) is the correctly rounded quotient.  The
-// theorem needs a, b and a/b normal (no overflow or underflow).  An exact
-// quotient (r == 0) returns q0 itself, which also keeps the sign of a zero.
-// Three operations instead of a full division when the divisor is reused.
-template <typename T>
-__device__ __forceinline__ T div_by_rcp(T a, T b, T y) {
-  const T q0 = a * y;
-  const T r = dev_fma(-q0, b, a);
-  return r == T(0) ? q0 : dev_fma(r, y, q0);
-}
-// FP32 form: within 1.5 ulp is enough, one multiplication.
-template <>
-__device__ __forceinline__ float div_by_rcp<float>(float a, float, float y) {
-  return a * y;
-}
-
-// div_by_rcp for a dividend that is never a zero (and never subnormal): with
-// q0 != 0, an exact quotient (r == 0) gives fma(0, y, q0) == q0, so the
-// zero-residual test is not needed.  The solver's uses: dt*p with |p| >=
-// 1e-12 (smaller face contributions are flushed to +0 before, and dt*(+0)
-// is the exact quotient +0 both ways: r = +0, fma(+0, y, +0) = +0), and
-// h*dx/2 with h > 0 (a depth, far above the subnormal range; the same
-// three operations as div_by_rcp there).
+// theorem needs a, b and a/b normal (no overflow or underflow).  Three
+// operations instead of a full division when the divisor is reused.  For a
+// dividend that is never a zero (and never subnormal): with q0 != 0, an exact
+// quotient (r == 0) gives fma(0, y, q0) == q0.  The solver's uses: dt*p with
+// |p| >= 1e-12 (smaller face contributions are flushed to +0 before, and dt*(+0)
+// is the exact quotient +0 both ways: r = +0, fma(+0, y, +0) = +0), and h*dx/2
+// (a depth far above the subnormal range, or a zero whose sign does not matter).
 template <typename T>
 __device__ __forceinline__ T div_nz(T a, T b, T y) {
   const T q0 = a * y;
@@ -96,7 +81,7 @@ __device__ __forceinline__ float div_nz<float>(float a, float, float y) {
 }
 
 // a / b rounded to nearest for a divisor b shared by several quotients, from
-// y = RN(1/b): div_by_rcp where Markstein's conditions provably hold (|a| >=
+// y = RN(1/b): Markstein's quotient where its conditions provably hold (|a| >=
 // 2^-900 so the residual a - b*q0 is exact, and q0 = RN(a*y) between 2^-1000
 // and 2^1000 so the quotient is normal), a plain division otherwise.  A zero
 // dividend gives the signed zero of a/b.  Bit-identical to a / b for every

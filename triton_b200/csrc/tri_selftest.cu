@@ -1,12 +1,13 @@
 // tri_selftest.cu -- tri_selftest_division: checks on the device that the
 // exact quotients from a correctly rounded reciprocal equal the IEEE quotient
-// bit for bit: div_by_rcp over operands shaped like the step's (dt*d/dx,
+// bit for bit: div_nz over operands shaped like the step's (dt*d/dx,
 // h*dx/2/dt: magnitudes 1e-14 .. 1e7 over divisors 1e-3 .. 1e3) and
 // div_shared over every finite dividend magnitude (subnormals included,
 // zeros of both signs) and divisors of either sign from 1e-30 to 1e30.  Also
-// the straight-line forms of the FP64 flux tile (tri_common.cuh) over their
-// whole range, 2^-300 .. 2^300, a part of it at operands whose result lies
-// next to the midpoint of two doubles or whose mantissa is all ones.
+// the straight-line forms of the FP64 flux tile (tri_common.cuh) over the range
+// of its faces, 2^-300 .. 2^300 (depths end at 2^100), a part of it at operands
+// whose result lies next to the midpoint of two doubles or whose mantissa is all
+// ones, and over that of its friction terms, 2^-700 .. 2^760.
 #include <cuda_runtime.h>
 
 #include "tri_common.cuh"
@@ -66,6 +67,13 @@ __device__ int line_check(unsigned long long r1, unsigned long long r2) {
   const double a = ldexp(1.0 + (double)(r2 >> 12) * 0x1p-52, (int)(r2 % 601) - 300) * ((r2 & 16) ? -1.0 : 1.0);
   bad += differ(div_line(a, x, rx), a / x);
   bad += div_line(0.0, x, rx) != 0.0;
+  const int ew = (int)((r1 >> 8) % 1460) - 700;  // friction terms and their denominators
+  const double w = ldexp(m, ew), rw = 1.0 / w;
+  bad += differ(sqrt_line(w, rsqrt_line(w)), sqrt(w));
+  bad += differ(recip_line(w), rw);
+  const int lo = max(-300, ew - 960), hi = min(751, ew + 760);
+  const double d = ldexp(1.0 + (double)(r2 >> 12) * 0x1p-52, lo + (int)((r2 >> 8) % (unsigned)(hi - lo + 1)));
+  bad += differ(div_line(d, w, rw), d / w);
   return bad;
 }
 
@@ -79,7 +87,7 @@ __global__ void k_div_check(long long n, unsigned long long seed, unsigned long 
     const double b = exp10(eb);
     if ((r2 & 0xFF) == 0) a = 0.0;
     const double y = 1.0 / b;
-    const double q = div_by_rcp(a, b, y);
+    const double q = div_nz(a, b, y);
     const double ref = a / b;
     if (__double_as_longlong(q) != __double_as_longlong(ref)) local++;
     // div_shared over any finite dividend (subnormal to 1e300) and divisors
