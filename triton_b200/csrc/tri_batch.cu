@@ -40,8 +40,7 @@ struct tri_batch {
   uint32_t ntiles = 0, nwet = 0;
   int rb = 8, variant = 1, flux_blocks = 1;
   bool shape_set = false;  // tuned or set by the caller: the default no longer applies
-  // graph mode: member of every post kernel block, tile flags ([tiles], then
-  // [tiles] pinned), the tiles' wave speeds, their forcing
+  // graph mode: member of every post kernel block, the tiles' forcing
   int32_t* d_post_mem = nullptr;
   uint32_t npost = 0;
   int32_t* d_tlists = nullptr;
@@ -87,8 +86,6 @@ MemberDev<T> member_dev(tri_domain* d, int rb, uint32_t& tiles, uint32_t& wet) {
   m.dx = (T)a.dx;
   m.rdx = (T)(1.0 / a.dx);
   m.hextra = (T)a.hextra;
-  m.dxd = a.dx;
-  m.courant = a.courant;
   const uint32_t strips = (uint32_t)((a.cols - 2 + kStripCols - 1) / kStripCols);
   const uint32_t rowb = (uint32_t)((a.rows - 2 + rb - 1) / rb);
   m.tile_begin = tiles;
@@ -308,9 +305,9 @@ int launch_batch(tri_batch* b, int n) {
   return TRI_OK;
 }
 
-// Prepares every member's clock for a batched advance of at most 'limit'
-// steps (members at or past
-// their end stay halted for the whole call); counts the members that step.
+// Prepares every member's clock for a batched advance of at most 'limit' steps
+// (members at or past their end stay halted for the whole call); counts the
+// members that step.
 // Clocks go to the device on the batch stream, ahead of the batched launches;
 // a member without a valid CFL dt (new, or state uploaded) gets it first on
 // its own stream.

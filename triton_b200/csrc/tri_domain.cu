@@ -220,7 +220,6 @@ StepArgs step_args(tri_domain* d) {
   a.flux_blocks = d->flux_blocks;
   a.flux_variant = d->flux_variant;
   a.dx = d->desc.cell_size;
-  a.courant = d->desc.courant;
   a.hextra = d->desc.hextra;
   a.nsrc = d->nsrc;
   a.src_cells = d->src_cells;
@@ -261,7 +260,7 @@ int build_tile_lists(tri_domain* d) {
   TRI_CUDA_TRY(cudaStreamSynchronize(d->stream));
   if (nt != d->tz_tiles) {
     free_devp(d->tflag);
-      d->tz_tiles = 0;
+    d->tz_tiles = 0;
     if (cudaMalloc((void**)&d->tflag, 3 * (size_t)nt) != cudaSuccess)
       return set_error(TRI_E_NOMEM, "cudaMalloc of %lld tile flags failed", (long long)nt);
     d->tz_tiles = nt;

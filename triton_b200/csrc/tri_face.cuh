@@ -324,16 +324,16 @@ __device__ __forceinline__ FaceOut<T> face_flux(const CellQ<T>& c1, const CellQ<
       p2 += right2 ? T(0) : y2;
       q1 += right2 ? y1 : T(0);
       q2 += right2 ? y2 : T(0);
-    if (brink) {
-      const bool dry2 = h2 < E12 && hp + div_rare(be2, lam2) < -E12;
-      const bool dry1 = !dry2 && h1 < E12 && hp - div_rare(be0, lam0) < -E12;
-      if (dry1 || dry2) {
-        const T m = w0 + w2;
-        p0 = dry2 ? m : T(0);
-        q0 = dry2 ? T(0) : m;
-        p1 = p2 = q1 = q2 = T(0);
+      if (brink) {
+        const bool dry2 = h2 < E12 && hp + div_rare(be2, lam2) < -E12;
+        const bool dry1 = !dry2 && h1 < E12 && hp - div_rare(be0, lam0) < -E12;
+        if (dry1 || dry2) {
+          const T m = w0 + w2;
+          p0 = dry2 ? m : T(0);
+          q0 = dry2 ? T(0) : m;
+          p1 = p2 = q1 = q2 = T(0);
+        }
       }
-    }
     } else {
       p0 = p1 = p2 = q0 = q1 = q2 = T(0);
       if (h2 < E12 && hp + div_rare(be2, lam2) < -E12) {

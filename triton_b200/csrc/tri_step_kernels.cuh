@@ -721,8 +721,7 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, FluxUnit u,
   const bool upd = mid && c >= 1 && c <= cols - 2;
   const bool gcol = incol && (c == 0 || c == cols - 1);  // ghost column owned by this lane
   const bool owner = incol && (mid || gcol);
-  constexpr bool kAcct = true;  // FP64 volume accounts in both forms
-  double acc_b = 0.0, acc_r = 0.0, acc_c = 0.0;
+  double acc_b = 0.0, acc_r = 0.0, acc_c = 0.0;  // FP64 volume accounts in both forms
   const double sxq = (double)X.K.dt / (double)X.K.dx;  // dt/dx of the boundary discharges
 
   bool wrote_nonzero = false;  // any value this lane writes is not +0
@@ -812,13 +811,11 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, FluxUnit u,
       double clip;
       update_cell<T, kLine>(prev, pp, Y.b0, Y.b1, Y.b2, pn2, dt, hextra, hn, qn, vn, clip,
                             cell_hash((uint32_t)id, 2u * XU.step), odd);
-      if (kAcct) {
-        // Inflow through the south face of a cell of the last interior row
-        // (the other boundary faces are counted where their parts are
-        // formed, below), and the depth the update clipped back to zero.
-        if (r - 1 == XU.rows - 2) acc_b += sxq * (double)prev.qy - (double)Y.b0;
-        acc_c += clip;
-      }
+      // Inflow through the south face of a cell of the last interior row
+      // (the other boundary faces are counted where their parts are
+      // formed, below), and the depth the update clipped back to zero.
+      if (r - 1 == XU.rows - 2) acc_b += sxq * (double)prev.qy - (double)Y.b0;
+      acc_c += clip;
       if (XU.nroff > 0) {  // update_runoff (kernels.h:128-149)
         const T h0 = hn;
         // with one zone its rate, without the zone map
@@ -838,7 +835,7 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, FluxUnit u,
           qn = T(0);
           vn = T(0);
         }
-        if (kAcct) acc_r += (double)hn - (double)h0;
+        acc_r += (double)hn - (double)h0;
       }
       T* __restrict__ ho = XU.ho;
       T* __restrict__ qxo = XU.qxo;
@@ -864,7 +861,7 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, FluxUnit u,
     left.hd = shfl_up1(cur.hd);
     const FaceOut<T> Xf = face_flux<T, true, kLine>(left, cur, XL.K, crossx, dzx);
     const T e0 = shfl_down1(Xf.a0), e1 = shfl_down1(Xf.a1), e2 = shfl_down1(Xf.a2);
-    if (kAcct && upd) {
+    if (upd) {
       // Inflow through faces shared with ghost cells, in depth units.  The
       // update is in fluctuation form, so the mass flux through a face of
       // boundary cell i is F(Q_i).n plus the fluctuation it receives there:
@@ -885,15 +882,13 @@ __device__ __forceinline__ bool flux_tile_form(const FluxCtx<T>& X0, FluxUnit u,
     prev = cur;
   }
   if (kLine && __any_sync(0xffffffffu, odd)) return false;
-  if (kAcct) {
-    acc_b = warp_sum<T>(acc_b);
-    acc_r = warp_sum<T>(acc_r);
-    acc_c = warp_sum<T>(acc_c);
-    if (lane == 0) {
-      if (acc_b != 0.0) atomicAdd(&X.clk->acc_step[kAccBoundary], acc_b);
-      if (acc_r != 0.0) atomicAdd(&X.clk->acc_step[kAccRunoff], acc_r);
-      if (acc_c != 0.0) atomicAdd(&X.clk->acc_step[kAccClip], acc_c);
-    }
+  acc_b = warp_sum<T>(acc_b);
+  acc_r = warp_sum<T>(acc_r);
+  acc_c = warp_sum<T>(acc_c);
+  if (lane == 0) {
+    if (acc_b != 0.0) atomicAdd(&X.clk->acc_step[kAccBoundary], acc_b);
+    if (acc_r != 0.0) atomicAdd(&X.clk->acc_step[kAccRunoff], acc_r);
+    if (acc_c != 0.0) atomicAdd(&X.clk->acc_step[kAccClip], acc_c);
   }
   if (kTrack) {
     const bool nz = __any_sync(0xffffffffu, wrote_nonzero);
@@ -1051,9 +1046,9 @@ static_assert(WetStage<float>::kBand + 2 <= 32, "staged rows span at most two be
 // once more on every group from 'from' on so no copy still writes this
 // block's shared memory when it exits.
 template <int kGroups>
-__device__ __forceinline__ void stage_abandon(DevClock* clk, uint64_t* bar, int from, uint32_t parity) {
+__device__ __forceinline__ void stage_abandon(DevClock* clk, uint64_t* bar, int from) {
   atomicExch(&clk->status, kStatusStageTimeout);
-  for (int g = from; g < kGroups; ++g) mbar_wait(&bar[g], parity);
+  for (int g = from; g < kGroups; ++g) mbar_wait(&bar[g], 0);
 }
 
 // Test hook (one thread of one block): a bounded wait on a barrier whose
@@ -1069,13 +1064,11 @@ static __device__ __noinline__ void wait_test(DevClock* clk) {
   if (!mbar_wait(&bar, 0, clk->wait_test)) atomicExch(&clk->status, kStatusTestWait);
 }
 
-// iter: how many bands this block has staged before (its barriers' phase).
 template <typename T>
 __device__ __forceinline__ unsigned long long wetdry_staged(DevClock* __restrict__ clk, const StateBufs<T>& sb,
                                                             const BedMap<T>& bed, T* __restrict__ maxh, int rows,
                                                             int cols, T hextra, float* __restrict__ arrival,
-                                                            float arrival_depth, int bx, int by, T* stage,
-                                                            int iter = 0) {
+                                                            float arrival_depth, int bx, int by, T* stage) {
   using S = WetStage<T>;
   constexpr bool kF32 = sizeof(T) == 4;
   const int buf = clk->now.dst;
@@ -1096,7 +1089,7 @@ __device__ __forceinline__ unsigned long long wetdry_staged(DevClock* __restrict
   float* tdel = reinterpret_cast<float*>(offs + S::kHRows);
   const int rlo = max(ra - 1, 0), rhi = min(rz + 1, rows - 1);
   const int tr0 = rlo >> 5, tc0 = cl >> 5;
-  if (iter == 0 && tid < S::kGroups) mbar_init(&bar[tid], 1);
+  if (tid < S::kGroups) mbar_init(&bar[tid], 1);
   if (tid < S::kHRows) {
     const int64_t r = (int64_t)(ra - 1 + tid);
     offs[tid] = (int)(r * cols - ((r * cols + cl) & ~(int64_t)(S::kVec - 1)));
@@ -1164,8 +1157,8 @@ __device__ __forceinline__ unsigned long long wetdry_staged(DevClock* __restrict
   const bool incol = c < cols;
   const bool intcol = c >= 1 && c <= cols - 2;
   // FP32 form: tile deltas of columns c-1, c, c+1 in tile rows 0 and 1
-  // (BedMap::local_v; where a delta is zero the level is the offset itself,
-  // up to the sign of a zero, which no comparison below sees)
+  // (where a delta is zero the level is the offset itself, up to the sign of a
+  // zero, which no comparison below sees)
   T dw0 = T(0), dw1 = T(0), dc0 = T(0), dc1 = T(0), de0 = T(0), de1 = T(0);
   if (kF32 && intcol) {
     const int tw = ((c - 1) >> 5) - tc0, tc = (c >> 5) - tc0, te = ((c + 1) >> 5) - tc0;
@@ -1195,8 +1188,8 @@ __device__ __forceinline__ unsigned long long wetdry_staged(DevClock* __restrict
     for (int jq = 0; jq < S::kBand; ++jq) {
       const int r = ra + jq;
       if (r > rz) break;
-      if (jq % S::kGR == 0 && !mbar_wait(&bar[jq / S::kGR], (uint32_t)iter & 1)) {
-        stage_abandon<S::kGroups>(clk, bar, jq / S::kGR, (uint32_t)iter & 1);
+      if (jq % S::kGR == 0 && !mbar_wait(&bar[jq / S::kGR], 0)) {
+        stage_abandon<S::kGroups>(clk, bar, jq / S::kGR);
         return kDtKeyInf;
       }
       const int j = jq + 1;

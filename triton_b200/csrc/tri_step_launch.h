@@ -120,7 +120,7 @@ struct StepArgs {
   const void* rates;
   int rows, cols;
   int rb, flux_blocks, flux_variant;
-  double dx, courant, hextra;
+  double dx, hextra;
   int nsrc;
   const int32_t* src_cells;
   const double* hyg_t;
@@ -174,7 +174,7 @@ template <typename T>
 void flux_occupancy(int variant, int* per_sm);
 
 // A batch of member domains advanced together (one step of each member per
-// batched step).  Device pointers; wave offsets are host arrays.
+// batched step).  Device pointers.
 struct BatchArgs {
   const void* mem;  // MemberDev<T>[nm] in device memory
   int nm;

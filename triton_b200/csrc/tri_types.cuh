@@ -92,8 +92,6 @@ struct BedMap<double> {
   const double* base;  // unused
   int ntc;
   __device__ __forceinline__ double ref_of(int, int) const { return 0.0; }
-  __device__ __forceinline__ double local(size_t id, int, int, double) const { return z[id]; }
-  __device__ __forceinline__ double local_v(double zv, int, int, double) const { return zv; }
   __device__ __forceinline__ double base_at(int, int) const { return 0.0; }
   __device__ __forceinline__ double absolute(size_t id, int, int) const { return z[id]; }
 };
@@ -103,16 +101,7 @@ struct BedMap<float> {
   const double* base;  // FP64 base level of each 32x32 tile
   int ntc;             // tiles per row
   __device__ __forceinline__ double ref_of(int r, int c) const { return base[(r >> 5) * ntc + (c >> 5)]; }
-  __device__ __forceinline__ float local(size_t id, int r, int c, double ref) const {
-    const double b = base[(r >> 5) * ntc + (c >> 5)];
-    return b == ref ? z[id] : z[id] + (float)(b - ref);
-  }
   __device__ __forceinline__ double base_at(int r, int c) const { return base[(r >> 5) * ntc + (c >> 5)]; }
-  // the same for an offset already read (from shared memory)
-  __device__ __forceinline__ float local_v(float zv, int r, int c, double ref) const {
-    const double b = base[(r >> 5) * ntc + (c >> 5)];
-    return b == ref ? zv : zv + (float)(b - ref);
-  }
   __device__ __forceinline__ double absolute(size_t id, int r, int c) const {
     return base[(r >> 5) * ntc + (c >> 5)] + (double)z[id];
   }
@@ -154,7 +143,6 @@ struct MemberDev {
   float arrival_depth;
   int rows, cols, rb;
   T dx, rdx, hextra;
-  double dxd, courant;
   uint32_t tile_begin, tile_end;  // this member's tiles in the flux queue
   uint32_t wet_begin, wet_nbx;    // first wet-dry block, blocks per band row
   uint32_t post_begin, post_count;  // blocks of the post kernel
